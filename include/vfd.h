@@ -128,7 +128,15 @@ vfd_status vfd_world_fft_dims(const vfd_world *w, int *fft3);
 vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes);
 
 /* ---- autotuning (VFD_METHOD_SEPARABLE worlds) ---------------------------
- * Per axis, the pass that runs it: the register FFT (kernel radius <= 8),
+ * The per-axis operators of a substep (mask, convolve, crop) act on different
+ * axes and commute, so a tick of m substeps is one pass per axis that applies
+ * the axis' operator to the power m: a banded matrix, applied as a banded
+ * product on the tensor cores.  Worlds run on these products wherever they
+ * are the faster form (kernels up to 56 voxels of half-width after folding; a
+ * single substep of narrow kernels on large fields stays on the FFT passes),
+ * unless vfd_autotune_set pinned their FFT passes.  What follows chooses
+ * among the FFT passes.
+ * Per axis, the FFT pass: the register FFT (kernel radius <= 8),
  * overlap-save FFT-64 blocks (radius <= 16) at 3 or 4 resident CTAs per SM,
  * or a full-line FFT with a chosen padded length (the three cheapest
  * 7-smooth lengths >= n + r), radix order and kernel variant.  The reference
@@ -156,11 +164,11 @@ typedef struct vfd_axis_tuning {
  * vfd_world_create calls with that shape use the cached choice; with the
  * environment variable VFD_AUTOTUNE=1 they tune an uncached shape first. */
 vfd_status vfd_autotune(const vfd_world_desc *desc, int device, int reps, vfd_axis_tuning *out3);
-/* The pass each axis of this world runs (ms: the tuned time, 0 if the
+/* The FFT pass of each axis of this world (ms: the tuned time, 0 if the
  * world was not created from a tuned choice). */
 vfd_status vfd_world_tuning(const vfd_world *w, vfd_axis_tuning *out3);
 /* Stores a choice for desc's shape in the cache (a saved tuning, or a pinned
- * pass): later worlds of the shape run it.  An axis whose world cannot run
+ * pass): later worlds of the shape run it, and no banded products.  An axis whose world cannot run
  * the stored method (register FFT beyond radius 8 or on an unaligned x
  * line, overlap-save beyond radius 16) falls back to the default pass. */
 vfd_status vfd_autotune_set(const vfd_world_desc *desc, int device, const vfd_axis_tuning *in3);
@@ -298,7 +306,7 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
 typedef struct vfd_batch vfd_batch;
 vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **out);
 vfd_status vfd_batch_tick(vfd_batch *b, int n_substeps, void *stream);
-/* Per-axis pass choice for the batch as a whole: times every candidate
+/* Per-axis FFT pass choice for the batch as a whole: times every candidate
  * (register FFT, overlap-save at 3 and at 4 resident CTAs per SM, full-line
  * FFT) over all the batch's fields -- one warm-up and `reps` timed launches
  * each, CUDA events -- and keeps the fastest per axis (out3, may be NULL).

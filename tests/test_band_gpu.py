@@ -1,0 +1,177 @@
+"""GPU tests of the banded-product passes (m substeps folded into one operator
+per axis, applied on the tensor cores) at the sizes where their tiling,
+operators and folding change: lines of one block, one more and one less,
+partly filled tiles, the three ways input blocks are copied, narrow and wide
+kernels, several groups of folded substeps, the padding rule's affine part.
+
+Tolerance: a pass rounds its inputs (relative to the line's offset), three
+parts of value and weight (2^-24 each), a K / 16-step accumulation whose
+truncation is relative to values about the offset, and the sum with the
+offset's product: at most 4 units of 2^-24 of the field's level; three passes
+a group and the final decay and deposit give 14 * 2^-24 = 8.4e-7 a group."""
+import numpy as np
+import pytest
+
+import oracle
+import vfd
+
+pytestmark = pytest.mark.gpu
+
+PER_GROUP = 14 * 2.0 ** -24
+
+
+def rel_l2(a, b):
+    a = np.asarray(a, np.float64)
+    return float(np.sqrt(((a - b) ** 2).sum() / max((b ** 2).sum(), 1e-300)))
+
+
+def check(grid, sig, substeps, groups=1, pad=vfd.PAD_ZERO, epi=0, base=0.0, dec=0.04, radius=None, nf=2, seed=9):
+    nx, ny, nz = grid
+    V = nx * ny * nz
+    params = [vfd.field_params(sig, dec, radius=radius, baseline=base * (f + 1)) for f in range(nf)]
+    ins = []
+    with vfd.World(nx, ny, nz, params, pad_mode=pad, epi_boundary=epi) as w:
+        for f in range(nf):
+            u = vfd.synth_field(seed, 1, f, (nz, ny, nx))
+            idx, amt = vfd.synth_sources(seed, 1, f, 23, V)
+            ins.append((u, idx, amt))
+            w.upload(f, u)
+            w.set_sources(f, idx, amt)
+        w.tick(substeps)
+        outs = [w.download(f) for f in range(nf)]
+        mass = w.mass()
+    for f, (u, idx, amt) in enumerate(ins):
+        b = float(np.float32(base * (f + 1)))
+        ref = oracle.tick(u, sig, dec, substeps, idx, amt, b=b, pad_mode=pad, epi=epi, radius3=radius)
+        e = rel_l2(outs[f], ref)
+        assert e <= groups * PER_GROUP, (grid, sig, substeps, f, e)
+        m, s = mass[f], outs[f].astype(np.float64).sum()
+        scale = max(abs(m["input_sum"]), abs(s), 1e-30)
+        assert abs(m["input_sum"] - m["conv_sum"] - sum(m["leaked"])) <= 1e-6 * scale
+        assert abs(m["total"] - s) <= 1e-6 * max(abs(s), 1e-30)
+
+
+# x lines of one block, its neighbours and several; nx % 4 != 0 (4-byte
+# copies), % 4 == 0 (16-byte copies along y), % 32 == 0 (bulk tensor copies)
+@pytest.mark.parametrize("grid", [(64, 5, 3), (63, 9, 4), (65, 3, 7), (68, 70, 9), (128, 66, 3), (96, 64, 65),
+                                  (129, 33, 1), (1, 64, 130), (260, 4, 11)])
+@pytest.mark.parametrize("substeps", [1, 10])
+def test_line_lengths_and_copies(gpu, grid, substeps):
+    check(grid, 1.3, substeps)
+
+
+# half-widths of 4 and 8 up to the widest operator (radius 56), and kernels
+# wider than short lines
+@pytest.mark.parametrize("radius", [1, 4, 9, 17, 33, 56])
+def test_kernel_widths(gpu, radius):
+    check((200, 36, 40), radius / 3.0, 1, radius=radius)
+
+
+# groups: sigma 2.6 folds 11 substeps (half-width <= 56), 0.6 folds 16
+@pytest.mark.parametrize("sigma,substeps,groups", [(2.6, 11, 1), (2.6, 12, 2), (2.6, 25, 3), (0.6, 16, 1), (0.6, 17, 2),
+                                                   (5.0, 3, 1), (5.0, 7, 3)])
+def test_folded_groups(gpu, sigma, substeps, groups):
+    check((140, 70, 68), sigma, substeps, groups=groups)
+
+
+@pytest.mark.parametrize("substeps", [1, 2, 10, 19])
+@pytest.mark.parametrize("epi", [1, 2, 65, 130, 200])
+def test_padding_rule(gpu, substeps, epi):
+    check((132, 20, 35), 1.1, substeps, groups=(substeps + 15) // 16, pad=vfd.PAD_CONSTANT_VF, epi=epi, base=3e-4)
+
+
+def test_signs_and_scales(gpu):
+    """Fields of either sign and of scales 1e-20 and 1e20 (the offset and the
+    bf16 parts keep FP32's range), one field each in one launch."""
+    nx, ny, nz = 72, 40, 33
+    rng = np.random.default_rng(4)
+    us = [(rng.standard_normal((nz, ny, nx)) * s).astype(np.float32) for s in (1.0, 1e-20, 1e20)]
+    with vfd.World(nx, ny, nz, [vfd.field_params(1.4, 0.02)] * 3) as w:
+        for f, u in enumerate(us):
+            w.upload(f, u)
+        w.tick(4)
+        outs = [w.download(f) for f in range(3)]
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    for u, o in zip(us, outs):
+        ref = oracle.tick(u, 1.4, 0.02, 4, *none)
+        # four substeps shrink unit noise to about 1/30: the bound is on the input's scale
+        err = np.sqrt(((o - ref) ** 2).sum() / (u.astype(np.float64) ** 2).sum())
+        assert err <= PER_GROUP
+
+
+def test_non_finite_values_stay_local(gpu):
+    """A NaN reaches its own lines only; the rest of the field is untouched."""
+    nx, ny, nz = 160, 24, 70
+    u = vfd.synth_field(2, 0, 0, (nz, ny, nx))
+    bad = u.copy()
+    bad[40, 12, 20] = np.nan
+    outs = []
+    for v in (u, bad):
+        with vfd.World(nx, ny, nz, [vfd.field_params(0.6, 0.0)]) as w:
+            w.upload(0, v)
+            w.tick(1)
+            outs.append(w.download(0))
+    hit = ~np.isfinite(outs[1])
+    assert hit[40, 12, 20]
+    # x lines of the window's blocks, every y of the line block, z blocks likewise: never the far x half
+    assert not hit[:, :, 136:].any()
+    np.testing.assert_array_equal(outs[0][~hit], outs[1][~hit])
+
+
+def test_single_field_and_world_launches_agree(gpu):
+    """vfd_diffuse_host runs one field a launch, a batch all worlds in one."""
+    grid, sig = (100, 41, 37), [0.9, 1.7, 2.3]
+    nx, ny, nz = grid
+    params = [vfd.field_params(s, 0.03) for s in sig]
+    us = [vfd.synth_field(6, 0, f, (nz, ny, nx)) for f in range(3)]
+    with vfd.World(nx, ny, nz, params) as w, vfd.World(nx, ny, nz, params) as v, vfd.World(40, 30, 20, params) as o:
+        for f, u in enumerate(us):
+            w.upload(f, u)
+            v.upload(f, u)
+            o.upload(f, vfd.synth_field(7, 0, f, (20, 30, 40)))
+        w.tick(5)
+        outs = [w.download(f) for f in range(3)]
+        with vfd.Batch([o, v]) as b:
+            b.tick(5)
+        for f in range(3):
+            np.testing.assert_array_equal(outs[f], v.download(f))
+        host = [np.empty_like(u) for u in us]
+        w.diffuse_host(us, host, 5)
+    for f in range(3):
+        np.testing.assert_array_equal(outs[f], host[f])
+
+
+def test_batch_results_do_not_depend_on_neighbours(gpu):
+    """Worlds on banded products, on FFT passes (a single substep of a large
+    world with narrow kernels; pinned passes) and with several groups of
+    folded substeps share a batch: each result equals its own single tick."""
+    vfd.autotune_clear()
+    try:
+        vfd.autotune_set(44, 40, 36, [vfd.field_params(1.0, 0.02)] * 2, [{"method": "overlap_save"}] * 3)
+        specs = [((44, 40, 36), 1.0), ((176, 160, 96), 0.9), ((90, 33, 70), 2.6), ((64, 64, 32), 0.7)]
+        for substeps in (1, 12):
+            worlds, singles = [], []
+            for i, (g, sig) in enumerate(specs):
+                for out in (worlds, singles):
+                    w = vfd.World(*g, [vfd.field_params(sig, 0.02)] * 2)
+                    for f in range(2):
+                        w.upload(f, vfd.synth_field(3, i, f, g[::-1]))
+                    out.append(w)
+            with vfd.Batch(worlds) as b:
+                for _ in range(3):  # directly, captured, replayed
+                    b.tick(substeps)
+                b.tick(3)
+                b.tick(substeps)
+            for w, v in zip(worlds, singles):
+                for n in (substeps,) * 3 + (3, substeps):
+                    v.tick(n)
+                for f in range(2):
+                    np.testing.assert_array_equal(w.download(f), v.download(f))
+                got, ref = w.mass(), v.mass()
+                for f in range(2):
+                    assert got[f]["total"] == pytest.approx(ref[f]["total"], rel=1e-12)
+                    assert got[f]["input_sum"] == pytest.approx(ref[f]["input_sum"], rel=1e-12)
+                w.close()
+                v.close()
+    finally:
+        vfd.autotune_clear()

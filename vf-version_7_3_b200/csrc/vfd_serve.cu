@@ -127,8 +127,9 @@ namespace {
 
 size_t estimate_bytes(const Request &r)
 {
-    // fields + per-axis tables (generous) + sources
+    // fields + per-axis tables (generous) + banded operators + sources
     size_t b = sizeof(float) * (size_t)r.nx * r.ny * r.nz * r.nf;
+    for (int n : {r.nx, r.ny, r.nz}) b += (size_t)r.nf * 32 * 1024 * std::min((n + 63) / 64, 4);
     b += (size_t)r.nf * 3 * 4096 * sizeof(float) + 3 * 4096 * 8 + 64 * 1024;
     for (const auto &v : r.src_idx) b += v.size() * 8;
     return b;

@@ -26,10 +26,11 @@ bool tma_available()
 }
 
 bool tma_encode_3d(CUtensorMap *m, const float *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
-                   uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2)
+                   uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128)
 {
     if (!tma_available() || !m || !base) return false;
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (s1 & 15) != 0 || (s2 & 15) != 0) return false;
+    if (swizzle128 && b0 != 32) return false;
     if ((b0 * 4) % 16 != 0 || b0 < 1 || b1 < 1 || b2 < 1 || b0 > 256 || b1 > 256 || b2 > 256) return false;
     if (d0 < 1 || d1 < 1 || d2 < 1 || d0 >= (1ull << 32) || d1 >= (1ull << 32) || d2 >= (1ull << 32)) return false;
     if (s1 >= (1ull << 40) || s2 >= (1ull << 40)) return false;
@@ -38,8 +39,8 @@ bool tma_encode_3d(CUtensorMap *m, const float *base, uint64_t d0, uint64_t d1, 
     const cuuint32_t box[3] = {b0, b1, b2};
     const cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(base), dims, strides, box, estr,
-                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                          CU_TENSOR_MAP_INTERLEAVE_NONE,
+                          swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
 

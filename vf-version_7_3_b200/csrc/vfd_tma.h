@@ -23,9 +23,11 @@ bool tma_available();
 // (d0 contiguous), byte strides s1 (dim 1) and s2 (dim 2), box {b0, b1, b2},
 // zero fill out of bounds.  Returns false when the driver rejects it or the
 // layout breaks a TMA rule (16-byte aligned base and strides, b0 * 4 a
-// multiple of 16, every box dim <= 256).
+// multiple of 16, every box dim <= 256).  swizzle128: rows of 128 bytes (b0 =
+// 32) land with their 16-byte chunk c at c ^ (row & 7), the box at a multiple
+// of 1024 bytes.
 bool tma_encode_3d(CUtensorMap *m, const float *base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t s1,
-                   uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2);
+                   uint64_t s2, uint32_t b0, uint32_t b1, uint32_t b2, bool swizzle128 = false);
 
 #ifdef __CUDACC__
 // Cycles after which a wait for a bulk copy gives up (about 1 s at 2 GHz).

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "vfd.h"
+#include "vfd_band.h"
 #include "vfd_general.h"
 #include "vfd_internal.h"
 #include "vfd_os.h"
@@ -183,8 +184,8 @@ int variant_for_plan(const FftPlan &p, int need_nl)
     return -1;
 }
 
-// Real multipliers G(k)/F of the wrapped normalised Gaussian taps, FP64.
-static void gauss_spectrum(double sigma, int r, int F, std::vector<float> &out)
+// The normalised sampled Gaussian, FP64.
+static std::vector<double> gauss_taps(double sigma, int r)
 {
     std::vector<double> g(2 * r + 1);
     double s = 0.0;
@@ -193,6 +194,13 @@ static void gauss_spectrum(double sigma, int r, int F, std::vector<float> &out)
         s += g[j + r];
     }
     for (auto &x : g) x /= s;
+    return g;
+}
+
+// Real multipliers G(k)/F of the wrapped normalised Gaussian taps, FP64.
+static void gauss_spectrum(double sigma, int r, int F, std::vector<float> &out)
+{
+    const std::vector<double> g = gauss_taps(sigma, r);
     out.resize(F);
     const double two_pi = 6.283185307179586476925286766559;
     for (int k = 0; k < F; ++k) {
@@ -342,6 +350,20 @@ static cudaError_t launch_rf_groups(const OsJob *jobs, const std::vector<RfGroup
     return cudaSuccess;
 }
 
+// The operators of m folded substeps (vfd_band.h): one device allocation.
+struct BandPlan {
+    int m = 0;
+    unsigned char *d = nullptr;
+    size_t bytes = 0;
+    std::vector<BandJob> jobs;          // [axis][field]
+    BandJob *d_jobs[3] = {nullptr, nullptr, nullptr};
+    unsigned short *d_tjob[3] = {nullptr, nullptr, nullptr};
+    BandGeom geo[3];
+    int ntiles[3] = {0, 0, 0};
+    const double *d_init = nullptr;     // [field][MS_COUNT] accounting start
+    bool affine = false;                // d_init is not all zero
+};
+
 struct vfd_world {
     int device = 0;
     int nx = 0, ny = 0, nz = 0, nf = 0;
@@ -411,6 +433,13 @@ struct vfd_world {
     float *d_upd = nullptr;          // vfd_diffuse_update_host: the fields' dChem on the device
     std::vector<OsJob> oj_host;      // [axis][nf] overlap-save jobs (host copy, reused by batches)
 
+    // banded products (vfd_band.h): the passes of a separable world unless a
+    // pinned tuning or a kernel too wide for them keeps it on the FFT passes
+    bool band = false;
+    bool fft_ready = false;          // the FFT passes' arrays are set up (build_fft)
+    int band_mmax = 0;               // most substeps one operator folds (0: not known yet)
+    std::map<int, BandPlan> band_plans;
+
     std::string err;
 };
 
@@ -457,6 +486,7 @@ static void release(vfd_world *w)
     cudaFree(w->d_C);
     cudaFree(w->d_P);
     cudaFree(w->d_upd);
+    for (auto &kv : w->band_plans) cudaFree(kv.second.d);
     for (auto &t : w->timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -554,7 +584,7 @@ static cudaError_t upload_vec(T **d, const std::vector<T> &v)
     return cudaMemcpy(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
 }
 
-static OsJob make_os_job(const vfd_world *w, int f, int a, int tile_begin)
+static OsJob make_os_job(const vfd_world *w, int f, int a, int tile_begin, bool spectrum = true)
 {
     const AxisJob aj = make_job(w, f, a, 0, 16);
     OsJob j;
@@ -586,6 +616,7 @@ static OsJob make_os_job(const vfd_world *w, int f, int a, int tile_begin)
     }
     j.mask = os_plain_staging(j) ? 0 : 1;
     os_finish_job(j);
+    if (!spectrum) return j;
     std::vector<float> h;
     gauss_spectrum(w->params[f].sigma[a], j.r, OS_N, h);
     for (int k = 0; k < OS_N; ++k) j.HH[k] = make_float2(h[k], h[k]);
@@ -594,12 +625,379 @@ static OsJob make_os_job(const vfd_world *w, int f, int a, int tile_begin)
 
 static int os_field_tiles(const OsJob &j) { return j.nouter * j.tiles_per_outer; }
 
+// ---------------------------------------------------------------------------
+// Banded products.
+// ---------------------------------------------------------------------------
+static bool band_enabled()
+{
+    static int on = -1;
+    if (on < 0) {
+        const char *e = getenv("VFD_BAND");
+        on = (e && e[0] == '0') ? 0 : 1;
+    }
+    return on == 1;
+}
+
+// Half-width of field f's operator along axis a for m = 1 .. (returned count)
+// substeps: the dropped-tail width, or the whole line when that is shorter.
+static int band_widths(const vfd_world *w, int f, int a, int mmax, int *out)
+{
+    const int n = a == 0 ? w->nx : a == 1 ? w->ny : w->nz;
+    const int whole = (std::max(n - 1, 1) + 3) / 4 * 4;
+    const vfd_field_params &p = w->params[f];
+    if (whole <= BD_HMAX) {
+        // a line of at most BD_HMAX + 1 positions fits whatever the kernel
+        for (int m = 0; m < mmax; ++m) out[m] = std::min(whole, (std::min((m + 1) * p.radius[a], whole) + 3) / 4 * 4);
+        return mmax;
+    }
+    return band_half_widths(gauss_taps(p.sigma[a], p.radius[a]).data(), p.radius[a], mmax, BD_HMAX, out);
+}
+
+// Most substeps one operator of this world can fold (0: none).
+static int band_fold_limit(const vfd_world *w, int mmax)
+{
+    int top = mmax, hw[BD_MMAX];
+    for (int f = 0; f < w->nf && top > 0; ++f)
+        for (int a = 0; a < 3; ++a) {
+            bool seen = false;  // the same kernel on another axis of a long line
+            for (int c = 0; c < a; ++c)
+                seen = seen || (w->params[f].sigma[c] == w->params[f].sigma[a] &&
+                                w->params[f].radius[c] == w->params[f].radius[a] &&
+                                (c == 0 ? w->nx : c == 1 ? w->ny : w->nz) > BD_HMAX + 1);
+            if (!seen) top = std::min(top, band_widths(w, f, a, top, hw));
+        }
+    return top;
+}
+
+// Builds the operators of m substeps on the world's own stream and waits for
+// that stream only.
+static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
+{
+    const int nf = w->nf, dims[3] = {w->nx, w->ny, w->nz};
+    P.m = m;
+    P.jobs.assign((size_t)3 * nf, BandJob());
+    std::vector<BandAxis> ax((size_t)3 * nf);
+    std::vector<BandInit> in(nf);
+    std::vector<double> taps;
+    std::vector<size_t> o_taps((size_t)3 * nf), o_img((size_t)3 * nf), o_rho((size_t)3 * nf),
+        o_fn((size_t)3 * nf), o_aff((size_t)3 * nf);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off = (off + bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    int max_rows = 0, hw[BD_MMAX];
+    for (int a = 0; a < 3; ++a) {
+        int tile0 = 0;
+        for (int f = 0; f < nf; ++f) {
+            const int i = a * nf + f;
+            BandJob &J = P.jobs[i];
+            BandAxis &X = ax[i];
+            const vfd_field_params &p = w->params[f];
+            const AxisJob A = make_job(w, f, a, 0, 16);
+            memset(&J, 0, sizeof(J));
+            memset(&X, 0, sizeof(X));
+            if (band_widths(w, f, a, m, hw) < m) return cudaErrorInvalidConfiguration;
+            const int n = dims[a], H = hw[m - 1];
+            J.data = A.data;
+            J.mass = A.mass;
+            J.kind = a;
+            J.n = n;
+            J.H = H;
+            J.ksteps = (BD_BLK + 2 * H + 15) / 16;
+            J.nb = (n + BD_BLK - 1) / BD_BLK;
+            J.nin = (n + H + BD_BLK - 1) / BD_BLK;
+            J.nlines = (int)(w->V / n);
+            J.ntiles = (J.nlines + BD_LINES - 1) / BD_LINES;
+            J.tile0 = tile0;
+            tile0 += J.ntiles;
+            J.n0 = a == PASS_X ? 1 : a == PASS_Y ? w->nx : w->nx * w->ny;
+            J.outer_stride = a == PASS_Y ? A.outer_stride : 0;
+            J.pos_stride = A.pos_stride;
+            J.vec = (a == PASS_Z ? (int64_t)w->nx * w->ny : (int64_t)w->nx) % 4 == 0;
+            J.nx = w->nx;
+            J.ny = w->ny;
+            J.b = A.b;
+            J.keep = A.keep;
+            J.sums = 1;
+            J.mask = a == PASS_X && w->pad_mode == VFD_PAD_CONSTANT_VF;
+            for (int c = 0; c < 3; ++c) {
+                J.box_lo[c] = A.box_lo[c];
+                J.box_hi[c] = A.box_hi[c];
+            }
+            const double keep = 1.0 - p.decay_rate;
+            const double fold = a == PASS_X ? std::pow(keep, m - 1) : 1.0;
+            J.fscale = (float)fold;
+            const int naff = A.b != 0.0f ? m - 1 : 0;
+            const int lo = A.box_lo[a], hi = std::max(A.box_hi[a], A.box_lo[a]);
+            // one image for the blocks that see no boundary (adjacent ones), one
+            // for each other block
+            for (int b = 0; b < J.nb; ++b) {
+                const bool in_ = BD_BLK * b - H >= lo && BD_BLK * b + BD_BLK - 1 + H < hi;
+                if (in_ && J.b1 == J.b0) J.b0 = b;
+                if (in_) J.b1 = b + 1;
+                if (!in_ || J.b1 == J.b0 + 1) X.blk[X.nimg++] = b;
+            }
+            if (J.b1 == J.b0) J.b0 = J.b1 = J.nb;
+            for (int k = 0; k < J.nin; ++k)
+                if (BD_BLK * k - H >= lo + H && BD_BLK * k + BD_BLK - 1 - H < hi - H) J.plain |= 1ull << k;
+            X.n = n;
+            X.r = p.radius[a];
+            X.m = m;
+            X.H = H;
+            X.ksteps = J.ksteps;
+            X.nin = J.nin;
+            X.lo = lo;
+            X.hi = hi;
+            X.scale = X.fscale = fold;
+            X.naff = naff;
+            X.affs = J.nb * BD_BLK;
+            max_rows = std::max(max_rows, X.nimg * BD_BLK);
+            P.geo[a].ksteps = std::max(P.geo[a].ksteps, J.ksteps);
+            const std::vector<double> g = gauss_taps(p.sigma[a], p.radius[a]);
+            o_taps[i] = taps.size();
+            taps.insert(taps.end(), g.begin(), g.end());
+            o_img[i] = take((size_t)X.nimg * J.ksteps * BD_STEP_BYTES);
+            o_rho[i] = take(sizeof(float) * X.nimg * BD_BLK);
+            o_fn[i] = take(sizeof(float) * 2 * J.nin * BD_BLK);
+            o_aff[i] = take(sizeof(float) * (size_t)naff * X.affs);
+        }
+        P.ntiles[a] = tile0;
+    }
+    // staged on the host and copied in one piece: jobs, axes, accounting starts, taps
+    const size_t o_init = take(sizeof(double) * MS_COUNT * nf), o_dots = take(sizeof(double) * 3 * BD_MMAX * 3 * nf),
+                 o_affc = take(sizeof(float) * BD_MMAX * nf);
+    const size_t o_host = off;
+    const size_t o_jobs = take(sizeof(BandJob) * P.jobs.size()), o_axes = take(sizeof(BandAxis) * ax.size()),
+                 o_in = take(sizeof(BandInit) * nf), o_tp = take(sizeof(double) * taps.size());
+    const size_t o_maps = take(sizeof(CUtensorMap) * P.jobs.size());
+    size_t o_tj[3];
+    for (int a = 0; a < 3; ++a) o_tj[a] = take(sizeof(unsigned short) * P.ntiles[a]);
+    cudaError_t e = cudaMalloc(&P.d, off);
+    if (e != cudaSuccess) {
+        P.d = nullptr;
+        return e;
+    }
+    P.bytes = off;
+    unsigned char *d = P.d;
+    double *dots = reinterpret_cast<double *>(d + o_dots);
+    for (int f = 0; f < nf; ++f) {
+        for (int a = 0; a < 3; ++a) {
+            const int i = a * nf + f;
+            BandJob &J = P.jobs[i];
+            BandAxis &X = ax[i];
+            X.taps = reinterpret_cast<double *>(d + o_tp) + o_taps[i];
+            J.img = X.img = d + o_img[i];
+            J.rho = X.rho = reinterpret_cast<float *>(d + o_rho[i]);
+            J.fn = X.fn = reinterpret_cast<float *>(d + o_fn[i]);
+            X.aff = reinterpret_cast<float *>(d + o_aff[i]);
+            X.dots = dots + (size_t)i * 3 * BD_MMAX;
+            in[f].dots[a] = X.dots;
+        }
+        in[f].out = reinterpret_cast<double *>(d + o_init) + (size_t)f * MS_COUNT;
+        in[f].affc = reinterpret_cast<float *>(d + o_affc) + (size_t)f * BD_MMAX;
+        in[f].naff = ax[f].naff;
+        in[f].keep = 1.0 - w->params[f].decay_rate;
+        in[f].c = (in[f].keep - 1.0) * (double)P.jobs[f].b;
+        P.affine = P.affine || in[f].naff > 0;
+        BandJob &JX = P.jobs[f], &JY = P.jobs[nf + f], &JZ = P.jobs[2 * nf + f];
+        JX.lw1 = JY.fn + JY.H;
+        JX.lw2 = JY.lw2 = JZ.fn + JZ.H;
+        JZ.naff = in[f].naff;
+        JZ.affc = in[f].affc;
+        for (int a = 0; a < 3; ++a) {
+            JZ.aff[a] = ax[a * nf + f].aff;
+            JZ.affs[a] = ax[a * nf + f].affs;
+        }
+    }
+    P.d_init = reinterpret_cast<double *>(d + o_init);
+    for (int a = 0; a < 3; ++a) P.d_jobs[a] = reinterpret_cast<BandJob *>(d + o_jobs) + (size_t)a * nf;
+    std::vector<CUtensorMap> maps(P.jobs.size());
+    for (size_t i = 0; i < maps.size(); ++i)
+        P.jobs[i].map = band_encode_map(P.jobs[i], w->nz, &maps[i]) ? reinterpret_cast<CUtensorMap *>(d + o_maps) + i
+                                                                    : nullptr;
+    std::vector<unsigned char> host(off - o_host);
+    memcpy(host.data() + (o_maps - o_host), maps.data(), sizeof(CUtensorMap) * maps.size());
+    memcpy(host.data() + (o_jobs - o_host), P.jobs.data(), sizeof(BandJob) * P.jobs.size());
+    memcpy(host.data() + (o_axes - o_host), ax.data(), sizeof(BandAxis) * ax.size());
+    memcpy(host.data() + (o_in - o_host), in.data(), sizeof(BandInit) * nf);
+    memcpy(host.data() + (o_tp - o_host), taps.data(), sizeof(double) * taps.size());
+    for (int a = 0; a < 3; ++a) {
+        P.d_tjob[a] = reinterpret_cast<unsigned short *>(d + o_tj[a]);
+        unsigned short *t = reinterpret_cast<unsigned short *>(host.data() + (o_tj[a] - o_host));
+        for (int f = 0; f < nf; ++f) t = std::fill_n(t, P.jobs[(size_t)a * nf + f].ntiles, (unsigned short)f);
+    }
+    if ((e = cudaMemcpyAsync(d + o_host, host.data(), host.size(), cudaMemcpyHostToDevice, w->s_in)) == cudaSuccess &&
+        (e = launch_band_setup(reinterpret_cast<BandAxis *>(d + o_axes), 3 * nf, max_rows,
+                               reinterpret_cast<BandInit *>(d + o_in), nf, w->s_in)) == cudaSuccess)
+        e = cudaStreamSynchronize(w->s_in);
+    if (e != cudaSuccess) {
+        cudaFree(P.d);
+        P.d = nullptr;
+    }
+    return e;
+}
+
+// The plan of m substeps, built on first use.
+static cudaError_t band_plan(vfd_world *w, int m, const BandPlan **out)
+{
+    auto it = w->band_plans.find(m);
+    if (it == w->band_plans.end()) {
+        BandPlan P;
+        cudaError_t e = build_band_plan(w, m, P);
+        if (e != cudaSuccess) return e;
+        it = w->band_plans.emplace(m, std::move(P)).first;
+    }
+    *out = &it->second;
+    return cudaSuccess;
+}
+
+static bool stream_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// The sizes of the groups a tick's substeps are folded into: as few as
+// `limit` substeps a group allow, of sizes that differ by one at most.
+static std::vector<int> band_groups(int n_substeps, int limit)
+{
+    const int g = (n_substeps + limit - 1) / limit, base = n_substeps / g, rem = n_substeps % g;
+    std::vector<int> out(g, base);
+    for (int i = 0; i < rem; ++i) ++out[i];
+    return out;
+}
+
+// Whether a tick runs on the banded products.  From two substeps on they are
+// three passes over the fields instead of three a substep.  A single substep
+// of worlds that take the register-FFT pass on every axis (radius <= 8) stays
+// on it when the kernels are narrow and the fields not small: a banded pass
+// takes the same time at every radius up to 8, an FFT pass's blocks give 64 -
+// 2r outputs.  Measured, 8 fields, one substep, banded / FFT (us): mean radius
+// 3.5: 64x64x32 35 / 46, 96x64x64 54 / 58, 128x96x96 95 / 85, 256x128x192 309 /
+// 304, 512x256x256 1236 / 1168; mean radius 5.1: 512x256x384 2094 / 2067; mean
+// radius 6.5: 35 / 46, 53 / 68, 96 / 116, 307 / 378, 1226 / 1318.
+constexpr int64_t BAND_SMALL = (int64_t)4 << 20;  // voxels x fields
+static bool runs_band(const vfd_world *w, int n_substeps)
+{
+    if (!w->band) return false;
+    if (n_substeps > 1 || !(w->use_rf[0] && w->use_rf[1] && w->use_rf[2]) || w->V * w->nf <= BAND_SMALL) return true;
+    int radii = 0;
+    for (int f = 0; f < w->nf; ++f)
+        for (int a = 0; a < 3; ++a) radii += w->params[f].radius[a];
+    return 2 * radii > 11 * 3 * w->nf;  // mean radius above 5.5
+}
+
+// What band_groups may fold for a tick of this world.  Operators that are
+// not built yet cannot be while `st` is being captured: then the
+// single-substep ones, which every world has, run the tick.
+static int band_limit(vfd_world *w, int n_substeps, cudaStream_t st)
+{
+    if (n_substeps == 1) return 1;
+    if (w->band_mmax == 0) w->band_mmax = band_fold_limit(w, BD_MMAX);
+    if (stream_capturing(st))
+        for (int m : band_groups(n_substeps, w->band_mmax))
+            if (!w->band_plans.count(m)) return 1;
+    return w->band_mmax;
+}
+
 // True when the pass stages samples unchanged (no padding-rule transform).
 static bool os_plain_staging(const OsJob &j)
 {
     if (j.kind != PASS_X) return true;
     return j.b == 0.0f && j.box_lo[0] == 0 && j.box_hi[0] == j.nx && j.box_lo[1] == 0 && j.box_hi[1] == j.ny &&
            j.box_lo[2] == 0 && j.box_hi[2] == j.nlines / j.ny;
+}
+
+// The twiddles and per-axis spectra of a world's FFT lengths.
+static cudaError_t build_axis_tables(vfd_world *w)
+{
+    cudaError_t e;
+    for (int a = 0; a < 3; ++a) {
+        std::vector<float2> tw;
+        twiddles(w->F[a], tw);
+        if ((e = cudaMalloc(&w->d_tw[a], sizeof(float2) * w->F[a])) != cudaSuccess) return e;
+        if ((e = cudaMemcpy(w->d_tw[a], tw.data(), sizeof(float2) * w->F[a], cudaMemcpyHostToDevice)) != cudaSuccess)
+            return e;
+    }
+    {
+        std::vector<float> spec((size_t)w->nf * 3 * w->Fmax, 0.0f), tmp;
+        for (int f = 0; f < w->nf; ++f)
+            for (int a = 0; a < 3; ++a) {
+                gauss_spectrum(w->params[f].sigma[a], w->params[f].radius[a], w->F[a], tmp);
+                std::copy(tmp.begin(), tmp.end(), spec.begin() + ((size_t)f * 3 + a) * w->Fmax);
+            }
+        if ((e = cudaMalloc(&w->d_spec, sizeof(float) * spec.size())) != cudaSuccess) return e;
+        if ((e = cudaMemcpy(w->d_spec, spec.data(), sizeof(float) * spec.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
+// What the FFT passes of a separable world need: tables, jobs and tiles of
+// every pass it may take.  Worlds whose ticks run on banded products build
+// it only when a batch with other worlds needs it.
+static cudaError_t build_fft(vfd_world *w)
+{
+    if (w->fft_ready) return cudaSuccess;
+    cudaError_t e;
+    if ((e = build_axis_tables(w)) != cudaSuccess) return e;
+    {
+        std::vector<AxisJob> jobs;
+        for (int a = 0; a < 3; ++a) {
+            int tb = 0;
+            for (int f = 0; f < w->nf; ++f) {
+                jobs.push_back(make_job(w, f, a, tb, kAxisVariants[w->variant[a]].nl));
+                tb += w->tiles_per_field[a];
+            }
+        }
+        for (int a = 0; a < 3; ++a)
+            for (int f = 0; f < w->nf; ++f) jobs.push_back(make_job(w, f, a, 0, kAxisVariants[w->variant[a]].nl));
+        if ((e = cudaMalloc(&w->d_jobs, sizeof(AxisJob) * jobs.size())) != cudaSuccess) return e;
+        if ((e = cudaMemcpy(w->d_jobs, jobs.data(), sizeof(AxisJob) * jobs.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+            return e;
+    }
+    if (w->use_os[0] || w->use_os[1] || w->use_os[2]) {
+        std::vector<OsJob> oj;
+        for (int a = 0; a < 3; ++a) {
+            int tb = 0;
+            w->os_tiles[a].assign(w->nf, 0);
+            for (int f = 0; f < w->nf; ++f) {
+                oj.push_back(make_os_job(w, f, a, tb));
+                w->os_tiles[a][f] = os_field_tiles(oj.back());
+                tb += w->os_tiles[a][f];
+            }
+        }
+        w->oj_host.assign(oj.begin(), oj.end());
+        for (int a = 0; a < 3; ++a)
+            for (int f = 0; f < w->nf; ++f) oj.push_back(make_os_job(w, f, a, 0));
+        if ((e = os_prepare()) != cudaSuccess) return e;
+        if ((e = cudaMalloc(&w->d_osjobs, sizeof(OsJob) * oj.size())) != cudaSuccess) return e;
+        if ((e = cudaMemcpy(w->d_osjobs, oj.data(), sizeof(OsJob) * oj.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+            return e;
+        for (int a = 0; a < 3; ++a) {
+            std::vector<OsTileInfo> all, one;
+            for (int f = 0; f < w->nf; ++f) {
+                os_append_tiles(oj[(size_t)a * w->nf + f], f, all);
+                os_append_tiles(oj[(size_t)(3 + a) * w->nf + f], 0, one);
+            }
+            if ((e = upload_vec(&w->d_os_tiles[a], all)) != cudaSuccess ||
+                (e = upload_vec(&w->d_os_ftiles[a], one)) != cudaSuccess)
+                return e;
+        }
+        for (int a = 0; a < 3; ++a) {
+            if (!w->use_rf[a]) continue;
+            if ((e = rf_prepare()) != cudaSuccess) return e;
+            if ((e = build_rf_groups(&oj[(size_t)a * w->nf], w->nf, w->rf[a])) != cudaSuccess) return e;
+            w->rf_field[a].resize(w->nf);
+            for (int f = 0; f < w->nf; ++f)
+                if ((e = build_rf_groups(&oj[(size_t)(3 + a) * w->nf + f], 1, w->rf_field[a][f])) != cudaSuccess)
+                    return e;
+        }
+    }
+    w->fft_ready = true;
+    return cudaSuccess;
 }
 
 extern "C" {
@@ -645,6 +1043,7 @@ struct AxisChoice {
 };
 struct ShapeChoice {
     AxisChoice ax[3];
+    bool pinned = false;  // the FFT passes of ax run whatever else would (vfd_autotune_set, timing)
 };
 
 static std::mutex g_tune_mu;
@@ -836,84 +1235,11 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
     if ((e = cudaSetDevice(device)) != cudaSuccess) return bail(e, "cudaSetDevice");
     if ((e = cudaMalloc(&w->d_fields, sizeof(float) * w->V * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc fields");
     if ((e = cudaMemset(w->d_fields, 0, sizeof(float) * w->V * w->nf)) != cudaSuccess) return bail(e, "cudaMemset fields");
-    for (int a = 0; a < 3; ++a) {
-        std::vector<float2> tw;
-        twiddles(w->F[a], tw);
-        if ((e = cudaMalloc(&w->d_tw[a], sizeof(float2) * w->F[a])) != cudaSuccess) return bail(e, "cudaMalloc twiddles");
-        if ((e = cudaMemcpy(w->d_tw[a], tw.data(), sizeof(float2) * w->F[a], cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(e, "cudaMemcpy twiddles");
-    }
-    {
-        std::vector<float> spec((size_t)w->nf * 3 * w->Fmax, 0.0f), tmp;
-        for (int f = 0; f < w->nf; ++f)
-            for (int a = 0; a < 3; ++a) {
-                gauss_spectrum(w->params[f].sigma[a], w->params[f].radius[a], w->F[a], tmp);
-                std::copy(tmp.begin(), tmp.end(), spec.begin() + ((size_t)f * 3 + a) * w->Fmax);
-            }
-        if ((e = cudaMalloc(&w->d_spec, sizeof(float) * spec.size())) != cudaSuccess) return bail(e, "cudaMalloc spectra");
-        if ((e = cudaMemcpy(w->d_spec, spec.data(), sizeof(float) * spec.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(e, "cudaMemcpy spectra");
-    }
+    if (general && (e = build_axis_tables(w)) != cudaSuccess) return bail(e, "twiddles and spectra");
     if ((e = cudaMalloc(&w->d_mass, sizeof(double) * MS_COUNT * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc mass");
     if ((e = cudaMemset(w->d_mass, 0, sizeof(double) * MS_COUNT * w->nf)) != cudaSuccess) return bail(e, "cudaMemset mass");
     if ((e = cudaMalloc(&w->d_err, sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc err");
     if ((e = cudaMemset(w->d_err, 0, sizeof(int))) != cudaSuccess) return bail(e, "cudaMemset err");
-    {
-        std::vector<AxisJob> jobs;
-        for (int a = 0; a < 3; ++a) {
-            int tb = 0;
-            for (int f = 0; f < w->nf; ++f) {
-                jobs.push_back(make_job(w, f, a, tb, kAxisVariants[w->variant[a]].nl));
-                tb += w->tiles_per_field[a];
-            }
-        }
-        for (int a = 0; a < 3; ++a)
-            for (int f = 0; f < w->nf; ++f) jobs.push_back(make_job(w, f, a, 0, kAxisVariants[w->variant[a]].nl));
-        if ((e = cudaMalloc(&w->d_jobs, sizeof(AxisJob) * jobs.size())) != cudaSuccess) return bail(e, "cudaMalloc jobs");
-        if ((e = cudaMemcpy(w->d_jobs, jobs.data(), sizeof(AxisJob) * jobs.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(e, "cudaMemcpy jobs");
-    }
-    if (w->use_os[0] || w->use_os[1] || w->use_os[2]) {
-        std::vector<OsJob> oj;
-        for (int a = 0; a < 3; ++a) {
-            int tb = 0;
-            w->os_tiles[a].assign(w->nf, 0);
-            for (int f = 0; f < w->nf; ++f) {
-                oj.push_back(make_os_job(w, f, a, tb));
-                w->os_tiles[a][f] = os_field_tiles(oj.back());
-                tb += w->os_tiles[a][f];
-            }
-        }
-        w->oj_host.assign(oj.begin(), oj.end());
-        for (int a = 0; a < 3; ++a)
-            for (int f = 0; f < w->nf; ++f) oj.push_back(make_os_job(w, f, a, 0));
-        if ((e = os_prepare()) != cudaSuccess) return bail(e, "overlap-save twiddles");
-        if ((e = cudaMalloc(&w->d_osjobs, sizeof(OsJob) * oj.size())) != cudaSuccess) return bail(e, "cudaMalloc os jobs");
-        if ((e = cudaMemcpy(w->d_osjobs, oj.data(), sizeof(OsJob) * oj.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(e, "cudaMemcpy os jobs");
-        for (int a = 0; a < 3; ++a) {
-            std::vector<OsTileInfo> all, one;
-            for (int f = 0; f < w->nf; ++f) {
-                os_append_tiles(oj[(size_t)a * w->nf + f], f, all);
-                os_append_tiles(oj[(size_t)(3 + a) * w->nf + f], 0, one);
-            }
-            if ((e = upload_vec(&w->d_os_tiles[a], all)) != cudaSuccess ||
-                (e = upload_vec(&w->d_os_ftiles[a], one)) != cudaSuccess)
-                return bail(e, "os tiles");
-        }
-        for (int a = 0; a < 3 && rf_enabled(); ++a) {
-            bool ok = w->use_os[a] && w->allow_rf[a];
-            for (int f = 0; f < w->nf; ++f) ok = ok && rf_eligible(oj[(size_t)a * w->nf + f]);
-            if (!ok) continue;
-            if ((e = rf_prepare()) != cudaSuccess) return bail(e, "register-FFT twiddles");
-            if ((e = build_rf_groups(&oj[(size_t)a * w->nf], w->nf, w->rf[a])) != cudaSuccess) return bail(e, "rf tiles");
-            w->rf_field[a].resize(w->nf);
-            for (int f = 0; f < w->nf; ++f)
-                if ((e = build_rf_groups(&oj[(size_t)(3 + a) * w->nf + f], 1, w->rf_field[a][f])) != cudaSuccess)
-                    return bail(e, "rf tiles");
-            w->use_rf[a] = true;
-        }
-    }
     if ((e = cudaMalloc(&w->d_dep, sizeof(DepositJob) * 2 * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc deposit jobs");
     if (general) {
         const int64_t nk = (int64_t)w->Fxh * w->F[1] * w->F[2];
@@ -933,6 +1259,19 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         }
     }
     if ((e = cudaStreamCreateWithFlags(&w->s_in, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
+    if (!general) {
+        for (int a = 0; a < 3 && rf_enabled(); ++a) {
+            bool ok = w->use_os[a] && w->allow_rf[a];
+            for (int f = 0; f < w->nf && ok; ++f) ok = rf_eligible(make_os_job(w, f, a, 0, false));
+            w->use_rf[a] = ok;
+        }
+        if (band_enabled() && !(ch && ch->pinned) && band_fold_limit(w, 1) >= 1) {
+            const BandPlan *P = nullptr;
+            if ((e = band_plan(w, 1, &P)) != cudaSuccess) return bail(e, "banded operators");
+            w->band = true;
+        }
+        if (!runs_band(w, 1) && (e = build_fft(w)) != cudaSuccess) return bail(e, "FFT passes");
+    }
     if ((e = cudaStreamCreateWithFlags(&w->s_cmp, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
     if ((e = cudaStreamCreateWithFlags(&w->s_out, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
     w->ev_in.resize(w->nf);
@@ -976,6 +1315,7 @@ vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes)
     b += sizeof(float) * (size_t)w->nf * 3 * w->Fmax + sizeof(double) * MS_COUNT * w->nf;
     b += sizeof(AxisJob) * 6 * w->nf + sizeof(DepositJob) * 2 * w->nf;
     b += (sizeof(int32_t) + sizeof(float)) * (size_t)w->src_cap;
+    for (const auto &kv : w->band_plans) b += kv.second.bytes;
     if (w->method != VFD_METHOD_SEPARABLE) {
         const size_t nk = (size_t)w->Fxh * w->F[1] * w->F[2];
         b += sizeof(float2) * nk * w->nf;
@@ -1562,6 +1902,25 @@ static vfd_status enqueue_axis(vfd_world *w, int a, int field, cudaStream_t st)
     return VFD_OK;
 }
 
+// n_substeps on the FFT passes of a separable world.
+static vfd_status enqueue_fft_substeps(vfd_world *w, int field, int n_substeps, cudaStream_t st)
+{
+    VFD_CUDA(w, build_fft(w));
+    for (int s = 0; s < n_substeps; ++s) {
+        if (field < 0)
+            VFD_CUDA(w, cudaMemsetAsync(w->d_mass, 0, sizeof(double) * MS_COUNT * w->nf, st));
+        else
+            VFD_CUDA(w, cudaMemsetAsync(w->d_mass + (int64_t)field * MS_COUNT, 0, sizeof(double) * MS_COUNT, st));
+        for (int a = 0; a < 3; ++a) {
+            LaunchTimer lt(w, a, st);
+            vfd_status r = enqueue_axis(w, a, field, st);
+            if (r != VFD_OK) return r;
+            lt.done();
+        }
+    }
+    return VFD_OK;
+}
+
 static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStream_t st,
                                const UpdateArgs *upd = nullptr)
 {
@@ -1583,17 +1942,32 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
         }
         return VFD_OK;
     }
-    for (int s = 0; s < n_substeps; ++s) {
-        if (field < 0)
-            VFD_CUDA(w, cudaMemsetAsync(w->d_mass, 0, sizeof(double) * MS_COUNT * w->nf, st));
-        else
-            VFD_CUDA(w, cudaMemsetAsync(w->d_mass + (int64_t)field * MS_COUNT, 0, sizeof(double) * MS_COUNT, st));
-        for (int a = 0; a < 3; ++a) {
-            LaunchTimer lt(w, a, st);
-            vfd_status r = enqueue_axis(w, a, field, st);
-            if (r != VFD_OK) return r;
-            lt.done();
+    const bool band = runs_band(w, n_substeps);
+    if (band) {
+        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps, st));
+        double *mass = w->d_mass + (field < 0 ? 0 : (int64_t)field * MS_COUNT);
+        const size_t mbytes = sizeof(double) * MS_COUNT * (field < 0 ? w->nf : 1);
+        for (size_t g = 0; g < groups.size(); ++g) {
+            const BandPlan *P = nullptr;
+            VFD_CUDA(w, band_plan(w, groups[g], &P));
+            const bool last = g + 1 == groups.size();  // the accounting is the last group's
+            if (last && P->affine)
+                VFD_CUDA(w, cudaMemcpyAsync(mass, P->d_init + (field < 0 ? 0 : (int64_t)field * MS_COUNT), mbytes,
+                                            cudaMemcpyDeviceToDevice, st));
+            else if (last)
+                VFD_CUDA(w, cudaMemsetAsync(mass, 0, mbytes, st));
+            for (int a = 0; a < 3; ++a) {
+                LaunchTimer lt(w, a, st);
+                const BandJob *J = field < 0 ? nullptr : &P->jobs[(size_t)a * w->nf + field];
+                VFD_CUDA(w, launch_band(P->d_jobs[a], P->d_tjob[a], J ? J->tile0 : 0, J ? J->ntiles : P->ntiles[a], a,
+                                        P->geo[a], last, st));
+                lt.done();
+            }
         }
+    }
+    if (!band) {
+        const vfd_status r = enqueue_fft_substeps(w, field, n_substeps, st);
+        if (r != VFD_OK) return r;
     }
     if (upd) {
         // the update as one pass per field after the z pass (whose output
@@ -1677,7 +2051,8 @@ vfd_status vfd_read_mass(vfd_world *w, vfd_mass *out, void *stream)
         out[f].reserved = 0.0;
     }
     if (herr) return fail(w, VFD_ERR_DEVICE_FAULT, "a kernel rejected an out-of-range index");
-    if (rf_take_timeout()) return fail(w, VFD_ERR_TIMEOUT, "an axis pass gave up waiting for a bulk copy");
+    if (rf_take_timeout() || band_take_timeout())
+        return fail(w, VFD_ERR_TIMEOUT, "an axis pass gave up waiting for a bulk copy");
     return VFD_OK;
 }
 
@@ -1756,9 +2131,10 @@ struct TuneRun {
     bool have[3] = {false, false, false};
 };
 
-static vfd_status tune_candidate(TuneRun &T, const ShapeChoice &proto, const bool *axes)
+static vfd_status tune_candidate(TuneRun &T, ShapeChoice proto, const bool *axes)
 {
     vfd_world *w = nullptr;
+    proto.pinned = true;
     vfd_status s = world_create(T.d, T.device, &proto, &w);
     if (s == VFD_ERR_NOT_SUPPORTED || s == VFD_ERR_OUT_OF_MEMORY) return VFD_OK;  // candidate does not fit
     if (s != VFD_OK) return s;
@@ -1917,6 +2293,7 @@ vfd_status vfd_autotune_set(const vfd_world_desc *desc, int device, const vfd_ax
         return fail(nullptr, VFD_ERR_NOT_SUPPORTED, "tunings cover VFD_METHOD_SEPARABLE worlds");
     const int dims[3] = {desc->nx, desc->ny, desc->nz};
     ShapeChoice ch;
+    ch.pinned = true;
     for (int a = 0; a < 3; ++a) {
         const vfd_axis_tuning &t = in3[a];
         AxisChoice &c = ch.ax[a];
@@ -2078,7 +2455,34 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
 // ---------------------------------------------------------------------------
 }  // extern "C"
 
+// The banded passes of a batch's tick of some number of substeps: each world
+// goes through its own groups of folded substeps, launch g holding every
+// world's group g.
+struct BatchBand {
+    struct Launch {
+        BandJob *d_jobs[3] = {nullptr, nullptr, nullptr};
+        unsigned short *d_tjob[3] = {nullptr, nullptr, nullptr};
+        BandGeom geo[3];
+        int ntiles[3] = {0, 0, 0};
+    };
+    unsigned char *d = nullptr;  // arena
+    std::vector<Launch> launches;
+    std::vector<std::pair<vfd_world *, const double *>> affine;  // accounting starts that are not zero
+};
+constexpr size_t BATCH_BANDS = 4;  // substep counts whose arrays a batch keeps
+
+// A world's tick runs on banded products or on FFT passes whatever else is in
+// the batch (a request's result does not depend on its neighbours): a batch
+// launches each axis pass for the worlds of either kind.
 struct vfd_batch {
+    std::map<int, BatchBand> bands;                   // by a tick's substeps
+    std::vector<vfd_world *> fft_worlds;              // the worlds whose FFT passes the arrays below hold
+    bool fft_ready = false;
+    bool fft_each = false;                            // they take different passes: each world launches its own
+    int tuned_method[3] = {PASS_METHOD_AUTO, PASS_METHOD_AUTO, PASS_METHOD_AUTO};
+    unsigned char *d_fft_arena = nullptr;
+    double **d_fft_mass_ptrs = nullptr;               // their accounting blocks
+    int *d_fft_mass_counts = nullptr;
     int device = 0;
     std::vector<vfd_world *> worlds;
     int variant[3] = {0, 0, 0};
@@ -2211,6 +2615,8 @@ static void batch_release(vfd_batch *b)
     // complete when it is destroyed)
     if (b->d_arena) cudaStreamSynchronize(b->st);
     give_arena(b->device, b->d_arena);
+    give_arena(b->device, b->d_fft_arena);
+    for (auto &kv : b->bands) give_arena(b->device, kv.second.d);
     bool kept = false;
     if (b->st && b->ev_in && b->ev_out && b->device >= 0 && b->device < 64) {
         const unsigned long long c = current_context_id();
@@ -2235,7 +2641,7 @@ extern "C" {
 static bool batch_rf_possible(const vfd_batch *b, const std::vector<OsJob> &oj, int a)
 {
     if (!rf_enabled() || !b->use_os[a]) return false;
-    for (auto *w : b->worlds)
+    for (auto *w : b->fft_worlds)
         if (!w->allow_rf[a]) return false;
     for (int i = 0; i < b->njobs; ++i)
         if (!rf_eligible(oj[(size_t)a * b->njobs + i])) return false;
@@ -2267,6 +2673,16 @@ static cudaError_t take_stream(vfd_batch *b)
     return cudaSuccess;
 }
 
+// The worlds whose ticks of n_substeps run on FFT passes.
+static std::vector<vfd_world *> batch_fft_worlds(const vfd_batch *b, int n_substeps)
+{
+    std::vector<vfd_world *> out;
+    for (auto *w : b->worlds)
+        if (!runs_band(w, n_substeps)) out.push_back(w);
+    return out;
+}
+static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *> &ws);
+
 vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **out)
 {
     if (!out) return bfail(nullptr, VFD_ERR_INVALID_ARG, "out is NULL");
@@ -2294,20 +2710,12 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
             return bfail(nullptr, VFD_ERR_NOT_SUPPORTED, "no kernel variant fits every world's FFT plan");
         }
     }
-    std::vector<AxisJob> jobs;
-    for (int a = 0; a < 3; ++a) {
-        const int nl = kAxisVariants[b->variant[a]].nl;
-        int tb = 0;
-        for (auto *w : b->worlds)
-            for (int f = 0; f < w->nf; ++f) {
-                jobs.push_back(make_job(w, f, a, tb, nl));
-                tb += field_tiles(w, a, nl);
-            }
-        b->tiles[a] = tb;
+    int64_t njobs = 0;
+    for (auto *w : b->worlds) njobs += w->nf;
+    if (njobs > 65535) {
+        delete b;
+        return bfail(nullptr, VFD_ERR_NOT_SUPPORTED, "more than 65535 fields in a batch");
     }
-    b->njobs = (int)jobs.size() / 3;
-    std::vector<OsJob> oj;
-    std::vector<OsTileInfo> tile_info[3];
     for (int a = 0; a < 3; ++a) {
         bool all = true;
         int rmn = 1 << 30;
@@ -2322,10 +2730,93 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
         for (auto *w : b->worlds)
             if (w->os_minb[a] != b->os_minb[a]) b->os_minb[a] = 0;
     }
+    std::vector<double *> mp;
+    std::vector<int> mc;
+    for (auto *w : b->worlds) {
+        mp.push_back(w->d_mass);
+        mc.push_back(MS_COUNT * w->nf);
+    }
+    ArenaBuilder ar;
+    const size_t o_mp = ar.add(mp.data(), sizeof(double *) * mp.size());
+    const size_t o_mc = ar.add(mc.data(), sizeof(int) * mc.size());
+    DeviceGuard g(b->device);
+    cudaError_t e = cudaSuccess;
+    if ((e = take_arena(b->device, ar.host.size(), &b->d_arena)) != cudaSuccess ||
+        (e = cudaMemcpy(b->d_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
+        (e = take_stream(b)) != cudaSuccess) {
+        std::string msg = std::string("batch setup: ") + cudaGetErrorString(e);
+        batch_release(b);
+        delete b;
+        return bfail(nullptr, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA, msg);
+    }
+    b->d_mass_ptrs = reinterpret_cast<double **>(b->d_arena + o_mp);
+    b->d_mass_counts = reinterpret_cast<int *>(b->d_arena + o_mc);
+    b->gens.assign(n_worlds, ~0ull);
+    // the FFT passes of single-substep ticks: set up now rather than in the first
+    const vfd_status st = batch_prepare_fft(b, batch_fft_worlds(b, 1));
+    if (st != VFD_OK) {
+        const std::string msg = b->err;
+        batch_release(b);
+        delete b;
+        return bfail(nullptr, st, msg);
+    }
+    *out = b;
+    return VFD_OK;
+}
+
+// The arrays of the FFT passes, set up when a tick or the tuner needs them (a
+// server rebuilds its batch whenever the active set changes, and its batches
+// may never need them).
+static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *> &ws)
+{
+    if (b->fft_ready && ws == b->fft_worlds) return VFD_OK;
+    if (b->fft_ready) {
+        // another set of worlds than the arrays hold
+        VFD_BCUDA(b, cudaStreamSynchronize(b->st));
+        for (int a = 0; a < 3; ++a) {
+            if (b->os_tiles_owned[a]) cudaFree(b->d_os_tiles[a]);
+            b->d_os_tiles[a] = nullptr;
+            b->os_tiles_owned[a] = true;
+            free_rf_groups(b->rf[a]);
+            b->use_rf[a] = false;
+        }
+        give_arena(b->device, b->d_fft_arena);
+        b->d_fft_arena = nullptr;
+        b->fft_ready = false;
+    }
+    b->fft_worlds = ws;
+    b->njobs = 0;
+    for (auto *w : ws) b->njobs += w->nf;
+    if (b->njobs == 0) {
+        b->fft_ready = true;
+        return VFD_OK;
+    }
+    for (auto *w : ws) VFD_BCUDA(b, build_fft(w));
+    b->fft_each = false;
+    for (int a = 0; a < 3; ++a)
+        for (auto *w : ws)
+            if (b->tuned_method[a] == PASS_METHOD_AUTO &&
+                (w->use_rf[a] != ws[0]->use_rf[a] || w->use_os[a] != b->can_os[a]))
+                b->fft_each = true;
+    for (int a = 0; a < 3; ++a)  // a tuned axis keeps its pass
+        if (b->tuned_method[a] != PASS_METHOD_AUTO) b->use_os[a] = b->can_os[a] && b->tuned_method[a] != PASS_METHOD_FULL;
+    std::vector<AxisJob> jobs;
+    for (int a = 0; a < 3; ++a) {
+        const int nl = kAxisVariants[b->variant[a]].nl;
+        int tb = 0;
+        for (auto *w : ws)
+            for (int f = 0; f < w->nf; ++f) {
+                jobs.push_back(make_job(w, f, a, tb, nl));
+                tb += field_tiles(w, a, nl);
+            }
+        b->tiles[a] = tb;
+    }
+    std::vector<OsJob> oj;
+    std::vector<OsTileInfo> tile_info[3];
     if (b->use_os[0] || b->use_os[1] || b->use_os[2]) {
         for (int a = 0; a < 3; ++a) {
             int tb = 0;
-            for (auto *w : b->worlds)
+            for (auto *w : ws)
                 for (int f = 0; f < w->nf; ++f) {
                     if (w->oj_host.size() == (size_t)3 * w->nf) {
                         oj.push_back(w->oj_host[(size_t)a * w->nf + f]);  // the world's own job, re-based
@@ -2344,7 +2835,9 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
     // the others when it times that pass), else the full-line pass.
     RfGroupHost rfh[3];
     for (int a = 0; a < 3 && !oj.empty(); ++a) {
-        if (batch_rf_possible(b, oj, a)) {
+        const int want = b->tuned_method[a];
+        if (want == PASS_METHOD_FULL) continue;
+        if (want != PASS_METHOD_OS && batch_rf_possible(b, oj, a)) {
             rf_group_host(&oj[(size_t)a * b->njobs], b->njobs, rfh[a]);
             if (!rfh[a].tiles.empty()) continue;
         }
@@ -2353,11 +2846,13 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
     }
     std::vector<double *> mp;
     std::vector<int> mc;
-    for (auto *w : b->worlds) {
+    for (auto *w : ws) {
         mp.push_back(w->d_mass);
         mc.push_back(MS_COUNT * w->nf);
     }
     ArenaBuilder ar;
+    const size_t o_mp = ar.add(mp.data(), sizeof(double *) * mp.size());
+    const size_t o_mc = ar.add(mc.data(), sizeof(int) * mc.size());
     const size_t o_jobs = ar.add(jobs.data(), sizeof(AxisJob) * jobs.size());
     const size_t o_oj = ar.add(oj.data(), sizeof(OsJob) * oj.size());
     size_t o_ost[3], o_rft[3], o_rfm[3];
@@ -2366,21 +2861,16 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
         o_rft[a] = ar.add(rfh[a].tiles.data(), sizeof(OsTileInfo) * rfh[a].tiles.size());
         o_rfm[a] = ar.add(rfh[a].maps.data(), sizeof(CUtensorMap) * rfh[a].maps.size());
     }
-    const size_t o_mp = ar.add(mp.data(), sizeof(double *) * mp.size());
-    const size_t o_mc = ar.add(mc.data(), sizeof(int) * mc.size());
-    DeviceGuard g(b->device);
     cudaError_t e = cudaSuccess;
     if ((!oj.empty() && (e = os_prepare()) != cudaSuccess) ||
         ((rfh[0].tiles.size() + rfh[1].tiles.size() + rfh[2].tiles.size()) > 0 && (e = rf_prepare()) != cudaSuccess) ||
-        (e = take_arena(b->device, ar.host.size(), &b->d_arena)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = take_stream(b)) != cudaSuccess) {
-        std::string msg = std::string("batch setup: ") + cudaGetErrorString(e);
-        batch_release(b);
-        delete b;
-        return bfail(nullptr, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA, msg);
-    }
-    unsigned char *base = b->d_arena;
+        (e = take_arena(b->device, ar.host.size(), &b->d_fft_arena)) != cudaSuccess ||
+        (e = cudaMemcpy(b->d_fft_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
+                     std::string("batch setup: ") + cudaGetErrorString(e));
+    b->d_fft_mass_ptrs = reinterpret_cast<double **>(b->d_fft_arena + o_mp);
+    b->d_fft_mass_counts = reinterpret_cast<int *>(b->d_fft_arena + o_mc);
+    unsigned char *base = b->d_fft_arena;
     b->d_jobs = reinterpret_cast<AxisJob *>(base + o_jobs);
     b->d_osjobs = oj.empty() ? nullptr : reinterpret_cast<OsJob *>(base + o_oj);
     for (int a = 0; a < 3; ++a) {
@@ -2398,12 +2888,84 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
             b->use_rf[a] = true;
         }
     }
-    b->d_mass_ptrs = reinterpret_cast<double **>(base + o_mp);
-    b->d_mass_counts = reinterpret_cast<int *>(base + o_mc);
-    b->gens.assign(n_worlds, ~0ull);
     b->oj.swap(oj);
-    *out = b;
+    b->fft_ready = true;
     return VFD_OK;
+}
+
+// The job arrays of a tick's banded passes.
+static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
+{
+    if (b->bands.count(n_substeps)) return VFD_OK;
+    if (b->bands.size() >= BATCH_BANDS) {
+        VFD_BCUDA(b, cudaStreamSynchronize(b->st));
+        for (auto &kv : b->bands) give_arena(b->device, kv.second.d);
+        b->bands.clear();
+    }
+    BatchBand B;
+    struct Host {
+        std::vector<BandJob> jobs[3];
+        std::vector<unsigned short> tjob[3];
+        size_t o_j[3], o_t[3];
+    };
+    std::vector<Host> host;
+    for (auto *w : b->worlds) {
+        if (!runs_band(w, n_substeps)) continue;
+        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps, b->st));
+        if (host.size() < groups.size()) {
+            host.resize(groups.size());
+            B.launches.resize(groups.size());
+        }
+        for (size_t g = 0; g < groups.size(); ++g) {
+            const BandPlan *P = nullptr;
+            const cudaError_t e = band_plan(w, groups[g], &P);
+            if (e != cudaSuccess)
+                return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
+                             std::string("banded operators: ") + cudaGetErrorString(e));
+            const bool last = g + 1 == groups.size();  // the accounting is the last group's
+            for (int a = 0; a < 3; ++a) {
+                for (int f = 0; f < w->nf; ++f) {
+                    BandJob j = P->jobs[(size_t)a * w->nf + f];
+                    j.tile0 = (int)host[g].tjob[a].size();
+                    j.sums = last;
+                    host[g].tjob[a].insert(host[g].tjob[a].end(), j.ntiles, (unsigned short)host[g].jobs[a].size());
+                    host[g].jobs[a].push_back(j);
+                }
+                B.launches[g].geo[a].ksteps = std::max(B.launches[g].geo[a].ksteps, P->geo[a].ksteps);
+            }
+            if (last && P->affine) B.affine.push_back({w, P->d_init});
+        }
+    }
+    ArenaBuilder ar;
+    for (auto &h : host)
+        for (int a = 0; a < 3; ++a) {
+            h.o_j[a] = ar.add(h.jobs[a].data(), sizeof(BandJob) * h.jobs[a].size());
+            h.o_t[a] = ar.add(h.tjob[a].data(), sizeof(unsigned short) * h.tjob[a].size());
+        }
+    if (!host.empty()) {
+        VFD_BCUDA(b, take_arena(b->device, ar.host.size(), &B.d));
+        const cudaError_t e = cudaMemcpy(B.d, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            give_arena(b->device, B.d);
+            return bfail(b, VFD_ERR_CUDA, std::string("batch setup: ") + cudaGetErrorString(e));
+        }
+    }
+    for (size_t g = 0; g < host.size(); ++g)
+        for (int a = 0; a < 3; ++a) {
+            B.launches[g].d_jobs[a] = reinterpret_cast<BandJob *>(B.d + host[g].o_j[a]);
+            B.launches[g].d_tjob[a] = reinterpret_cast<unsigned short *>(B.d + host[g].o_t[a]);
+            B.launches[g].ntiles[a] = (int)host[g].tjob[a].size();
+        }
+    b->bands.emplace(n_substeps, std::move(B));
+    return VFD_OK;
+}
+
+// Sets up what a tick of n_substeps needs, outside any capture.
+static vfd_status batch_prepare(vfd_batch *b, int n_substeps)
+{
+    const vfd_status st = batch_prepare_band(b, n_substeps);
+    if (st != VFD_OK) return st;
+    return batch_prepare_fft(b, batch_fft_worlds(b, n_substeps));
 }
 
 // Times one axis pass of the whole batch as configured now (one warm-up,
@@ -2434,6 +2996,9 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
     if (reps < 1) reps = 3;
     DeviceGuard g(b->device);
     VFD_BCUDA(b, cudaStreamSynchronize(b->st));
+    // the tuner times every world, and one pass an axis for all of them
+    const vfd_status ready = batch_prepare_fft(b, b->worlds);
+    if (ready != VFD_OK) return ready;
     // the passes run on the worlds' own fields: save them, restore after
     std::vector<float *> saved(b->worlds.size(), nullptr);
     auto restore = [&](bool copy) {
@@ -2504,6 +3069,7 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
         b->use_os[a] = bc.method == PASS_METHOD_OS;
         b->os_minb[a] = bc.minb;
         b->tuned_ms[a] = best;
+        b->tuned_method[a] = bc.method;
         if (out3) {
             out3[a].method = bc.method == PASS_METHOD_RF ? VFD_PASS_REGISTER_FFT
                              : bc.method == PASS_METHOD_OS ? VFD_PASS_OVERLAP_SAVE
@@ -2518,6 +3084,7 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     restore(true);
+    b->fft_each = false;
     // the next tick runs directly and re-captures its graph with the chosen passes
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -2538,8 +3105,22 @@ vfd_status vfd_batch_destroy(vfd_batch *b)
 
 static vfd_status batch_enqueue(vfd_batch *b, int n_substeps)
 {
-    for (int s = 0; s < n_substeps; ++s) {
-        VFD_BCUDA(b, launch_zero_blocks(b->d_mass_ptrs, b->d_mass_counts, (int)b->worlds.size(), b->st));
+    VFD_BCUDA(b, launch_zero_blocks(b->d_mass_ptrs, b->d_mass_counts, (int)b->worlds.size(), b->st));
+    const BatchBand &B = b->bands.at(n_substeps);
+    for (const auto &x : B.affine)
+        VFD_BCUDA(b, cudaMemcpyAsync(x.first->d_mass, x.second, sizeof(double) * MS_COUNT * x.first->nf,
+                                     cudaMemcpyDeviceToDevice, b->st));
+    for (const auto &L : B.launches)
+        for (int a = 0; a < 3; ++a)
+            VFD_BCUDA(b, launch_band(L.d_jobs[a], L.d_tjob[a], 0, L.ntiles[a], a, L.geo[a], true, b->st));
+    for (size_t i = 0; b->fft_each && i < b->fft_worlds.size(); ++i) {
+        const vfd_status st = enqueue_fft_substeps(b->fft_worlds[i], -1, n_substeps, b->st);
+        if (st != VFD_OK) return bfail(b, st, b->fft_worlds[i]->err);
+    }
+    for (int s = 0; s < n_substeps && b->njobs > 0 && !b->fft_each; ++s) {
+        if (s > 0)
+            VFD_BCUDA(b, launch_zero_blocks(b->d_fft_mass_ptrs, b->d_fft_mass_counts, (int)b->fft_worlds.size(),
+                                            b->st));
         for (int a = 0; a < 3; ++a) {
             if (b->use_rf[a])
                 VFD_BCUDA(b, launch_rf_groups(b->d_osjobs + a * b->njobs, b->rf[a], a, b->st));
@@ -2583,6 +3164,10 @@ vfd_status vfd_batch_tick(vfd_batch *b, int n_substeps, void *stream)
         b->same_ticks = 0;
     }
     ++b->same_ticks;
+    {
+        const vfd_status st = batch_prepare(b, n_substeps);
+        if (st != VFD_OK) return st;
+    }
     VFD_BCUDA(b, cudaEventRecord(b->ev_in, (cudaStream_t)stream));
     VFD_BCUDA(b, cudaStreamWaitEvent(b->st, b->ev_in, 0));
     if (!b->exec && b->same_ticks < 2) {
