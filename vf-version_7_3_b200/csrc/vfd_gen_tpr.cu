@@ -492,18 +492,19 @@ struct C2rSums {
 
 // One real output value at x of a row: the crop / update epilogue; the
 // values for the mass totals are added to the FP32 group sums gc and go.
-__device__ __forceinline__ void c2r_store(const GenRowPass &p, float t, float *dst, float *drow, int x, float &gc,
-                                          float &go)
+// UPD: dval is the update's dChem value there, drow its row (zeroed).
+template <bool UPD>
+__device__ __forceinline__ void c2r_store(const GenRowPass &p, float t, float *dst, float *drow, float dval, int x,
+                                          float &gc, float &go)
 {
     if (p.fuse_crop) {
         gc += t;
         t = p.keep * (t + p.b * p.k0);
-        if (p.fuse_update) {
+        if (UPD) {
+            t = t * p.upd_scale + dval;
+            drow[x] = 0.0f;
+        } else if (p.fuse_update) {
             t *= p.upd_scale;
-            if (drow) {
-                t += drow[x];
-                drow[x] = 0.0f;
-            }
         }
         go += t;
     }
@@ -514,7 +515,7 @@ __device__ __forceinline__ void c2r_store(const GenRowPass &p, float t, float *d
 // a (real part) and b (imaginary part); positions >= nstore go to the leak
 // sum.  The mass sums run in FP32 over groups of 4 positions, each group
 // widened once into the FP64 totals.
-template <int N, int NL>
+template <int N, int NL, bool UPD>
 __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int r0, int l, int n2, int F2, int GS,
                                       C2rSums &s)
 {
@@ -525,15 +526,27 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
     tpr_dft<N, true>(v);
     const RowRef ra = row_ref(p, r0 + l, p.r_s1, p.r_s2), rb = row_ref(p, r0 + NL + l, p.r_s1, p.r_s2);
     float *da = p.rdst + ra.off, *db = p.rdst + rb.off;
-    float *ua = (p.fuse_update && p.dchem) ? p.dchem + ra.off : nullptr;
-    float *ub = (p.fuse_update && p.dchem) ? p.dchem + rb.off : nullptr;
+    float *ua = UPD ? p.dchem + ra.off : nullptr, *ub = UPD ? p.dchem + rb.off : nullptr;
     float gc = 0.0f, go = 0.0f, gl = 0.0f;
+    // The update's dChem values, read four positions ahead of the stores: each
+    // store may alias the next load, so loads between the stores waited for one
+    // another (48 in a row: 512x256x384 x 8, x 26.8 ms a tick; like this 3.5).
+    float qa[4], qb[4];
+    auto ahead = [&](int n1) {
+        const int x = n2 + F2 * n1;
+        qa[n1 & 3] = (UPD && ra.ok && x < p.nstore) ? ua[x] : 0.0f;
+        qb[n1 & 3] = (UPD && rb.ok && x < p.nstore) ? ub[x] : 0.0f;
+    };
+#pragma unroll
+    for (int n1 = 0; n1 < (N < 4 ? N : 4); ++n1) ahead(n1);
 #pragma unroll
     for (int n1 = 0; n1 < N; ++n1) {
         const int x = n2 + F2 * n1;
+        const float ea = qa[n1 & 3], eb = qb[n1 & 3];
+        if (n1 + 4 < N) ahead(n1 + 4);
         if (x < p.nstore) {
-            if (ra.ok) c2r_store(p, v[n1].x, da, ua, x, gc, go);
-            if (rb.ok) c2r_store(p, v[n1].y, db, ub, x, gc, go);
+            if (ra.ok) c2r_store<UPD>(p, v[n1].x, da, ua, ea, x, gc, go);
+            if (rb.ok) c2r_store<UPD>(p, v[n1].y, db, ub, eb, x, gc, go);
         } else {
             gl += v[n1].x + v[n1].y;
         }
@@ -546,7 +559,7 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
     }
 }
 
-template <int NL, int MAXT, int MINB, int MAXN>
+template <int NL, int MAXT, int MINB, int MAXN, bool UPD>
 __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p, int f1)
 {
     constexpr int NR = 2 * NL;
@@ -575,7 +588,7 @@ __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p,
         if (l < NL) {
             switch (F1) {
 #define VFD_C2R_A(n) \
-    case n: if constexpr (n <= MAXN) c2r_a<n, NL>(p, m, r0, l, n2, F2, GS, s); break;
+    case n: if constexpr (n <= MAXN) c2r_a<n, NL, UPD>(p, m, r0, l, n2, F2, GS, s); break;
                 VFD_TPR_SIZES(VFD_C2R_A)
 #undef VFD_C2R_A
             default: break;
@@ -649,14 +662,18 @@ static cudaError_t tpr_attr()
 template <int NL, int MAXT, int MINB, int MAXN>
 static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream_t st)
 {
-    cudaError_t e = inverse ? tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN>>() : tpr_attr<r2c_tpr_kernel<NL, MAXT, MINB, MAXN>>();
+    const bool upd = p.fuse_crop && p.fuse_update && p.dchem;
+    cudaError_t e = !inverse ? tpr_attr<r2c_tpr_kernel<NL, MAXT, MINB, MAXN>>()
+                    : upd    ? tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true>>()
+                             : tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false>>();
     if (e != cudaSuccess) return e;
     const int blocks = (p.nrows + 2 * NL - 1) / (2 * NL);
     if (blocks <= 0) return cudaSuccess;
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    if (inverse) c2r_tpr_kernel<NL, MAXT, MINB, MAXN><<<blocks, nt, sm, st>>>(p, f1);
+    if (inverse && upd) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true><<<blocks, nt, sm, st>>>(p, f1);
+    else if (inverse) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false><<<blocks, nt, sm, st>>>(p, f1);
     else r2c_tpr_kernel<NL, MAXT, MINB, MAXN><<<blocks, nt, sm, st>>>(p, f1);
     note_launch();
     return cudaGetLastError();
