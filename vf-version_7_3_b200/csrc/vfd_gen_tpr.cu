@@ -224,9 +224,39 @@ __device__ __forceinline__ void col_ai(const GenColPass &p, const TprSmem &m, fl
 
 // One tile = NL consecutive lines of one outer index; thread (l, g) with the
 // line fastest takes group g of each pass.
-template <int NL, int MAXT, int MINB, int MAXN>
-__global__ void __launch_bounds__(MAXT, MINB) c2c_tpr_kernel(const GenColPass p, int f1)
+// The parameter block as field blockIdx.y of the launch runs it.
+__device__ __forceinline__ GenRowPass tpr_row_field(const GenRowPass &p, const GenFields &ff)
 {
+    const int f = blockIdx.y;
+    GenRowPass q = p;
+    q.rsrc += f * ff.r;
+    q.rdst += f * ff.r;
+    q.cdst += f * ff.c;
+    q.csrc += f * ff.c;
+    q.b = ff.b[f];
+    q.keep = ff.keep[f];
+    q.k0 = ff.k0[f];
+    q.upd_scale = ff.upd_scale[f];
+    q.dchem = ff.dchem[f];
+    if (q.mass_in) q.mass_in += f * ff.mass;
+    if (q.mass_leak) q.mass_leak += f * ff.mass;
+    if (q.mass_conv) q.mass_conv += f * ff.mass;
+    if (q.mass_out) q.mass_out += f * ff.mass;
+    return q;
+}
+__device__ __forceinline__ GenColPass tpr_col_field(const GenColPass &p, const GenFields &ff)
+{
+    GenColPass q = p;
+    q.data += blockIdx.y * ff.c;
+    q.kspec += blockIdx.y * ff.k;
+    return q;
+}
+
+// MF (here and below): the launch holds several fields (blockIdx.y).
+template <int NL, int MAXT, int MINB, int MAXN, bool MF>
+__global__ void __launch_bounds__(MAXT, MINB) c2c_tpr_kernel(const GenColPass p_, const GenFields ff, int f1)
+{
+    const GenColPass p = MF ? tpr_col_field(p_, ff) : p_;
     constexpr int LS = NL + 1;
     extern __shared__ __align__(16) float2 tsm[];
     const int F = p.plan.F, F1 = f1, F2 = F / f1;
@@ -382,9 +412,10 @@ __device__ __forceinline__ void r2c_b(const TprSmem &m, int l, int k1, int F1, i
     }
 }
 
-template <int NL, int MAXT, int MINB, int MAXN>
-__global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p, int f1)
+template <int NL, int MAXT, int MINB, int MAXN, bool MF>
+__global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p_, const GenFields ff, int f1)
 {
+    const GenRowPass p = MF ? tpr_row_field(p_, ff) : p_;
     constexpr int LS = NL + 1, NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
     __shared__ double red[32];
@@ -559,9 +590,10 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
     }
 }
 
-template <int NL, int MAXT, int MINB, int MAXN, bool UPD>
-__global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p, int f1)
+template <int NL, int MAXT, int MINB, int MAXN, bool UPD, bool MF>
+__global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_, const GenFields ff, int f1)
 {
+    const GenRowPass p = MF ? tpr_row_field(p_, ff) : p_;
     constexpr int NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
     __shared__ double red[32];
@@ -659,37 +691,37 @@ static cudaError_t tpr_attr()
     return e;
 }
 
-template <int NL, int MAXT, int MINB, int MAXN>
-static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream_t st)
+template <int NL, int MAXT, int MINB, int MAXN, bool MF>
+static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream_t st, const GenFields &ff)
 {
-    const bool upd = p.fuse_crop && p.fuse_update && p.dchem;
-    cudaError_t e = !inverse ? tpr_attr<r2c_tpr_kernel<NL, MAXT, MINB, MAXN>>()
-                    : upd    ? tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true>>()
-                             : tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false>>();
+    const bool upd = p.fuse_crop && p.fuse_update && ff.dchem[0];
+    cudaError_t e = !inverse ? tpr_attr<r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>>()
+                    : upd    ? tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF>>()
+                             : tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF>>();
     if (e != cudaSuccess) return e;
-    const int blocks = (p.nrows + 2 * NL - 1) / (2 * NL);
-    if (blocks <= 0) return cudaSuccess;
+    const dim3 blocks((unsigned)((p.nrows + 2 * NL - 1) / (2 * NL)), (unsigned)ff.n);
+    if (p.nrows <= 0) return cudaSuccess;
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    if (inverse && upd) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true><<<blocks, nt, sm, st>>>(p, f1);
-    else if (inverse) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false><<<blocks, nt, sm, st>>>(p, f1);
-    else r2c_tpr_kernel<NL, MAXT, MINB, MAXN><<<blocks, nt, sm, st>>>(p, f1);
+    if (inverse && upd) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
+    else if (inverse) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
+    else r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
     note_launch();
     return cudaGetLastError();
 }
 
-template <int NL, int MAXT, int MINB, int MAXN>
-static cudaError_t cols_nl(const GenColPass &p, int f1, cudaStream_t st)
+template <int NL, int MAXT, int MINB, int MAXN, bool MF>
+static cudaError_t cols_nl(const GenColPass &p, int f1, cudaStream_t st, const GenFields &ff)
 {
-    cudaError_t e = tpr_attr<c2c_tpr_kernel<NL, MAXT, MINB, MAXN>>();
+    cudaError_t e = tpr_attr<c2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>>();
     if (e != cudaSuccess) return e;
     const int64_t blocks = (int64_t)p.nouter * ((p.nlines + NL - 1) / NL);
     if (blocks <= 0) return cudaSuccess;
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    c2c_tpr_kernel<NL, MAXT, MINB, MAXN><<<(unsigned)blocks, nt, sm, st>>>(p, f1);
+    c2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF><<<dim3((unsigned)blocks, (unsigned)ff.n), nt, sm, st>>>(p, ff, f1);
     note_launch();
     return cudaGetLastError();
 }
@@ -704,21 +736,46 @@ static bool tpr_use16(bool rows, int F, int f1)
     return tpr_nl(rows) == 16 || g > 24;
 }
 
-cudaError_t launch_tpr_rows(const GenRowPass &p, int f1, bool inverse, cudaStream_t st)
+// Several fields in one launch: only on the 8-line kernels.  For one field
+// the parameter block stays in constant memory, which the kernels' register
+// budget counts on.
+cudaError_t launch_tpr_rows(const GenRowPass &p, int f1, bool inverse, cudaStream_t st, const GenFields &ff)
 {
-    if (!tpr_split_ok(p.plan.F, f1)) return cudaErrorInvalidValue;
-    if (tpr_use16(true, p.plan.F, f1)) return rows_nl<16, 512, 1, 32>(p, f1, inverse, st);
-    return rows_nl<8, 256, 3, 24>(p, f1, inverse, st);
+    if (!tpr_split_ok(p.plan.F, f1) || ff.n < 1 || ff.n > GEN_FIELDS) return cudaErrorInvalidValue;
+    const bool use16 = tpr_use16(true, p.plan.F, f1);
+    if (ff.n > 1 && !use16) return rows_nl<8, 256, 3, 24, true>(p, f1, inverse, st, ff);
+    for (int f = 0; f < ff.n; ++f) {
+        const GenRowPass q = row_field(p, ff, f);
+        GenFields one;
+        one.dchem[0] = q.dchem;
+        const cudaError_t e = use16 ? rows_nl<16, 512, 1, 32, false>(q, f1, inverse, st, one)
+                                    : rows_nl<8, 256, 3, 24, false>(q, f1, inverse, st, one);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t launch_tpr_cols(const GenColPass &p, int f1, cudaStream_t st)
+cudaError_t launch_tpr_cols(const GenColPass &p, int f1, cudaStream_t st, const GenFields &ff)
 {
-    if (!tpr_split_ok(p.plan.F, f1)) return cudaErrorInvalidValue;
-    if (tpr_use16(false, p.plan.F, f1)) return cols_nl<16, 512, 1, 32>(p, f1, st);
+    if (!tpr_split_ok(p.plan.F, f1) || ff.n < 1 || ff.n > GEN_FIELDS) return cudaErrorInvalidValue;
+    const bool use16 = tpr_use16(false, p.plan.F, f1);
     // measured on B200 (512x256x384 world): the forward-only and inverse-only
     // passes run best at 4 resident CTAs (64 registers), the fused z pass and
     // the row passes at 3 (85 registers)
-    return p.mode == GEN_FWD_MUL_INV ? cols_nl<8, 256, 3, 24>(p, f1, st) : cols_nl<8, 256, 4, 24>(p, f1, st);
+    const bool fused = p.mode == GEN_FWD_MUL_INV;
+    if (ff.n > 1 && !use16)
+        return fused ? cols_nl<8, 256, 3, 24, true>(p, f1, st, ff) : cols_nl<8, 256, 4, 24, true>(p, f1, st, ff);
+    for (int f = 0; f < ff.n; ++f) {
+        GenColPass q = p;
+        q.data += f * ff.c;
+        if (q.kspec) q.kspec += f * ff.k;
+        const GenFields one;
+        const cudaError_t e = use16   ? cols_nl<16, 512, 1, 32, false>(q, f1, st, one)
+                              : fused ? cols_nl<8, 256, 3, 24, false>(q, f1, st, one)
+                                      : cols_nl<8, 256, 4, 24, false>(q, f1, st, one);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace vfd

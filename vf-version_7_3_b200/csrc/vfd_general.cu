@@ -557,35 +557,60 @@ static bool tpr_enabled()
     return on == 1;
 }
 
-cudaError_t launch_gen_rows(int variant, const GenRowPass &p, bool inverse, cudaStream_t st)
+cudaError_t launch_gen_rows(int variant, const GenRowPass &p, bool inverse, cudaStream_t st, const GenFields *ff)
 {
-    const int f1 = tpr_enabled() ? tpr_split(p.plan.F) : 0;
-    if (f1 > 0) return launch_tpr_rows(p, f1, inverse, st);
-    switch (variant) {
-#define VFD_GEN_ROW_CASE(i, NL, TL, MAXP, MINB) \
-    case i: return launch_rows_t<NL, TL, MAXP, MINB>(p, inverse, st);
-        VFD_AXIS_VARIANTS(VFD_GEN_ROW_CASE)
-#undef VFD_GEN_ROW_CASE
-    default: return cudaErrorInvalidValue;
+    GenFields one;
+    if (!ff) {
+        one.b[0] = p.b;
+        one.keep[0] = p.keep;
+        one.k0[0] = p.k0;
+        one.upd_scale[0] = p.upd_scale;
+        one.dchem[0] = p.dchem;
+        ff = &one;
     }
+    const int f1 = tpr_enabled() ? tpr_split(p.plan.F) : 0;
+    if (f1 > 0) return launch_tpr_rows(p, f1, inverse, st, *ff);
+    for (int f = 0; f < ff->n; ++f) {
+        const GenRowPass q = row_field(p, *ff, f);
+        cudaError_t e = cudaErrorInvalidValue;
+        switch (variant) {
+#define VFD_GEN_ROW_CASE(i, NL, TL, MAXP, MINB) \
+    case i: e = launch_rows_t<NL, TL, MAXP, MINB>(q, inverse, st); break;
+            VFD_AXIS_VARIANTS(VFD_GEN_ROW_CASE)
+#undef VFD_GEN_ROW_CASE
+        default: break;
+        }
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
-cudaError_t launch_gen_cols(int variant, const GenColPass &p, cudaStream_t st)
+cudaError_t launch_gen_cols(int variant, const GenColPass &p, cudaStream_t st, const GenFields *ff)
 {
+    const GenFields one;
+    if (!ff) ff = &one;
     const int f1 = tpr_enabled() ? tpr_split(p.plan.F) : 0;
     if (f1 > 0) {
         // a pass whose register-engine tile would not fit in shared memory
         // runs on the Stockham kernels
-        const cudaError_t e = launch_tpr_cols(p, f1, st);
+        const cudaError_t e = launch_tpr_cols(p, f1, st, *ff);
         if (e != cudaErrorInvalidConfiguration) return e;
     }
-    switch (variant) {
+    for (int f = 0; f < ff->n; ++f) {
+        GenColPass q = p;
+        q.data += f * ff->c;
+        if (q.kspec) q.kspec += f * ff->k;
+        cudaError_t e = cudaErrorInvalidValue;
+        switch (variant) {
 #define VFD_GEN_COL_CASE(i, NL, TL, MAXP, MINB) \
-    case i: return launch_cols_t<NL, TL, MAXP, MINB>(p, st);
-        VFD_AXIS_VARIANTS(VFD_GEN_COL_CASE)
+    case i: e = launch_cols_t<NL, TL, MAXP, MINB>(q, st); break;
+            VFD_AXIS_VARIANTS(VFD_GEN_COL_CASE)
 #undef VFD_GEN_COL_CASE
-    default: return cudaErrorInvalidValue;
+        default: break;
+        }
+        if (e != cudaSuccess) return e;
     }
+    return cudaSuccess;
 }
 
 static int grid_for(int64_t n)

@@ -54,17 +54,48 @@ struct GenColPass {
     int kspec_smem;           // set by the Stockham launcher: spectrum tile staged in shared memory
 };
 
+// Fields that share a launch: field f's pass is the parameter block with its
+// pointers moved by f strides and its scalars replaced by f's.
+constexpr int GEN_FIELDS = 8;
+struct GenFields {
+    int n = 1;
+    int64_t r = 0, c = 0, k = 0;  // strides of the real rows, the spectra and the kernel spectra
+    float b[GEN_FIELDS] = {}, keep[GEN_FIELDS] = {}, k0[GEN_FIELDS] = {}, upd_scale[GEN_FIELDS] = {};
+    float *dchem[GEN_FIELDS] = {};
+    int mass = 0;                 // doubles between the fields' accounting blocks
+};
+
+// p as field f of ff runs it.
+inline GenRowPass row_field(const GenRowPass &p, const GenFields &ff, int f)
+{
+    GenRowPass q = p;
+    if (q.rsrc) q.rsrc += f * ff.r;
+    if (q.rdst) q.rdst += f * ff.r;
+    if (q.cdst) q.cdst += f * ff.c;
+    if (q.csrc) q.csrc += f * ff.c;
+    q.b = ff.b[f];
+    q.keep = ff.keep[f];
+    q.k0 = ff.k0[f];
+    q.upd_scale = ff.upd_scale[f];
+    q.dchem = ff.dchem[f];
+    for (double **m : {&q.mass_in, &q.mass_leak, &q.mass_conv, &q.mass_out})
+        if (*m) *m += f * ff.mass;
+    return q;
+}
+
 // Register engine (vfd_gen_tpr.cu).  tpr_split: F = f1 * f2 with
 // f1 <= f2 <= 32 both lengths the engine runs (f2 as small as possible), 0
 // when F has no such split.  The launchers take the split to use; they
 // return cudaErrorInvalidConfiguration, without launching, when the tile
 // does not fit in shared memory.
 int tpr_split(int F);
-cudaError_t launch_tpr_rows(const GenRowPass &p, int f1, bool inverse, cudaStream_t st);
-cudaError_t launch_tpr_cols(const GenColPass &p, int f1, cudaStream_t st);
+cudaError_t launch_tpr_rows(const GenRowPass &p, int f1, bool inverse, cudaStream_t st, const GenFields &ff);
+cudaError_t launch_tpr_cols(const GenColPass &p, int f1, cudaStream_t st, const GenFields &ff);
 
-cudaError_t launch_gen_rows(int variant, const GenRowPass &p, bool inverse, cudaStream_t st);
-cudaError_t launch_gen_cols(int variant, const GenColPass &p, cudaStream_t st);
+// ff: the fields of the launch (NULL: one, p's own).
+cudaError_t launch_gen_rows(int variant, const GenRowPass &p, bool inverse, cudaStream_t st,
+                            const GenFields *ff = nullptr);
+cudaError_t launch_gen_cols(int variant, const GenColPass &p, cudaStream_t st, const GenFields *ff = nullptr);
 cudaError_t launch_pad(float *P, const float *u, int nx, int ny, int nz, int Fx, int Fy, int Fz, const int *lo,
                        const int *hi, float b, cudaStream_t st);
 cudaError_t launch_modulate(float2 *C, const float2 *K, int64_t n, float scale, cudaStream_t st);

@@ -427,7 +427,8 @@ struct vfd_world {
     int Fxh = 0;
     int gvar[3] = {0, 0, 0};         // kernel variants of the x rows, y and z columns
     float2 *d_kspec = nullptr;       // [f][Fz][Fy][Fxh], unscaled K
-    float2 *d_C = nullptr;           // spectrum scratch
+    float2 *d_C = nullptr;           // spectrum scratch of gen_group fields
+    int gen_group = 1;               // fields a launch of the general transform holds
     float *d_P = nullptr;            // full real grid scratch (plain)
     std::vector<float> k0;           // K(0,0,0) = sum of the window, per field
     float *d_upd = nullptr;          // vfd_diffuse_update_host: the fields' dChem on the device
@@ -574,6 +575,17 @@ static bool os_enabled()
 }
 
 static bool os_plain_staging(const OsJob &j);
+
+// Fields a launch of the fused general transform holds: as many as keep the
+// launch's spectra within 64 MB, half of L2, so that the next pass finds them
+// there.  A field of its own launch left the chip idle on small grids (75x50x33 x
+// 8: 5 launches a field of 100-360 CTAs each, 400 us a tick; together 60); where
+// one field's spectra exceed that, the launches are full and share nothing.
+static int general_group(const vfd_world *w)
+{
+    const int64_t bytes = (int64_t)sizeof(float2) * w->Fxh * w->F[1] * w->nz;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(w->nf, GEN_FIELDS), ((int64_t)64 << 20) / bytes));
+}
 
 // Copies v to a new device array (at least one element).
 template <class T>
@@ -1252,7 +1264,8 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         }
         w->k0.assign(w->nf, 1.0f);
         const int64_t nc = (w->method == VFD_METHOD_PLAIN) ? nk : (int64_t)w->Fxh * w->F[1] * w->nz;
-        if ((e = cudaMalloc(&w->d_C, sizeof(float2) * nc)) != cudaSuccess) return bail(e, "cudaMalloc spectrum scratch");
+        if (w->method == VFD_METHOD_FFT3D) w->gen_group = general_group(w);
+        if ((e = cudaMalloc(&w->d_C, sizeof(float2) * nc * w->gen_group)) != cudaSuccess) return bail(e, "cudaMalloc spectrum scratch");
         if (w->method == VFD_METHOD_PLAIN) {
             if ((e = cudaMalloc(&w->d_P, sizeof(float) * (int64_t)w->F[0] * w->F[1] * w->F[2])) != cudaSuccess)
                 return bail(e, "cudaMalloc padded grid");
@@ -1319,7 +1332,7 @@ vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes)
     if (w->method != VFD_METHOD_SEPARABLE) {
         const size_t nk = (size_t)w->Fxh * w->F[1] * w->F[2];
         b += sizeof(float2) * nk * w->nf;
-        b += sizeof(float2) * ((w->method == VFD_METHOD_PLAIN) ? nk : (size_t)w->Fxh * w->F[1] * w->nz);
+        b += sizeof(float2) * ((w->method == VFD_METHOD_PLAIN) ? nk : (size_t)w->Fxh * w->F[1] * w->nz) * w->gen_group;
         if (w->method == VFD_METHOD_PLAIN) b += sizeof(float) * (size_t)w->F[0] * w->F[1] * w->F[2];
     }
     *bytes = b;
@@ -1761,9 +1774,10 @@ struct UpdateArgs {
     const float *decay;   // n_fields entries
 };
 
-// One substep of field f with the general 3D transform; with `upd` the crop
-// store applies the update epilogue.
-static vfd_status enqueue_general_substep(vfd_world *w, int f, cudaStream_t st, const UpdateArgs *upd = nullptr)
+// One substep of fields f .. f + n - 1 with the general 3D transform (n > 1:
+// VFD_METHOD_FFT3D only, n <= gen_group); with `upd` the crop store applies
+// the update epilogue (to fields that all have a dChem, or none).
+static vfd_status enqueue_general_substep(vfd_world *w, int f, int n, cudaStream_t st, const UpdateArgs *upd = nullptr)
 {
     const int Fx = w->F[0], Fy = w->F[1], Fz = w->F[2];
     const int64_t nk = (int64_t)w->Fxh * Fy * Fz;
@@ -1771,10 +1785,22 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, cudaStream_t st, 
     double *mass = w->d_mass + (int64_t)f * MS_COUNT;
     const float2 *K = w->d_kspec + nk * f;
     const float invN = (float)(1.0 / ((double)Fx * Fy * Fz));
-    const float b = w->pad_mode == VFD_PAD_CONSTANT_VF ? w->params[f].baseline : 0.0f;
-    const float keep = (float)(1.0 - w->params[f].decay_rate);
     int lo[3], hi[3];
     interior_box(w, lo, hi);
+    GenFields ff;
+    ff.n = n;
+    ff.r = w->V;
+    ff.c = (int64_t)w->Fxh * Fy * w->nz;
+    ff.k = nk;
+    ff.mass = MS_COUNT;
+    for (int i = 0; i < n; ++i) {
+        ff.b[i] = w->pad_mode == VFD_PAD_CONSTANT_VF ? w->params[f + i].baseline : 0.0f;
+        ff.keep[i] = (float)(1.0 - w->params[f + i].decay_rate);
+        ff.k0[i] = w->k0[f + i];
+        ff.upd_scale[i] = upd ? upd->decay[f + i] : 1.0f;
+        ff.dchem[i] = upd && upd->dchem ? upd->dchem[f + i] : nullptr;
+    }
+    const float b = ff.b[0], keep = ff.keep[0];
     GenRowPass r;
     memset(&r, 0, sizeof(r));
     r.plan = w->plan[0];
@@ -1798,16 +1824,15 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, cudaStream_t st, 
             r.box_lo[i] = lo[i];
             r.box_hi[i] = hi[i];
         }
-        r.b = b;
         r.mass_in = mass + MS_INPUT;
         {
             LaunchTimer lt(w, 0, st);
-            VFD_CUDA(w, launch_gen_rows(w->gvar[0], r, false, st));
+            VFD_CUDA(w, launch_gen_rows(w->gvar[0], r, false, st, &ff));
             lt.done();
         }
         {
             LaunchTimer lt(w, 1, st);
-            VFD_CUDA(w, launch_gen_cols(w->gvar[1], col_pass(w, PASS_Y, w->d_C, w->nz, w->ny, Fy, GEN_FORWARD), st));
+            VFD_CUDA(w, launch_gen_cols(w->gvar[1], col_pass(w, PASS_Y, w->d_C, w->nz, w->ny, Fy, GEN_FORWARD), st, &ff));
             lt.done();
         }
         {
@@ -1817,29 +1842,23 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, cudaStream_t st, 
             c.k_s_pos = (int64_t)w->Fxh * Fy;
             c.scale = invN;
             LaunchTimer lt(w, 2, st);
-            VFD_CUDA(w, launch_gen_cols(w->gvar[2], c, st));
+            VFD_CUDA(w, launch_gen_cols(w->gvar[2], c, st, &ff));
             lt.done();
         }
         {
             LaunchTimer lt(w, 1, st);
-            VFD_CUDA(w, launch_gen_cols(w->gvar[1], col_pass(w, PASS_Y, w->d_C, w->nz, Fy, w->ny, GEN_INVERSE), st));
+            VFD_CUDA(w, launch_gen_cols(w->gvar[1], col_pass(w, PASS_Y, w->d_C, w->nz, Fy, w->ny, GEN_INVERSE), st, &ff));
             lt.done();
         }
         r.fuse_pad = 0;
         r.fuse_crop = 1;
-        r.keep = keep;
-        r.k0 = w->k0[f];
-        if (upd) {
-            r.fuse_update = 1;
-            r.upd_scale = upd->decay[f];
-            r.dchem = upd->dchem ? upd->dchem[f] : nullptr;
-        }
+        r.fuse_update = upd ? 1 : 0;
         r.mass_in = nullptr;
         r.mass_leak = mass + MS_LEAK_X;
         r.mass_conv = mass + MS_CONV;
         r.mass_out = mass + MS_OUT;
         LaunchTimer lt(w, 0, st);
-        VFD_CUDA(w, launch_gen_rows(w->gvar[0], r, true, st));
+        VFD_CUDA(w, launch_gen_rows(w->gvar[0], r, true, st, &ff));
         lt.done();
         return VFD_OK;
     }
@@ -1926,12 +1945,16 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
 {
     if (w->method != VFD_METHOD_SEPARABLE) {
         const int f0 = field < 0 ? 0 : field, f1 = field < 0 ? w->nf : field + 1;
-        for (int s = 0; s < n_substeps; ++s)
-            for (int f = f0; f < f1; ++f) {
-                VFD_CUDA(w, cudaMemsetAsync(w->d_mass + (int64_t)f * MS_COUNT, 0, sizeof(double) * MS_COUNT, st));
-                vfd_status r = enqueue_general_substep(w, f, st, s + 1 == n_substeps ? upd : nullptr);
+        for (int s = 0; s < n_substeps; ++s) {
+            const UpdateArgs *u = s + 1 == n_substeps ? upd : nullptr;
+            auto has_d = [&](int f) { return u && u->dchem && u->dchem[f]; };
+            VFD_CUDA(w, cudaMemsetAsync(w->d_mass + (int64_t)f0 * MS_COUNT, 0, sizeof(double) * MS_COUNT * (f1 - f0), st));
+            for (int f = f0, n = 0; f < f1; f += n) {
+                for (n = 1; f + n < f1 && n < w->gen_group && has_d(f + n) == has_d(f);) ++n;
+                vfd_status r = enqueue_general_substep(w, f, n, st, u);
                 if (r != VFD_OK) return r;
             }
+        }
         if (field < 0) {
             if (w->dep_njobs > 0)
                 VFD_CUDA(w, launch_deposit(w->d_dep, w->dep_njobs, w->d_src_idx, w->d_src_amt, w->src_total,
