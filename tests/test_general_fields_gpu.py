@@ -68,3 +68,44 @@ def test_fields_with_and_without_dchem(gpu):
 
 def test_more_fields_than_a_launch_holds(gpu):
     check((33, 20, 17), (40, 24, 21), 11)
+
+
+@pytest.mark.parametrize("method", [vfd.METHOD_FFT3D, vfd.METHOD_SEPARABLE])
+@pytest.mark.parametrize("kind", ["pageable", "pinned", "shared", "partial"])
+def test_update_host_buffers(gpu, method, kind):
+    """vfd_diffuse_update_host zeroes dChem in pinned buffers by copies from the
+    device, in others on the host; a buffer that several fields share is read
+    by all of them before it is zeroed."""
+    import torch
+    nx, ny, nz, nf = 40, 30, 22, 4
+    sig = [0.7 + 0.2 * f for f in range(nf)]
+    decay = [0.9] * nf
+    rng = np.random.default_rng(3)
+
+    def buffers(n):
+        a = [rng.random((nz, ny, nx), dtype=np.float32) * np.float32(1e-3) for _ in range(n)]
+        return a if kind == "pageable" else [torch.from_numpy(x).pin_memory().numpy() for x in a]
+
+    p, d = buffers(nf), buffers(nf)
+    if kind == "shared":
+        d = [d[0]] * nf
+    p0, d0 = [x.copy() for x in p], [x.copy() for x in d]
+    params = [vfd.field_params(s, 0.02) for s in sig]
+    with vfd.World(nx, ny, nz, params, method=method) as w:
+        if kind == "partial":
+            import ctypes as C
+            ps = (C.c_void_p * nf)(*[x.ctypes.data for x in p])
+            ds = (C.c_void_p * nf)(*[x.ctypes.data if f % 2 else None for f, x in enumerate(d)])
+            dec = np.array(decay, np.float32)
+            assert vfd.lib().vfd_diffuse_update_host(w.handle, ps, ds, dec.ctypes.data, 1) == 0
+        else:
+            w.diffuse_update_host(p, d, decay)
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    for f in range(nf):
+        has = kind != "partial" or f % 2
+        ref = oracle.tick(p0[f], sig[f], 0.02, 1, *none) * float(np.float32(0.9)) + (d0[f] if has else 0)
+        assert rel_l2(p[f], ref) <= REL_L2, f
+        if has:
+            assert not d[f].any()
+        else:
+            np.testing.assert_array_equal(d[f], d0[f])

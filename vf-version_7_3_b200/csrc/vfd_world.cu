@@ -2440,8 +2440,18 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
     const size_t bytes = sizeof(float) * w->V;
     if (host_d && !w->d_upd) VFD_CUDA(w, cudaMalloc(&w->d_upd, bytes * w->nf));
     std::vector<float *> dptr(w->nf, nullptr);
+    std::vector<char> pinned(w->nf, 0);
     for (int f = 0; f < w->nf; ++f)
-        if (host_d && host_d[f]) dptr[f] = w->d_upd + (int64_t)f * w->V;
+        if (host_d && host_d[f]) {
+            dptr[f] = w->d_upd + (int64_t)f * w->V;
+            cudaPointerAttributes at;
+            pinned[f] = cudaPointerGetAttributes(&at, host_d[f]) == cudaSuccess && at.type == cudaMemoryTypeHost;
+            if (!pinned[f]) cudaGetLastError();
+            // a buffer that another field's upload still reads is zeroed at the end
+            for (int g = 0; g < w->nf && pinned[f]; ++g)
+                for (const float *o : {(const float *)host_p[g], g != f ? (const float *)host_d[g] : nullptr})
+                    if (o && o < host_d[f] + w->V && host_d[f] < o + w->V) pinned[f] = 0;
+        }
     for (int f = 0; f < w->nf; ++f) {
         float *dev = w->d_fields + (int64_t)f * w->V;
         VFD_CUDA(w, cudaMemcpyAsync(dev, host_p[f], bytes, cudaMemcpyHostToDevice, w->s_in));
@@ -2457,11 +2467,16 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
         VFD_CUDA(w, cudaEventRecord(w->ev_cmp[f], w->s_cmp));
         VFD_CUDA(w, cudaStreamWaitEvent(w->s_out, w->ev_cmp[f], 0));
         VFD_CUDA(w, cudaMemcpyAsync(host_p[f], dev, bytes, cudaMemcpyDeviceToHost, w->s_out));
+        // dChem = 0 on the host (WHChemical.cpp:427): the update has zeroed the
+        // device's copy, which goes back to pinned buffers on the copy engine,
+        // beside the uploads of the next fields (256x128x192 x 8: one host
+        // thread's memset took 14 of the 22 ms of a call)
+        if (dptr[f] && pinned[f]) VFD_CUDA(w, cudaMemcpyAsync(host_d[f], dptr[f], bytes, cudaMemcpyDeviceToHost, w->s_out));
     }
-    // dChem = 0 on the host (WHChemical.cpp:427) once its copy has landed on the device
+    // pageable buffers: on the host, once their copies have landed on the device
     VFD_CUDA(w, cudaStreamSynchronize(w->s_in));
     for (int f = 0; f < w->nf; ++f)
-        if (dptr[f]) std::memset(host_d[f], 0, bytes);
+        if (dptr[f] && !pinned[f]) std::memset(host_d[f], 0, bytes);
     VFD_CUDA(w, cudaStreamSynchronize(w->s_out));
     VFD_CUDA(w, cudaStreamSynchronize(w->s_cmp));
     int herr = 0;
