@@ -911,6 +911,9 @@ __global__ void __launch_bounds__(BD_THREADS, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmem;
+    grid_dep_launch();
+    // the weights do not depend on the kernel before; the fields do
+    if (warp != BD_FETCH) grid_dep_wait();
     const BandTiles T{jobs, tjob, tile_begin, tile_end};
     // registers: 80 a thread at launch; 256 x (104 + 88 + 48) = 256 x (96 + 96 + 48) = 768 x 80
     if (warp < BD_CONV0) {
@@ -1127,10 +1130,10 @@ cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int t
     grow(nstage, BD_MAXSTAGE);
     grow(nslots, BD_MAXSLOT);
     const size_t sm = std::max(bytes(), BD_SMEM_MIN);
-    band_kernel<XP><<<std::min(ntiles, sms), BD_THREADS, sm, st>>>(jobs, tjob, tile_begin, tile_begin + ntiles,
-                                                                  sums ? 1 : 0, nstage, nslots, slot);
+    const cudaError_t e = launch_overlapped(ntiles <= 8 * sms, band_kernel<XP>, dim3((unsigned)std::min(ntiles, sms)), BD_THREADS, sm, st, jobs,
+                                            tjob, tile_begin, tile_begin + ntiles, sums ? 1 : 0, nstage, nslots, slot);
     note_launch();
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace

@@ -256,6 +256,8 @@ __device__ __forceinline__ GenColPass tpr_col_field(const GenColPass &p, const G
 template <int NL, int MAXT, int MINB, int MAXN, bool MF>
 __global__ void __launch_bounds__(MAXT, MINB) c2c_tpr_kernel(const GenColPass p_, const GenFields ff, int f1)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const GenColPass p = MF ? tpr_col_field(p_, ff) : p_;
     constexpr int LS = NL + 1;
     extern __shared__ __align__(16) float2 tsm[];
@@ -415,6 +417,8 @@ __device__ __forceinline__ void r2c_b(const TprSmem &m, int l, int k1, int F1, i
 template <int NL, int MAXT, int MINB, int MAXN, bool MF>
 __global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p_, const GenFields ff, int f1)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const GenRowPass p = MF ? tpr_row_field(p_, ff) : p_;
     constexpr int LS = NL + 1, NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
@@ -593,6 +597,8 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
 template <int NL, int MAXT, int MINB, int MAXN, bool UPD, bool MF>
 __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_, const GenFields ff, int f1)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     const GenRowPass p = MF ? tpr_row_field(p_, ff) : p_;
     constexpr int NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
@@ -634,6 +640,8 @@ __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_
 
 // ---------------------------------------------------------------------------
 // Host side.
+
+constexpr int64_t TPR_OVERLAP = 4096;
 
 static bool tpr_len(int n)
 {
@@ -704,11 +712,12 @@ static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    if (inverse && upd) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
-    else if (inverse) c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
-    else r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF><<<blocks, nt, sm, st>>>(p, ff, f1);
+    e = launch_overlapped((int64_t)blocks.x * blocks.y <= TPR_OVERLAP, !inverse ? r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>
+                          : upd    ? c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF>
+                                   : c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF>,
+                          blocks, (unsigned)nt, sm, st, p, ff, f1);
     note_launch();
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 template <int NL, int MAXT, int MINB, int MAXN, bool MF>
@@ -721,9 +730,10 @@ static cudaError_t cols_nl(const GenColPass &p, int f1, cudaStream_t st, const G
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    c2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF><<<dim3((unsigned)blocks, (unsigned)ff.n), nt, sm, st>>>(p, ff, f1);
+    e = launch_overlapped(blocks * ff.n <= TPR_OVERLAP, c2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>, dim3((unsigned)blocks, (unsigned)ff.n), (unsigned)nt, sm, st,
+                          p, ff, f1);
     note_launch();
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 static bool tpr_split_ok(int F, int f1) { return f1 >= 2 && F % f1 == 0 && tpr_len(f1) && tpr_len(F / f1); }

@@ -65,6 +65,33 @@ cudaError_t launch_sample(const float *src, int nx, int ny, int nz, int stride, 
 
 void note_launch();
 
+// Launches a kernel that may start while the kernel before it in the stream
+// runs out (programmatic dependent launch): its blocks take their places as
+// the other's leave, and set up what does not depend on it; grid_dep_wait
+// then waits until the other is complete and its writes are visible.
+template <class... P, class... A>
+cudaError_t launch_overlapped(bool overlap, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                              A... args)
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// Lets the next kernel of the stream start once every block has said so.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+#endif
+
 // Unique id of the calling thread's current CUDA context (0 when the driver
 // does not tell): caches of device pointers are keyed by it, because a
 // device reset loads the library into a new context.

@@ -248,6 +248,7 @@ __global__ void __launch_bounds__(256) deposit_kernel(const DepositJob *__restri
 {
     __shared__ double fsum[8];
     __shared__ int fbase;
+    grid_dep_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < 8) fsum[threadIdx.x] = 0.0;
@@ -403,9 +404,9 @@ cudaError_t launch_deposit(const DepositJob *jobs, int njobs, const int32_t *idx
 {
     if (total <= 0) return cudaSuccess;
     const int64_t blocks = (total + 255) / 256;
-    deposit_kernel<<<(unsigned)blocks, 256, 0, st>>>(jobs, njobs, idx, amt, total, err);
+    const cudaError_t e = launch_overlapped(blocks <= 1024, deposit_kernel, dim3((unsigned)blocks), 256, 0, st, jobs, njobs, idx, amt, total, err);
     note_launch();
-    return cudaGetLastError();
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
 }  // namespace vfd
