@@ -241,11 +241,11 @@ __device__ __forceinline__ int band_at(int line, int pos)
 }
 
 // ---------------------------------------------------------------------------
-// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.72-0.74 ms a pass for
-// ten folded substeps (4.4 TB/s of the 8 bytes a voxel it moves; without its
-// products 0.60), so a tick of ten substeps and its deposit takes 2.3-2.6 ms
-// against 19.0 ms on 30 register-FFT passes of 0.58-0.66 ms; 0.58-0.60 ms (y, z;
-// x 0.70) for one substep.  768x384x576: 9.3 against 60 ms.  What bounds it: HBM,
+// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.70-0.72 ms a pass for
+// ten folded substeps (4.5 TB/s of the 8 bytes a voxel it moves; without its
+// products 0.60), so a tick of ten substeps and its deposit takes 2.3 ms alone
+// and 2.6 ms back to back (power-limited), against 19.0 ms on 30 register-FFT
+// passes of 0.58-0.66 ms; 0.57-0.58 ms (y, z; x 0.76) for one substep.  768x384x576: 9.3 against 60 ms.  What bounds it: HBM,
 // with the products (48 cycles each, two issuing threads together) and the
 // ring of four input blocks limiting how far its stages overlap.
 // ---------------------------------------------------------------------------
@@ -432,6 +432,15 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
                 lw2 = __ldg(J.lw2 + l / J.n0);
             }
         }
+        // A wide band has its first block near the boundary only: the line's
+        // offset is then the middle sample, read while that block is under way.
+        const bool far = H > BD_BLK / 2;
+        if (far && l < J.nlines && (!mask || lo < hi)) {
+            const int mid = mask ? (lo + hi) >> 1 : n >> 1, o = XP ? 0 : l / J.n0;
+            off = __ldcg(XP ? J.data + (int64_t)l * n + mid
+                            : J.data + (int64_t)o * J.outer_stride + (l - o * J.n0) + mid * J.pos_stride);
+            if (mask) off -= b;
+        }
         double tP = 0.0, tL = 0.0;  // the line's sums
         // a block's functional weights, one position a lane, read a block ahead
         const float *fn = J.fn + 32 * half + lane;
@@ -458,16 +467,18 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
                 for (int i = 0; i < 16; ++i) v[i] = make_float2(f[2 * i * 32], f[(2 * i + 1) * 32]);
             }
             if (k == 0) {
-                // the line's offset: of two samples of its first block, the
-                // one nearer to zero
-                const int i1 = min(BD_BLK - 1, n - 1 + H), i0 = (H + i1) >> 1;
-                float s0 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i0));
-                float s1 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i1));
-                if (mask) {
-                    s0 = (i0 - H >= lo && i0 - H < hi) ? s0 - b : 0.0f;
-                    s1 = (i1 - H >= lo && i1 - H < hi) ? s1 - b : 0.0f;
+                if (!far) {
+                    // the line's offset: of two samples of its first block, the
+                    // one nearer to zero
+                    const int i1 = min(BD_BLK - 1, n - 1 + H), i0 = (H + i1) >> 1;
+                    float s0 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i0));
+                    float s1 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i1));
+                    if (mask) {
+                        s0 = (i0 - H >= lo && i0 - H < hi) ? s0 - b : 0.0f;
+                        s1 = (i1 - H >= lo && i1 - H < hi) ? s1 - b : 0.0f;
+                    }
+                    off = fabsf(s0) < fabsf(s1) ? s0 : s1;
                 }
-                off = fabsf(s0) < fabsf(s1) ? s0 : s1;
                 if (!(fabsf(off) < 1e30f)) off = 0.0f;
                 S.off[tile % BD_TILES][ln] = off;  // both halves store the same
             }
@@ -975,6 +986,29 @@ __global__ void __launch_bounds__(128) band_image_kernel(const BandAxis *axes)
         cur = nxt;
         nxt = t;
     }
+    // A weight w at distance j beyond H becomes w j^2 / H^2 at H and its excess
+    // over w is taken off the centre: the row keeps its sum and its variance
+    // (dropped, the tails of 1e-8 would cost 3e-7 of the variance a step).
+    // Half-widths for tails of 1e-8 are 8 % below those for 1e-10: ten substeps
+    // of radius 5.1 on average 2.66 -> 2.60 ms, the error against FP64 as before.
+    double at_lo = 0.0, at_hi = 0.0, centre = 0.0;
+    const double h2 = (double)X.H * X.H;
+    for (int q = lane; q < wd; q += 32) {
+        const int j = q - hw;
+        if (abs(j) <= X.H) continue;
+        const double f = cur[q] * ((double)j * j / h2);
+        (j < 0 ? at_lo : at_hi) += f;
+        centre += cur[q] - f;
+    }
+    at_lo = band_warp_sum(at_lo);
+    at_hi = band_warp_sum(at_hi);
+    centre = band_warp_sum(centre);
+    if (lane == 0 && hw > X.H) {
+        cur[hw - X.H] += at_lo;
+        cur[hw + X.H] += at_hi;
+        cur[hw] += centre;
+    }
+    __syncwarp();
     unsigned char *img = X.img + (size_t)im * X.ksteps * BD_STEP_BYTES;
     double sum = 0.0;
     for (int kk = lane; kk < X.ksteps * 16; kk += 32) {
@@ -1159,7 +1193,7 @@ int band_half_widths(const double *taps, int r, int mmax, int hmax, int *out)
         const int R = m * r;
         double tail = 0.0;
         int h = R;
-        while (h > 0 && tail + 2.0 * a[R + h] < 1e-10) {
+        while (h > 0 && tail + 2.0 * a[R + h] < 1e-8) {
             tail += 2.0 * a[R + h];
             --h;
         }

@@ -6,8 +6,8 @@
 // operators act on different axes and commute, so m substeps are
 // B_z^m B_y^m B_x^m: three passes over the field instead of 3 m.  B^m is a
 // banded n x n matrix, Toeplitz away from the line's ends; it is computed in
-// FP64 (its tails beyond a half-width H, whose sum is below 1e-10, are
-// dropped) and applied in blocks of 64 outputs.
+// FP64 (its tails beyond a half-width H, whose sum is below 1e-8, are
+// moved to H, keeping sum and variance) and applied in blocks of 64 outputs.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -85,8 +85,8 @@ struct BandInit {
 // whose 32-line runs would cross rows).
 bool band_encode_map(const BandJob &j, int nz, CUtensorMap *m);
 
-// out[m - 1]: the half-width of the m-fold kernel (taps: 2 r + 1 of FP64) at
-// which its dropped tails sum to less than 1e-10, rounded up to a multiple of
+// out[m - 1]: the half-width of the m-fold kernel (taps: 2 r + 1 of FP64) beyond
+// which its tails sum to less than 1e-8, rounded up to a multiple of
 // 4, for m = 1, 2, ... while it is at most hmax; returns the number of those.
 int band_half_widths(const double *taps, int r, int mmax, int hmax, int *out);
 
