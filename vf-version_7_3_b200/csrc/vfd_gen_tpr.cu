@@ -20,9 +20,14 @@
 // passes (NL consecutive lines, 128 bytes for NL = 16), positions n2 (the
 // first pass) or bins k1 (the C2R first pass) for the row passes.
 //
-// Shared memory: the tile, then (unused room for tw[m] = w_F^m) the pass
-// twiddles w_F^(k1 n2) in both orders (T[k1 F2 + n2] for lanes along n2,
-// Tt[n2 F1 + k1] for lanes along k1, so that neither gather conflicts).  The
+// What bounds them (512x256x384 x 8 fields with the update, 6.8 ms): issue
+// slots (45-65 % busy) and the latency of tiles of four CTAs an SM, at 2-3.7
+// TB/s; the row passes' index arithmetic and predicates are therefore kept to
+// one range test a position and one line's two rows a split step (x passes
+// 3.65 -> 3.2 ms).
+// Shared memory: the tile, then the pass twiddles w_F^(k1 n2) in the order the
+// pass reads them (T[k1 F2 + n2] for lanes along n2, C2R T[n2 F1 + k1] for
+// lanes along k1, so that neither gather conflicts).  The
 // first pass's global loads are issued before the twiddle staging and its
 // barrier, so they overlap.  The fused z pass reads its spectrum K straight
 // from global memory in pass B (lanes along lines: coalesced), which leaves
@@ -50,46 +55,47 @@ __device__ __forceinline__ double tpr_warp_sum(double v)
     return v;
 }
 
-// Block sum added to *dst (skipped when dst is NULL or the sum is zero).
-__device__ __forceinline__ void tpr_block_sum(double v, double *dst, double *red)
+// Block sums of N values added to *dst[i] (skipped when dst[i] is NULL or the
+// sum is zero); red: 32 N doubles.
+template <int N>
+__device__ __forceinline__ void tpr_block_sums(const double (&v)[N], double *const (&dst)[N], double *red)
 {
-    v = tpr_warp_sum(v);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = (l < (int)(blockDim.x >> 5)) ? red[l] : 0.0;
-        v = tpr_warp_sum(v);
-        if (l == 0 && v != 0.0 && dst) atomicAdd(dst, v);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const double t = tpr_warp_sum(v[i]);
+        if (l == 0) red[32 * i + w] = t;
     }
     __syncthreads();
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if (w == i % nw && dst[i]) {
+            const double t = tpr_warp_sum(l < nw ? red[32 * i + l] : 0.0);
+            if (l == 0 && t != 0.0) atomicAdd(dst[i], t);
+        }
 }
 
 __device__ __forceinline__ float2 c_conj_mul(float2 a, float2 w) { return c_mul(a, make_float2(w.x, -w.y)); }
 
 struct TprSmem {
-    float2 *S, *tw, *T, *Tt;
+    float2 *S, *T;
 };
 __device__ __forceinline__ TprSmem tpr_smem_layout(float2 *base, int F, int NL)
 {
     TprSmem m;
     m.S = base;
-    m.tw = base + F * (NL + 1) + TPR_MAX;
-    m.T = m.tw + F;
-    m.Tt = m.T + F;
+    m.T = base + F * (NL + 1) + TPR_MAX;
     return m;
 }
-// T and Tt from the global table (no barrier: the caller's follows; the
-// small DFTs take their twiddles as immediates, so tw is not staged).
-// i / d as (i * ceil(2^21 / d)) >> 21, exact for i < 65536 and d <= 32.
-__device__ __forceinline__ void stage_twiddles(const TprSmem &m, const float2 *__restrict__ g, int F, int F1, int F2)
+// T from the global table, T[a * B + b] = w^(a b) (no barrier: the caller's
+// follows; the small DFTs take their twiddles as immediates).
+// i / B as (i * ceil(2^21 / B)) >> 21, exact for i < 65536 and B <= 32.
+__device__ __forceinline__ void stage_twiddles(const TprSmem &m, const float2 *__restrict__ g, int F, int B)
 {
-    const int m1 = ((1 << 21) + F1 - 1) / F1, m2 = ((1 << 21) + F2 - 1) / F2;
+    const int mb = ((1 << 21) + B - 1) / B;
     for (int i = threadIdx.x; i < F; i += blockDim.x) {
-        const int a = (i * m2) >> 21, b = i - a * F2;  // T: k1 = a, n2 = b
+        const int a = (i * mb) >> 21, b = i - a * B;
         m.T[i] = g[a * b];
-        const int c = (i * m1) >> 21, d = i - c * F1;  // Tt: n2 = c, k1 = d
-        m.Tt[i] = g[c * d];
     }
 }
 
@@ -97,6 +103,11 @@ __device__ __forceinline__ void tpr_cp8(float2 *smem, const float2 *gmem, bool v
 {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void tpr_cp16(float2 *smem, const float2 *gmem, bool valid)
+{
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void tpr_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void tpr_cp_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
@@ -125,7 +136,7 @@ __device__ __forceinline__ void col_a(const GenColPass &p, const TprSmem &m, con
             v[n1] = (lok && x < p.nload) ? col[(int64_t)x * p.pos_stride] : make_float2(0.f, 0.f);
         }
     }
-    stage_twiddles(m, p.tw, F, F1, F2);
+    stage_twiddles(m, p.tw, F, F2);
     __syncthreads();
     if (!active) return;
     tpr_dft<N, false>(v);
@@ -198,7 +209,7 @@ __device__ __forceinline__ void col_bi(const GenColPass &p, const TprSmem &m, co
             v[k2] = (lok && bin < p.nload) ? col[(int64_t)bin * p.pos_stride] : make_float2(0.f, 0.f);
         }
     }
-    stage_twiddles(m, p.tw, F, F1, F2);
+    stage_twiddles(m, p.tw, F, F2);
     __syncthreads();
     if (active) col_b_inverse<N, NL>(m, v, k1, F1, GS, l);
 }
@@ -317,48 +328,60 @@ __global__ void __launch_bounds__(MAXT, MINB) c2c_tpr_kernel(const GenColPass p_
 
 struct RowRef {
     bool ok;     // row < nrows
-    bool in;     // ok, and inside the padding box in (r1, r2) when padding is fused
-    int64_t off; // r1 * s1 + r2 * s2
+    int r1, r2;  // its indexes
 };
-__device__ __forceinline__ RowRef row_ref(const GenRowPass &p, int row, int64_t s1, int64_t s2)
+__device__ __forceinline__ RowRef row_ref(const GenRowPass &p, int row)
 {
-    RowRef r{row < p.nrows, false, 0};
-    if (r.ok) {
-        const int r1 = row % p.rows_per_plane, r2 = row / p.rows_per_plane;
-        r.off = (int64_t)r1 * s1 + (int64_t)r2 * s2;
-        r.in = !p.fuse_pad || (r1 >= p.box_lo[1] && r1 < p.box_hi[1] && r2 >= p.box_lo[2] && r2 < p.box_hi[2]);
-    }
-    return r;
+    const int r2 = row / p.rows_per_plane;
+    return RowRef{row < p.nrows, row - r2 * p.rows_per_plane, r2};
 }
 
 // R2C A (first pass): positions n2 + F2 n1 of rows a and b (the padding
 // rule v = u - b inside the box, 0 outside, when fused) loaded, twiddles
-// staged, barrier, DFT F1, times w^(k1 n2), slots.  Returns the FP64 sum of
-// the values (the input mass).
+// staged, barrier, DFT F1, times w^(k1 n2), slots.  coff: the rows' offsets in
+// the spectrum, -1 past the last row.  Returns the FP64 sum of the values (the
+// input mass).
 template <int N, int NL>
-__device__ __forceinline__ double r2c_a(const GenRowPass &p, const TprSmem &m, int r0, int l, int n2, int F2, int GS,
-                                        bool active)
+__device__ __forceinline__ double r2c_a(const GenRowPass &p, const TprSmem &m, int64_t *coff, int r0, int l, int n2,
+                                        int F2, int GS, bool active)
 {
     const int F1 = N, F = F1 * F2;
     float2 v[N];
     double acc_a = 0.0, acc_b = 0.0;
     if (active) {
-        const RowRef ra = row_ref(p, r0 + l, p.r_s1, p.r_s2), rb = row_ref(p, r0 + NL + l, p.r_s1, p.r_s2);
-        const float *sa = p.rsrc + ra.off, *sb = p.rsrc + rb.off;
+        const RowRef ra = row_ref(p, r0 + l), rb = row_ref(p, r0 + NL + l);
+        if (n2 == 0) {
+            coff[l] = ra.ok ? (int64_t)ra.r1 * p.c_s1 + (int64_t)ra.r2 * p.c_s2 : -1;
+            coff[NL + l] = rb.ok ? (int64_t)rb.r1 * p.c_s1 + (int64_t)rb.r2 * p.c_s2 : -1;
+        }
+        // positions lo <= x < lo + wa (wb) are read, the others are b: less b,
+        // those are the padding rule's zeros
+        const bool pad = p.fuse_pad;
+        const int lo = pad ? p.box_lo[0] : 0, hi = pad ? min(p.nload, p.box_hi[0]) : p.nload;
+        const float b = pad ? p.b : 0.0f;
+        auto width = [&](const RowRef &r) {
+            const bool in = r.ok && (!pad || (r.r1 >= p.box_lo[1] && r.r1 < p.box_hi[1] && r.r2 >= p.box_lo[2] &&
+                                              r.r2 < p.box_hi[2]));
+            return (unsigned)(in ? max(hi - lo, 0) : 0);
+        };
+        const unsigned wa = width(ra), wb = width(rb);
+        const float *sa = p.rsrc + (int64_t)ra.r1 * p.r_s1 + (int64_t)ra.r2 * p.r_s2 + n2;
+        const float *sb = p.rsrc + (int64_t)rb.r1 * p.r_s1 + (int64_t)rb.r2 * p.r_s2 + n2;
 #pragma unroll
         for (int n1 = 0; n1 < N; ++n1) {
-            const int x = n2 + F2 * n1;
-            const bool xin = x < p.nload && (!p.fuse_pad || (x >= p.box_lo[0] && x < p.box_hi[0]));
-            v[n1].x = (ra.in && xin) ? sa[x] : 0.0f;
-            v[n1].y = (rb.in && xin) ? sb[x] : 0.0f;
+            const int d = F2 * n1;
+            v[n1] = make_float2(b, b);
+            if ((unsigned)(n2 - lo + d) < wa) v[n1].x = sa[d];
+            if ((unsigned)(n2 - lo + d) < wb) v[n1].y = sb[d];
         }
-        if (p.fuse_pad) {
+        if (fabsf(b) < 3.0e38f) {
+#pragma unroll
+            for (int n1 = 0; n1 < N; ++n1) v[n1] = make_float2(v[n1].x - b, v[n1].y - b);
+        } else {  // no zeros from b - b
 #pragma unroll
             for (int n1 = 0; n1 < N; ++n1) {
-                const int x = n2 + F2 * n1;
-                const bool xin = x < p.nload && x >= p.box_lo[0] && x < p.box_hi[0];
-                v[n1].x = (ra.in && xin) ? v[n1].x - p.b : 0.0f;
-                v[n1].y = (rb.in && xin) ? v[n1].y - p.b : 0.0f;
+                const unsigned x = (unsigned)(n2 - lo + F2 * n1);
+                v[n1] = make_float2(x < wa ? v[n1].x - b : 0.0f, x < wb ? v[n1].y - b : 0.0f);
             }
         }
         if (p.mass_in) {
@@ -381,7 +404,7 @@ __device__ __forceinline__ double r2c_a(const GenRowPass &p, const TprSmem &m, i
             acc_b = (double)tb[0];
         }
     }
-    stage_twiddles(m, p.tw, F, F1, F2);
+    stage_twiddles(m, p.tw, F, F2);
     __syncthreads();
     if (active) {
         tpr_dft<N, false>(v);
@@ -423,6 +446,7 @@ __global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p_
     constexpr int LS = NL + 1, NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
     __shared__ double red[32];
+    __shared__ int64_t coff[NR];
     const int F = p.plan.F, F1 = f1, F2 = F / f1;
     const int GS = F2 * LS + ((F2 & 1) ^ 1);
     const TprSmem m = tpr_smem_layout(tsm, F, NL);
@@ -434,7 +458,7 @@ __global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p_
         const int n2 = threadIdx.x % F2, l = threadIdx.x / F2;
         switch (F1) {
 #define VFD_R2C_A(n) \
-    case n: if constexpr (n <= MAXN) acc = r2c_a<n, NL>(p, m, r0, l, n2, F2, GS, l < NL); break;
+    case n: if constexpr (n <= MAXN) acc = r2c_a<n, NL>(p, m, coff, r0, l, n2, F2, GS, l < NL); break;
             VFD_TPR_SIZES(VFD_R2C_A)
 #undef VFD_R2C_A
         default: break;
@@ -454,23 +478,21 @@ __global__ void __launch_bounds__(MAXT, MINB) r2c_tpr_kernel(const GenRowPass p_
     }
     __syncthreads();
 
-    // split the two real rows' half spectra: warp per output row, lanes along k
+    // split the two real rows' half spectra: 32 bins of a line's two rows a
+    // warp, lanes along k
     const int Fh = F / 2 + 1, NW = blockDim.x >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int q = warp; q < NR; q += NW) {
-        const int rr = r0 + q;
-        if (rr >= p.nrows) continue;
-        const int ln = q % NL;
-        const int s1 = rr % p.rows_per_plane, s2 = rr / p.rows_per_plane;
-        float2 *dst = p.cdst + (int64_t)s1 * p.c_s1 + (int64_t)s2 * p.c_s2;
-        for (int k = lane; k < Fh; k += 32) {
-            const float2 z = m.S[k * LS + ln];
-            const float2 zc = m.S[(k == 0 ? 0 : F - k) * LS + ln];  // Z(-k)
-            dst[k] = q < NL ? make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y))    // A(k)
-                            : make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));  // B(k)
-        }
+    const int items = NL * ((Fh + 31) >> 5);
+    for (int i = warp; i < items; i += NW) {
+        const int ln = i % NL, k = (i / NL) * 32 + lane;
+        if (k >= Fh) continue;
+        const int64_t oa = coff[ln], ob = coff[NL + ln];
+        const float2 z = m.S[k * LS + ln];
+        const float2 zc = m.S[(k == 0 ? 0 : F - k) * LS + ln];  // Z(-k)
+        if (oa >= 0) p.cdst[oa + k] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y - zc.y));   // A(k)
+        if (ob >= 0) p.cdst[ob + k] = make_float2(0.5f * (z.y + zc.y), -0.5f * (z.x - zc.x));  // B(k)
     }
-    tpr_block_sum(acc, p.mass_in, red);
+    tpr_block_sums<1>({acc}, {p.mass_in}, red);
 }
 
 // C2R B' (first pass).  The half spectra of the tile's 2 NL rows are first
@@ -485,16 +507,21 @@ template <int N, int NL>
 __device__ __forceinline__ void c2r_b(const GenRowPass &p, const TprSmem &m, int r0, int l, int k1, int F1, int GS,
                                       bool active)
 {
-    const int F2 = N, F = F1 * F2, H = F / 2, Fh = H + 1;
+    const int F2 = N, F = F1 * F2, H = F / 2, Fh = (H + 2) & ~1;  // bins of a row, rounded up to whole 16 bytes
     const int NW = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float2 *St = m.S;
+    // rows that start on 16-byte boundaries and have room for Fh bins: two bins a copy
+    const bool pairs = ((p.c_s1 | p.c_s2 | (reinterpret_cast<uintptr_t>(p.csrc) >> 3)) & 1) == 0;
     for (int q = warp; q < 2 * NL; q += NW) {
-        const RowRef r = row_ref(p, r0 + q, p.c_s1, p.c_s2);
-        const float2 *src = p.csrc + r.off;
-        for (int k = lane; k < Fh; k += 32) tpr_cp8(&St[q * Fh + k], r.ok ? src + k : p.csrc, r.ok);
+        const RowRef r = row_ref(p, r0 + q);
+        const float2 *src = r.ok ? p.csrc + (int64_t)r.r1 * p.c_s1 + (int64_t)r.r2 * p.c_s2 : p.csrc;
+        if (pairs)
+            for (int k = 2 * lane; k < Fh; k += 64) tpr_cp16(&St[q * Fh + k], r.ok ? src + k : src, r.ok);
+        else
+            for (int k = lane; k <= H; k += 32) tpr_cp8(&St[q * Fh + k], r.ok ? src + k : src, r.ok);
     }
     tpr_cp_commit();
-    stage_twiddles(m, p.tw, F, F1, F2);
+    stage_twiddles(m, p.tw, F, F1);
     tpr_cp_wait_all();
     __syncthreads();
     float2 v[N];
@@ -509,7 +536,7 @@ __device__ __forceinline__ void c2r_b(const GenRowPass &p, const TprSmem &m, int
             v[k2] = up ? make_float2(A.x + B.y, B.x - A.y) : make_float2(A.x - B.y, A.y + B.x);
         }
         tpr_dft<N, true>(v);
-        const float2 *t = m.Tt + k1;  // Tt[n2 F1 + k1], lanes along k1
+        const float2 *t = m.T + k1;  // T[n2 F1 + k1], lanes along k1
 #pragma unroll
         for (int n2 = 1; n2 < N; ++n2) v[n2] = c_conj_mul(v[n2], t[n2 * F1]);
     }
@@ -525,32 +552,16 @@ struct C2rSums {
     double leak = 0.0, conv = 0.0, out = 0.0;
 };
 
-// One real output value at x of a row: the crop / update epilogue; the
-// values for the mass totals are added to the FP32 group sums gc and go.
-// UPD: dval is the update's dChem value there, drow its row (zeroed).
-template <bool UPD>
-__device__ __forceinline__ void c2r_store(const GenRowPass &p, float t, float *dst, float *drow, float dval, int x,
-                                          float &gc, float &go)
-{
-    if (p.fuse_crop) {
-        gc += t;
-        t = p.keep * (t + p.b * p.k0);
-        if (UPD) {
-            t = t * p.upd_scale + dval;
-            drow[x] = 0.0f;
-        } else if (p.fuse_update) {
-            t *= p.upd_scale;
-        }
-        go += t;
-    }
-    dst[x] = t;
-}
+// What the C2R pass does with its real values: store them, crop (out = keep *
+// (t + b k0), times the update's retention), or crop with the update's dChem
+// added and zeroed.
+enum C2rEpilogue { C2R_PLAIN, C2R_CROP, C2R_UPDATE };
 
 // C2R A': slots of group n2 -> inverse DFT F1 -> positions n2 + F2 n1 of rows
 // a (real part) and b (imaginary part); positions >= nstore go to the leak
 // sum.  The mass sums run in FP32 over groups of 4 positions, each group
 // widened once into the FP64 totals.
-template <int N, int NL, bool UPD>
+template <int N, int NL, int EPI>
 __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int r0, int l, int n2, int F2, int GS,
                                       C2rSums &s)
 {
@@ -559,32 +570,58 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
 #pragma unroll
     for (int k1 = 0; k1 < N; ++k1) v[k1] = src[k1 * GS];
     tpr_dft<N, true>(v);
-    const RowRef ra = row_ref(p, r0 + l, p.r_s1, p.r_s2), rb = row_ref(p, r0 + NL + l, p.r_s1, p.r_s2);
-    float *da = p.rdst + ra.off, *db = p.rdst + rb.off;
-    float *ua = UPD ? p.dchem + ra.off : nullptr, *ub = UPD ? p.dchem + rb.off : nullptr;
+    const RowRef ra = row_ref(p, r0 + l), rb = row_ref(p, r0 + NL + l);
+    const int64_t oa = (int64_t)ra.r1 * p.r_s1 + (int64_t)ra.r2 * p.r_s2 + n2;
+    const int64_t ob = (int64_t)rb.r1 * p.r_s1 + (int64_t)rb.r2 * p.r_s2 + n2;
+    float *da = p.rdst + oa, *db = p.rdst + ob;
+    // dChem's rows lie as the field's, at one distance: two row pointers less in
+    // registers (the update's spills 776 -> 390 bytes)
+    const int64_t du = EPI == C2R_UPDATE ? reinterpret_cast<intptr_t>(p.dchem) - reinterpret_cast<intptr_t>(p.rdst) : 0;
+    auto dchem = [&](const float *x) {
+        float d;
+        asm("ld.global.f32 %0, [%1];\n" : "=f"(d) : "l"(reinterpret_cast<intptr_t>(x) + du));
+        return d;
+    };
+    // takes the value read, so that the read comes first
+    auto zero = [&](const float *x, float was) {
+        asm volatile("st.global.f32 [%0], %1;\n" ::"l"(reinterpret_cast<intptr_t>(x) + du), "f"(0.0f), "f"(was));
+    };
+    // positions left from n2 on in the stored part, in the row and in rows a, b
+    const int left = p.nstore - n2, la = ra.ok ? left : 0, lb = rb.ok ? left : 0;
+    const float keep = p.keep, bk = p.b, k0 = p.k0, us = p.fuse_update ? p.upd_scale : 1.0f;
     float gc = 0.0f, go = 0.0f, gl = 0.0f;
     // The update's dChem values, read four positions ahead of the stores: each
     // store may alias the next load, so loads between the stores waited for one
-    // another (48 in a row: 512x256x384 x 8, x 26.8 ms a tick; like this 3.5).
+    // another (48 in a row: 512x256x384 x 8, x 26.8 ms a tick; like this 3.2;
+    // six ahead 3.4; row a's before row b's 3.7).
     float qa[4], qb[4];
     auto ahead = [&](int n1) {
-        const int x = n2 + F2 * n1;
-        qa[n1 & 3] = (UPD && ra.ok && x < p.nstore) ? ua[x] : 0.0f;
-        qb[n1 & 3] = (UPD && rb.ok && x < p.nstore) ? ub[x] : 0.0f;
+        const int d = F2 * n1;
+        qa[n1 & 3] = 0.0f;
+        qb[n1 & 3] = 0.0f;
+        if (EPI == C2R_UPDATE && d < la) qa[n1 & 3] = dchem(da + d);
+        if (EPI == C2R_UPDATE && d < lb) qb[n1 & 3] = dchem(db + d);
+    };
+    auto put = [&](float t, float *dst, float dval, int d) {
+        if (EPI != C2R_PLAIN) {
+            gc += t;
+            t = keep * (t + bk * k0);
+            t = EPI == C2R_UPDATE ? t * us + dval : t * us;
+            if (EPI == C2R_UPDATE) zero(dst + d, dval);
+            go += t;
+        }
+        dst[d] = t;
     };
 #pragma unroll
     for (int n1 = 0; n1 < (N < 4 ? N : 4); ++n1) ahead(n1);
 #pragma unroll
     for (int n1 = 0; n1 < N; ++n1) {
-        const int x = n2 + F2 * n1;
+        const int d = F2 * n1;
         const float ea = qa[n1 & 3], eb = qb[n1 & 3];
         if (n1 + 4 < N) ahead(n1 + 4);
-        if (x < p.nstore) {
-            if (ra.ok) c2r_store<UPD>(p, v[n1].x, da, ua, ea, x, gc, go);
-            if (rb.ok) c2r_store<UPD>(p, v[n1].y, db, ub, eb, x, gc, go);
-        } else {
-            gl += v[n1].x + v[n1].y;
-        }
+        if (d < la) put(v[n1].x, da, ea, d);
+        if (d < lb) put(v[n1].y, db, eb, d);
+        if (d >= left) gl += v[n1].x + v[n1].y;
         if ((n1 & 3) == 3 || n1 == N - 1) {
             s.conv += (double)gc;
             s.out += (double)go;
@@ -594,7 +631,7 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
     }
 }
 
-template <int NL, int MAXT, int MINB, int MAXN, bool UPD, bool MF>
+template <int NL, int MAXT, int MINB, int MAXN, int EPI, bool MF>
 __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_, const GenFields ff, int f1)
 {
     grid_dep_launch();
@@ -602,7 +639,7 @@ __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_
     const GenRowPass p = MF ? tpr_row_field(p_, ff) : p_;
     constexpr int NR = 2 * NL;
     extern __shared__ __align__(16) float2 tsm[];
-    __shared__ double red[32];
+    __shared__ double red[3 * 32];
     const int F = p.plan.F, F1 = f1, F2 = F / f1;
     const int GS = F2 * (NL + 1) + ((F2 & 1) ^ 1);
     const TprSmem m = tpr_smem_layout(tsm, F, NL);
@@ -626,16 +663,14 @@ __global__ void __launch_bounds__(MAXT, MINB) c2r_tpr_kernel(const GenRowPass p_
         if (l < NL) {
             switch (F1) {
 #define VFD_C2R_A(n) \
-    case n: if constexpr (n <= MAXN) c2r_a<n, NL, UPD>(p, m, r0, l, n2, F2, GS, s); break;
+    case n: if constexpr (n <= MAXN) c2r_a<n, NL, EPI>(p, m, r0, l, n2, F2, GS, s); break;
                 VFD_TPR_SIZES(VFD_C2R_A)
 #undef VFD_C2R_A
             default: break;
             }
         }
     }
-    tpr_block_sum(s.leak, p.mass_leak, red);
-    tpr_block_sum(s.conv, p.mass_conv, red);
-    tpr_block_sum(s.out, p.mass_out, red);
+    tpr_block_sums<3>({s.leak, s.conv, s.out}, {p.mass_leak, p.mass_conv, p.mass_out}, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -682,8 +717,8 @@ static int tpr_threads(int F, int f1, int NL)
     return (NL * g + 31) / 32 * 32;
 }
 
-// the tile, tw, T and Tt
-static size_t tpr_smem(int F, int NL) { return ((size_t)F * (NL + 1) + TPR_MAX + 3 * (size_t)F) * sizeof(float2); }
+// the tile and T
+static size_t tpr_smem(int F, int NL) { return ((size_t)F * (NL + 2) + TPR_MAX) * sizeof(float2); }
 
 // The largest dynamic shared memory, once per kernel (one instantiation per
 // kernel, so one flag each) and CUDA context.
@@ -699,25 +734,28 @@ static cudaError_t tpr_attr()
     return e;
 }
 
-template <int NL, int MAXT, int MINB, int MAXN, bool MF>
-static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream_t st, const GenFields &ff)
+template <auto KERNEL>
+static cudaError_t rows_kernel(const GenRowPass &p, int f1, int NL, int MAXT, cudaStream_t st, const GenFields &ff)
 {
-    const bool upd = p.fuse_crop && p.fuse_update && ff.dchem[0];
-    cudaError_t e = !inverse ? tpr_attr<r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>>()
-                    : upd    ? tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF>>()
-                             : tpr_attr<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF>>();
+    cudaError_t e = tpr_attr<KERNEL>();
     if (e != cudaSuccess) return e;
     const dim3 blocks((unsigned)((p.nrows + 2 * NL - 1) / (2 * NL)), (unsigned)ff.n);
     if (p.nrows <= 0) return cudaSuccess;
     const int nt = tpr_threads(p.plan.F, f1, NL);
     const size_t sm = tpr_smem(p.plan.F, NL);
     if (nt > MAXT || sm > axis_smem_limit()) return cudaErrorInvalidConfiguration;
-    e = launch_overlapped((int64_t)blocks.x * blocks.y <= TPR_OVERLAP, !inverse ? r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>
-                          : upd    ? c2r_tpr_kernel<NL, MAXT, MINB, MAXN, true, MF>
-                                   : c2r_tpr_kernel<NL, MAXT, MINB, MAXN, false, MF>,
-                          blocks, (unsigned)nt, sm, st, p, ff, f1);
+    e = launch_overlapped((int64_t)blocks.x * blocks.y <= TPR_OVERLAP, KERNEL, blocks, (unsigned)nt, sm, st, p, ff, f1);
     note_launch();
     return e == cudaSuccess ? cudaGetLastError() : e;
+}
+template <int NL, int MAXT, int MINB, int MAXN, bool MF>
+static cudaError_t rows_nl(const GenRowPass &p, int f1, bool inverse, cudaStream_t st, const GenFields &ff)
+{
+    if (!inverse) return rows_kernel<r2c_tpr_kernel<NL, MAXT, MINB, MAXN, MF>>(p, f1, NL, MAXT, st, ff);
+    if (!p.fuse_crop) return rows_kernel<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, C2R_PLAIN, MF>>(p, f1, NL, MAXT, st, ff);
+    if (p.fuse_update && ff.dchem[0])
+        return rows_kernel<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, C2R_UPDATE, MF>>(p, f1, NL, MAXT, st, ff);
+    return rows_kernel<c2r_tpr_kernel<NL, MAXT, MINB, MAXN, C2R_CROP, MF>>(p, f1, NL, MAXT, st, ff);
 }
 
 template <int NL, int MAXT, int MINB, int MAXN, bool MF>

@@ -424,7 +424,7 @@ __global__ void wrap_window_kernel(float *P, const float *w, int kw, int kh, int
 // K[kz][ky][kx] = Gx(kx) Gy(ky) Gz(kz) for a separable Gaussian, from the
 // per-axis multipliers G(k)/F (so the F factors are restored here).
 __global__ void outer_spectrum_kernel(float2 *K, const float *sx, const float *sy, const float *sz, int Fx,
-                                      int Fy, int Fz, int Fxh)
+                                      int Fy, int Fz, int Fxh, int Fxs)
 {
     const int64_t n = (int64_t)Fxh * Fy * Fz;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -432,7 +432,7 @@ __global__ void outer_spectrum_kernel(float2 *K, const float *sx, const float *s
         const int64_t r = i / Fxh;
         const int ky = (int)(r % Fy), kz = (int)(r / Fy);
         const double v = (double)sx[kx] * Fx * (double)sy[ky] * Fy * (double)sz[kz] * Fz;
-        K[i] = make_float2((float)v, 0.0f);
+        K[kx + Fxs * r] = make_float2((float)v, 0.0f);
     }
 }
 
@@ -660,10 +660,10 @@ cudaError_t launch_sum(const float *P, int64_t n, double *out, cudaStream_t st)
 }
 
 cudaError_t launch_outer_spectrum(float2 *K, const float *sx, const float *sy, const float *sz, int Fx, int Fy,
-                                  int Fz, cudaStream_t st)
+                                  int Fz, int Fxs, cudaStream_t st)
 {
     const int Fxh = Fx / 2 + 1;
-    outer_spectrum_kernel<<<grid_for((int64_t)Fxh * Fy * Fz), 256, 0, st>>>(K, sx, sy, sz, Fx, Fy, Fz, Fxh);
+    outer_spectrum_kernel<<<grid_for((int64_t)Fxh * Fy * Fz), 256, 0, st>>>(K, sx, sy, sz, Fx, Fy, Fz, Fxh, Fxs);
     note_launch();
     return cudaGetLastError();
 }

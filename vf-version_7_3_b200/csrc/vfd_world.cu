@@ -425,8 +425,9 @@ struct vfd_world {
     // general 3D methods (VFD_METHOD_FFT3D / VFD_METHOD_PLAIN)
     int method = VFD_METHOD_SEPARABLE;
     int Fxh = 0;
+    int Fxs = 0;                     // elements between the spectra's rows
     int gvar[3] = {0, 0, 0};         // kernel variants of the x rows, y and z columns
-    float2 *d_kspec = nullptr;       // [f][Fz][Fy][Fxh], unscaled K
+    float2 *d_kspec = nullptr;       // [f][Fz][Fy][Fxs], unscaled K
     float2 *d_C = nullptr;           // spectrum scratch of gen_group fields
     int gen_group = 1;               // fields a launch of the general transform holds
     float *d_P = nullptr;            // full real grid scratch (plain)
@@ -576,14 +577,22 @@ static bool os_enabled()
 
 static bool os_plain_staging(const OsJob &j);
 
+// Elements between the rows of a general world's spectra: rows start on
+// 64-byte boundaries, so that the column passes' tiles (8 lines, 64 bytes a
+// position) are whole 32-byte sectors and the C2R pass copies two bins at a
+// time (512x256x384 x 8, rows of 289 bins: y and z passes 3.80 -> 3.68 ms a
+// tick).  The plain method keeps the packed layout its elementwise steps run
+// over.
+static int spectrum_stride(int method, int Fxh) { return method == VFD_METHOD_FFT3D ? (Fxh + 7) / 8 * 8 : Fxh; }
+
 // Fields a launch of the fused general transform holds: as many as keep the
 // launch's spectra within 64 MB, half of L2, so that the next pass finds them
 // there.  A field of its own launch left the chip idle on small grids (75x50x33 x
-// 8: 5 launches a field of 100-360 CTAs each, 400 us a tick; together 60); where
+// 8: 5 launches a field of 100-360 CTAs each, 400 us a tick; together 41); where
 // one field's spectra exceed that, the launches are full and share nothing.
 static int general_group(const vfd_world *w)
 {
-    const int64_t bytes = (int64_t)sizeof(float2) * w->Fxh * w->F[1] * w->nz;
+    const int64_t bytes = (int64_t)sizeof(float2) * w->Fxs * w->F[1] * w->nz;
     return (int)std::max<int64_t>(1, std::min<int64_t>(std::min(w->nf, GEN_FIELDS), ((int64_t)64 << 20) / bytes));
 }
 
@@ -1224,6 +1233,7 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         }
     if (general) {
         w->Fxh = w->F[0] / 2 + 1;
+        w->Fxs = spectrum_stride(w->method, w->Fxh);
         w->gvar[0] = w->variant[0];
         for (int a = 1; a < 3; ++a) {
             w->gvar[a] = pick_variant(std::vector<FftPlan>{w->plan[a]}, 16);
@@ -1254,16 +1264,16 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
     if ((e = cudaMemset(w->d_err, 0, sizeof(int))) != cudaSuccess) return bail(e, "cudaMemset err");
     if ((e = cudaMalloc(&w->d_dep, sizeof(DepositJob) * 2 * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc deposit jobs");
     if (general) {
-        const int64_t nk = (int64_t)w->Fxh * w->F[1] * w->F[2];
+        const int64_t nk = (int64_t)w->Fxs * w->F[1] * w->F[2];
         if ((e = cudaMalloc(&w->d_kspec, sizeof(float2) * nk * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc spectra");
         for (int f = 0; f < w->nf; ++f) {
             const float *sp = w->d_spec + (int64_t)f * 3 * w->Fmax;
             if ((e = launch_outer_spectrum(w->d_kspec + nk * f, sp, sp + w->Fmax, sp + 2 * w->Fmax, w->F[0], w->F[1],
-                                           w->F[2], 0)) != cudaSuccess)
+                                           w->F[2], w->Fxs, 0)) != cudaSuccess)
                 return bail(e, "outer spectrum");
         }
         w->k0.assign(w->nf, 1.0f);
-        const int64_t nc = (w->method == VFD_METHOD_PLAIN) ? nk : (int64_t)w->Fxh * w->F[1] * w->nz;
+        const int64_t nc = (w->method == VFD_METHOD_PLAIN) ? nk : (int64_t)w->Fxs * w->F[1] * w->nz;
         if (w->method == VFD_METHOD_FFT3D) w->gen_group = general_group(w);
         if ((e = cudaMalloc(&w->d_C, sizeof(float2) * nc * w->gen_group)) != cudaSuccess) return bail(e, "cudaMalloc spectrum scratch");
         if (w->method == VFD_METHOD_PLAIN) {
@@ -1330,9 +1340,9 @@ vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes)
     b += (sizeof(int32_t) + sizeof(float)) * (size_t)w->src_cap;
     for (const auto &kv : w->band_plans) b += kv.second.bytes;
     if (w->method != VFD_METHOD_SEPARABLE) {
-        const size_t nk = (size_t)w->Fxh * w->F[1] * w->F[2];
+        const size_t nk = (size_t)w->Fxs * w->F[1] * w->F[2];
         b += sizeof(float2) * nk * w->nf;
-        b += sizeof(float2) * ((w->method == VFD_METHOD_PLAIN) ? nk : (size_t)w->Fxh * w->F[1] * w->nz) * w->gen_group;
+        b += sizeof(float2) * ((w->method == VFD_METHOD_PLAIN) ? nk : (size_t)w->Fxs * w->F[1] * w->nz) * w->gen_group;
         if (w->method == VFD_METHOD_PLAIN) b += sizeof(float) * (size_t)w->F[0] * w->F[1] * w->F[2];
     }
     *bytes = b;
@@ -1418,11 +1428,11 @@ static GenColPass col_pass(const vfd_world *w, int a, float2 *data, int nouter, 
     c.nlines = w->Fxh;
     c.nouter = nouter;
     if (a == PASS_Y) {
-        c.outer_stride = (int64_t)w->F[1] * w->Fxh;
-        c.pos_stride = w->Fxh;
+        c.outer_stride = (int64_t)w->F[1] * w->Fxs;
+        c.pos_stride = w->Fxs;
     } else {
-        c.outer_stride = w->Fxh;
-        c.pos_stride = (int64_t)w->F[1] * w->Fxh;
+        c.outer_stride = w->Fxs;
+        c.pos_stride = (int64_t)w->F[1] * w->Fxs;
     }
     c.nload = nload;
     c.nstore = nstore;
@@ -1446,7 +1456,7 @@ vfd_status vfd_set_window(vfd_world *w, int field, const float *window, int kw, 
         std::max(cz, kd - 1 - cz) > Fz - w->nz)
         return fail(w, VFD_ERR_INVALID_ARG, "window wider than the FFT padding; pass larger fft lengths");
     DeviceGuard g(w->device);
-    const int64_t nk = (int64_t)w->Fxh * Fy * Fz;
+    const int64_t nk = (int64_t)w->Fxs * Fy * Fz;
     const int64_t np = (int64_t)Fx * Fy * Fz;
     const int64_t nwin = (int64_t)kw * kh * kd;
     float *P = nullptr, *dw = nullptr;
@@ -1472,8 +1482,8 @@ vfd_status vfd_set_window(vfd_world *w, int field, const float *window, int kw, 
         rp.rows_per_plane = Fy;
         rp.r_s1 = Fx;
         rp.r_s2 = (int64_t)Fx * Fy;
-        rp.c_s1 = w->Fxh;
-        rp.c_s2 = (int64_t)w->Fxh * Fy;
+        rp.c_s1 = w->Fxs;
+        rp.c_s2 = (int64_t)w->Fxs * Fy;
         rp.nload = Fx;
         rp.rsrc = P;
         rp.cdst = K;
@@ -1547,8 +1557,9 @@ vfd_status vfd_window_spectrum(const float *window, int kw, int kh, int kd, int 
     st = vfd_set_window(w, 0, window, kw, kh, kd, cx, cy, cz);
     if (st == VFD_OK) {
         DeviceGuard g(w->device);
-        const int64_t nk = (int64_t)w->Fxh * fy * fz;
-        cudaError_t e = cudaMemcpy(out, w->d_kspec, sizeof(float2) * nk, cudaMemcpyDeviceToHost);
+        const size_t row = sizeof(float2) * w->Fxh;
+        cudaError_t e = cudaMemcpy2D(out, row, w->d_kspec, sizeof(float2) * w->Fxs, row, (size_t)fy * fz,
+                                     cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) {
             g_thread_error = std::string("window spectrum: ") + cudaGetErrorString(e);
             st = VFD_ERR_CUDA;
@@ -1611,8 +1622,8 @@ vfd_status vfd_spectrum_window(const float *kspec, int fx, int fy, int fz, int k
             rp.rows_per_plane = fy;
             rp.r_s1 = fx;
             rp.r_s2 = (int64_t)fx * fy;
-            rp.c_s1 = w->Fxh;
-            rp.c_s2 = (int64_t)w->Fxh * fy;
+            rp.c_s1 = w->Fxs;
+            rp.c_s2 = (int64_t)w->Fxs * fy;
             rp.nstore = fx;
             rp.rdst = P;
             rp.csrc = K;
@@ -1643,10 +1654,11 @@ vfd_status vfd_set_spectrum(vfd_world *w, int field, const float *kspec, int fx,
                         std::to_string(w->F[1]) + "x" + std::to_string(w->F[2]) +
                         " (create the world with desc.fft = {FFTW, FFTH, FFTD})");
     DeviceGuard g(w->device);
-    const int64_t nk = (int64_t)w->Fxh * w->F[1] * w->F[2];
+    const int64_t nk = (int64_t)w->Fxs * w->F[1] * w->F[2];
     float2 *K = w->d_kspec + nk * field;
     // cudaMemcpyDefault: host (pinned or pageable) or device source
-    VFD_CUDA(w, cudaMemcpy(K, kspec, sizeof(float2) * nk, cudaMemcpyDefault));
+    const size_t row = sizeof(float2) * w->Fxh;
+    VFD_CUDA(w, cudaMemcpy2D(K, sizeof(float2) * w->Fxs, kspec, row, row, (size_t)w->F[1] * w->F[2], cudaMemcpyDefault));
     float2 dc;
     VFD_CUDA(w, cudaMemcpy(&dc, K, sizeof(float2), cudaMemcpyDeviceToHost));
     w->k0[field] = dc.x;
@@ -1780,7 +1792,7 @@ struct UpdateArgs {
 static vfd_status enqueue_general_substep(vfd_world *w, int f, int n, cudaStream_t st, const UpdateArgs *upd = nullptr)
 {
     const int Fx = w->F[0], Fy = w->F[1], Fz = w->F[2];
-    const int64_t nk = (int64_t)w->Fxh * Fy * Fz;
+    const int64_t nk = (int64_t)w->Fxs * Fy * Fz;
     float *u = w->d_fields + (int64_t)f * w->V;
     double *mass = w->d_mass + (int64_t)f * MS_COUNT;
     const float2 *K = w->d_kspec + nk * f;
@@ -1790,7 +1802,7 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, int n, cudaStream
     GenFields ff;
     ff.n = n;
     ff.r = w->V;
-    ff.c = (int64_t)w->Fxh * Fy * w->nz;
+    ff.c = (int64_t)w->Fxs * Fy * w->nz;
     ff.k = nk;
     ff.mass = MS_COUNT;
     for (int i = 0; i < n; ++i) {
@@ -1805,8 +1817,8 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, int n, cudaStream
     memset(&r, 0, sizeof(r));
     r.plan = w->plan[0];
     r.tw = w->d_tw[0];
-    r.c_s1 = w->Fxh;
-    r.c_s2 = (int64_t)w->Fxh * Fy;
+    r.c_s1 = w->Fxs;
+    r.c_s2 = (int64_t)w->Fxs * Fy;
     if (w->method == VFD_METHOD_FFT3D) {
         // pruned + fused: rows of the data only; C holds z < nz
         r.nrows = w->ny * w->nz;
@@ -1838,8 +1850,8 @@ static vfd_status enqueue_general_substep(vfd_world *w, int f, int n, cudaStream
         {
             GenColPass c = col_pass(w, PASS_Z, w->d_C, Fy, w->nz, w->nz, GEN_FWD_MUL_INV);
             c.kspec = K;
-            c.k_s_outer = w->Fxh;
-            c.k_s_pos = (int64_t)w->Fxh * Fy;
+            c.k_s_outer = w->Fxs;
+            c.k_s_pos = (int64_t)w->Fxs * Fy;
             c.scale = invN;
             LaunchTimer lt(w, 2, st);
             VFD_CUDA(w, launch_gen_cols(w->gvar[2], c, st, &ff));
