@@ -40,10 +40,10 @@ for p in (os.path.join(ROOT, "vf-version_7_3_b200"), ROOT):
 
 METRIC = "voxel-steps/s"
 # ncu dram__bytes_read.sum + dram__bytes_write.sum per axis-pass launch,
-# averaged over x, y, z (10.89 GB per launch on the 8 x 768x384x576 world,
-# profiles/rf_tma_pass_512x256x128.md), scaled to the human-scale world by
+# averaged over x, y, z (1.02 GB per launch on an 8 x 512x256x128 world,
+# profiles/band_pass_512x256x128.md), scaled to the human-scale world by
 # its voxel count (the passes read and write every voxel once).
-AXIS_TRAFFIC_BYTES = 3.23e9
+AXIS_TRAFFIC_BYTES = 3.06e9
 
 # The configurations, written out here so that the reference arm and the CPU
 # sample need no import of the product package (vfd/configs.py holds the
@@ -338,8 +338,10 @@ def run_reference(args, c):
 # ---------------------------------------------------------------------------
 def run_cfg2(args, dev=0, quiet=False):
     """Batched ensemble: 32 uneven worlds x 8 fields, 10 substeps per tick, all
-    fields of the rank's worlds in one launch per axis pass, the pass of
-    each axis chosen by vfd_batch_autotune, the tick replayed as a CUDA graph.
+    fields of the rank's worlds in one launch per axis (the tick's substeps
+    folded into one banded product), the tick replayed as a CUDA graph;
+    vfd_batch_autotune's choice among the FFT passes, which such ticks do not
+    use, is reported as fft_pass_tuning.
     Beside it: the same worlds through the plain per-field path
     (VFD_METHOD_PLAIN: unfused kernels, one field at a time, no graph).
     Under torchrun the worlds are sharded round-robin over the ranks."""
@@ -393,16 +395,11 @@ def run_cfg2(args, dev=0, quiet=False):
     ms = vd.max_over_ranks(e0.elapsed_time(e1), device=f"cuda:{dev}")
     # whole job: the voxel-steps of every rank's worlds over the slowest rank's time
     value = vd.sum_over_ranks(vox * args.steps, device=f"cuda:{dev}") / (ms / 1e3)
-    # the sum of the per-pass times against the graph's tick time: the cost
-    # of the launch boundaries inside the graph
-    pass_ms = sum(t["ms"] for t in tuning) * c["substeps"]
     batch.close()
     for w in worlds:
         w.close()
     res = {"value": value, "unit": METRIC, "ms_per_tick": ms / args.steps,
-           "launches_per_tick": launches / args.steps, "tuning": tuning, "autotune_s": tune_s,
-           "graph_vs_pass_sum": {"tick_ms": ms / args.steps, "pass_ms_sum": pass_ms,
-                                 "gap_frac": 1.0 - pass_ms / (ms / args.steps)},
+           "launches_per_tick": launches / args.steps, "fft_pass_tuning": tuning, "autotune_s": tune_s,
            "clocks": clk, "worlds": len(mine)}
     if ws == 1:
         # plain per-field path, one world at a time (bounded: 1 tick)
@@ -425,14 +422,15 @@ def run_cfg2(args, dev=0, quiet=False):
             w.close()
         plain = vox / (plain_ms / 1e3)
         peak, kind = peaks()
-        achieved = 24.0 * value / 1e9
+        achieved = 24.0 * value / c["substeps"] / 1e9
         res.update({"plain_gpu": {"value": plain, "unit": METRIC,
                                   "what": "VFD_METHOD_PLAIN: unfused pad/R2C/C2C/multiply/C2C/C2R/crop kernels, "
                                           "one field per launch sequence, no graph"},
                     "batched_over_plain": value / plain,
                     "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                                  "frac": achieved / peak, "peak_source": f"{kind} hbm_gbs",
-                                 "note": "whole tick, 24 B per voxel-step (3 axis passes x 8 B)"}})
+                                 "note": "whole tick, 24 B per voxel and tick (3 axis passes x 8 B, the "
+                                         "substeps folded)"}})
     return res
 
 
@@ -680,7 +678,7 @@ def main():
     per_pass = {k: prof[k][0] / max(prof[k][1], 1) for k in prof}
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": AXIS_TRAFFIC_BYTES,
-                "kernel": "axis passes: rf_row_tma_kernel (x), rf_col_tma_kernel (y, z)",
+                "kernel": "axis passes: band_kernel (x; y and z), a tick's substeps in one pass per axis",
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms,
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "share_of_step": axis_ms / ms if ms > 0 else None,
