@@ -70,7 +70,9 @@ def peaks():
 
 
 class ClockSampler:
-    """nvidia-smi samples of SM clock and throttle reasons during the timed region."""
+    """Samples of SM clock and throttle reasons during the timed region: through
+    NVML every few milliseconds (a timed region may be as short as 20 ms), or
+    from nvidia-smi where its Python binding is missing.  Reads only."""
 
     FIELDS = ("clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -82,6 +84,19 @@ class ClockSampler:
         self.lines = []
 
     def start(self):
+        self.sampling = False
+        try:
+            import pynvml
+            pynvml.nvmlInit()
+            self.nvml, self.handle = pynvml, pynvml.nvmlDeviceGetHandleByIndex(self.dev)
+            self.max_mhz = float(pynvml.nvmlDeviceGetMaxClockInfo(self.handle, pynvml.NVML_CLOCK_SM))
+            self._sample()
+            self.lines, self.sampling = [], True
+            self.t = threading.Thread(target=self._poll, daemon=True)
+            self.t.start()
+            return
+        except Exception:
+            self.lines = []
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.dev), f"--query-gpu={self.FIELDS}",
@@ -92,18 +107,41 @@ class ClockSampler:
         except Exception:
             self.proc = None
 
+    # clocks event reasons bits: hw_slowdown, hw_thermal_slowdown, sw_thermal_slowdown, sw_power_cap
+    REASON_BITS = (0x8, 0x40, 0x20, 0x4)
+
+    def _sample(self):
+        n = self.nvml
+        mhz = n.nvmlDeviceGetClockInfo(self.handle, n.NVML_CLOCK_SM)
+        get = getattr(n, "nvmlDeviceGetCurrentClocksEventReasons", None) or n.nvmlDeviceGetCurrentClocksThrottleReasons
+        bits = get(self.handle)
+        self.lines.append(f"{mhz},{self.max_mhz},0,{bits}," +
+                          ",".join("Active" if bits & b else "Not Active" for b in self.REASON_BITS))
+
+    def _poll(self):
+        while self.sampling:
+            try:
+                self._sample()
+            except Exception:
+                return
+            time.sleep(0.002)
+
     def _read(self):
         for line in self.proc.stdout:
             self.lines.append(line.strip())
 
     def stop(self):
-        if not self.proc:
+        if self.sampling:
+            self.sampling = False
+            self.t.join(timeout=5)
+        elif not self.proc:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
-        self.proc.terminate()
-        try:
-            self.proc.wait(timeout=5)
-        except Exception:
-            self.proc.kill()
+        else:
+            self.proc.terminate()
+            try:
+                self.proc.wait(timeout=5)
+            except Exception:
+                self.proc.kill()
         sm, mx, reasons = [], [], set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
         for ln in self.lines:
