@@ -40,9 +40,9 @@ for p in (os.path.join(ROOT, "vf-version_7_3_b200"), ROOT):
 
 METRIC = "voxel-steps/s"
 # ncu dram__bytes_read.sum + dram__bytes_write.sum per axis-pass launch,
-# averaged over x, y, z (1.02 GB per launch on an 8 x 512x256x128 world,
-# profiles/band_pass_512x256x128.md), scaled to the human-scale world by
-# its voxel count (the passes read and write every voxel once).
+# averaged over x, y, z (1.02 GB per launch on an 8 x 512x256x128 world, ten
+# folded substeps), scaled to the human-scale world by its voxel count (the
+# passes read and write every voxel once).
 AXIS_TRAFFIC_BYTES = 3.06e9
 
 # The configurations, written out here so that the reference arm and the CPU
