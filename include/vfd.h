@@ -249,7 +249,8 @@ vfd_status vfd_set_boundary(vfd_world *w, int epi_boundary, const float *baselin
  * for every field f (the reference's pChem = dChem + tChem*cytokineDecay[ic],
  * dChem = 0; its decay table is woundHealingWorld.cpp:2640-2648).  dchem
  * holds n_fields device pointers of V floats (an entry, or dchem itself, may
- * be NULL: d = 0).  In VFD_METHOD_FFT3D / VFD_METHOD_PLAIN worlds the update
+ * be NULL: d = 0).  Fields are updated in order: of an array that several of
+ * them are given, the first takes the values, the others find zeros.  In VFD_METHOD_FFT3D / VFD_METHOD_PLAIN worlds the update
  * is fused into the crop store of the inverse x transform; separable worlds
  * run it as one extra pass over the fields.  Registered sources
  * (vfd_set_sources) are deposited after the update.  vfd_read_mass then

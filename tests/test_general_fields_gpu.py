@@ -70,6 +70,50 @@ def test_more_fields_than_a_launch_holds(gpu):
     check((33, 20, 17), (40, 24, 21), 11)
 
 
+@pytest.mark.parametrize("method,kind", [(vfd.METHOD_FFT3D, k) for k in ("same", "overlapping", "next", "previous")]
+                         + [(vfd.METHOD_SEPARABLE, "same"), (vfd.METHOD_SEPARABLE, "overlapping")])
+def test_shared_dchem(gpu, method, kind):
+    """Device dChem arrays that fields share, or that are fields of the world:
+    the fields are updated in order, so the first takes the values and the
+    others find zeros.  The grid's spectra fit one launch of several fields."""
+    import torch
+    nx, ny, nz, nf = 40, 30, 22, 4
+    V = nx * ny * nz
+    sig = [0.6 + 0.07 * f for f in range(nf)]
+    decay = [np.float32(0.9 + 0.01 * f) for f in range(nf)]
+    us = [vfd.synth_field(3, 0, f, (nz, ny, nx)) for f in range(nf)]
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    buf = torch.rand((2 * V,), device="cuda") * 1e-3
+    # one run of memory: the world's fields, then the two arrays
+    mem = np.concatenate([u.ravel() for u in us] + [buf.cpu().numpy()]).astype(np.float64)
+    D = nf * V
+    at = {"same": [D, D, D + V, D], "overlapping": [D, D + V // 3, D + V, None],
+          "next": [V, 2 * V, D, None], "previous": [D, 0, V, 2 * V]}[kind]
+    with vfd.World(nx, ny, nz, [vfd.field_params(s, 0.02, radius=4) for s in sig], method=method) as w:
+        for f, u in enumerate(us):
+            w.upload(f, u)
+        ptr = [None if a is None else w.device_ptr(0) + 4 * a if a < D else buf.data_ptr() + 4 * (a - D) for a in at]
+        w.tick_update(decay, [p or 0 for p in ptr], 1)
+        outs = np.concatenate([w.download(f).ravel() for f in range(nf)] + [buf.cpu().numpy()])
+
+    def tick(f):
+        u = mem[f * V:(f + 1) * V].astype(np.float32).reshape(nz, ny, nx)
+        return oracle.tick(u, sig[f], 0.02, 1, *none, radius3=4).ravel() * float(decay[f])
+
+    def update(f, t):
+        d = np.zeros(V) if at[f] is None else mem[at[f]:at[f] + V].copy()
+        if at[f] is not None:
+            mem[at[f]:at[f] + V] = 0.0
+        mem[f * V:(f + 1) * V] = d + t
+
+    for f in range(nf):
+        update(f, tick(f))
+    assert rel_l2(outs, mem) <= REL_L2
+    for f in range(nf):
+        assert rel_l2(outs[f * V:(f + 1) * V], mem[f * V:(f + 1) * V]) <= REL_L2, f
+    np.testing.assert_array_equal(outs[D:] == 0, mem[D:] == 0)
+
+
 @pytest.mark.parametrize("method", [vfd.METHOD_FFT3D, vfd.METHOD_SEPARABLE])
 @pytest.mark.parametrize("kind", ["pageable", "pinned", "shared", "partial"])
 def test_update_host_buffers(gpu, method, kind):

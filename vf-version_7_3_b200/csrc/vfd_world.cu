@@ -1952,6 +1952,30 @@ static vfd_status enqueue_fft_substeps(vfd_world *w, int field, int n_substeps, 
     return VFD_OK;
 }
 
+// Whether an update of field f may run in one launch with one of field g: an
+// update reads and zeroes its dChem, so neither field's dChem may be the
+// other's, nor the other's values.  (Fields of separate launches run in
+// order: of a shared dChem the first takes the values, the next finds zeros.)
+static bool updates_independent(const vfd_world *w, const UpdateArgs &u, int f, int g)
+{
+    auto overlap = [&](const float *p, const float *q) { return p && q && p < q + w->V && q < p + w->V; };
+    auto values = [&](int i) { return w->d_fields + (int64_t)i * w->V; };
+    const float *df = u.dchem ? u.dchem[f] : nullptr, *dg = u.dchem ? u.dchem[g] : nullptr;
+    return !overlap(df, dg) && !overlap(df, values(g)) && !overlap(dg, values(f));
+}
+
+// How many fields from f on (before `end`) one launch of the general
+// transform takes: all with a dChem or all without, updates independent.
+static int general_fields(const vfd_world *w, const UpdateArgs *u, int f, int end)
+{
+    auto has_d = [&](int i) { return u && u->dchem && u->dchem[i]; };
+    int n = 1;
+    for (; f + n < end && n < w->gen_group && has_d(f + n) == has_d(f); ++n)
+        for (int i = f; u && i < f + n; ++i)
+            if (!updates_independent(w, *u, i, f + n)) return n;
+    return n;
+}
+
 static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStream_t st,
                                const UpdateArgs *upd = nullptr)
 {
@@ -1959,10 +1983,9 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
         const int f0 = field < 0 ? 0 : field, f1 = field < 0 ? w->nf : field + 1;
         for (int s = 0; s < n_substeps; ++s) {
             const UpdateArgs *u = s + 1 == n_substeps ? upd : nullptr;
-            auto has_d = [&](int f) { return u && u->dchem && u->dchem[f]; };
             VFD_CUDA(w, cudaMemsetAsync(w->d_mass + (int64_t)f0 * MS_COUNT, 0, sizeof(double) * MS_COUNT * (f1 - f0), st));
             for (int f = f0, n = 0; f < f1; f += n) {
-                for (n = 1; f + n < f1 && n < w->gen_group && has_d(f + n) == has_d(f);) ++n;
+                n = general_fields(w, u, f, f1);
                 vfd_status r = enqueue_general_substep(w, f, n, st, u);
                 if (r != VFD_OK) return r;
             }
