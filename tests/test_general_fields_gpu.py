@@ -70,7 +70,7 @@ def test_more_fields_than_a_launch_holds(gpu):
     check((33, 20, 17), (40, 24, 21), 11)
 
 
-@pytest.mark.parametrize("method,kind", [(vfd.METHOD_FFT3D, k) for k in ("same", "overlapping", "next", "previous")]
+@pytest.mark.parametrize("method,kind", [(vfd.METHOD_FFT3D, k) for k in ("same", "overlapping", "own", "next", "previous")]
                          + [(vfd.METHOD_SEPARABLE, "same"), (vfd.METHOD_SEPARABLE, "overlapping")])
 def test_shared_dchem(gpu, method, kind):
     """Device dChem arrays that fields share, or that are fields of the world:
@@ -87,7 +87,7 @@ def test_shared_dchem(gpu, method, kind):
     # one run of memory: the world's fields, then the two arrays
     mem = np.concatenate([u.ravel() for u in us] + [buf.cpu().numpy()]).astype(np.float64)
     D = nf * V
-    at = {"same": [D, D, D + V, D], "overlapping": [D, D + V // 3, D + V, None],
+    at = {"same": [D, D, D + V, D], "overlapping": [D, D + V // 3, D + V, None], "own": [0, V, 2 * V, D],
           "next": [V, 2 * V, D, None], "previous": [D, 0, V, 2 * V]}[kind]
     with vfd.World(nx, ny, nz, [vfd.field_params(s, 0.02, radius=4) for s in sig], method=method) as w:
         for f, u in enumerate(us):

@@ -577,14 +577,16 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
     // dChem's rows lie as the field's, at one distance: two row pointers less in
     // registers (the update's spills 776 -> 390 bytes)
     const int64_t du = EPI == C2R_UPDATE ? reinterpret_cast<intptr_t>(p.dchem) - reinterpret_cast<intptr_t>(p.rdst) : 0;
+    // Both accesses keep their places: the read after grid_dep_wait (an earlier
+    // kernel may write dChem) and before its position's stores, the zero before
+    // the store of the sum (dChem may be the field itself: d + t stays).
     auto dchem = [&](const float *x) {
         float d;
-        asm("ld.global.f32 %0, [%1];\n" : "=f"(d) : "l"(reinterpret_cast<intptr_t>(x) + du));
+        asm volatile("ld.global.f32 %0, [%1];\n" : "=f"(d) : "l"(reinterpret_cast<intptr_t>(x) + du) : "memory");
         return d;
     };
-    // takes the value read, so that the read comes first
-    auto zero = [&](const float *x, float was) {
-        asm volatile("st.global.f32 [%0], %1;\n" ::"l"(reinterpret_cast<intptr_t>(x) + du), "f"(0.0f), "f"(was));
+    auto zero = [&](const float *x) {
+        asm volatile("st.global.f32 [%0], %1;\n" ::"l"(reinterpret_cast<intptr_t>(x) + du), "f"(0.0f) : "memory");
     };
     // positions left from n2 on in the stored part, in the row and in rows a, b
     const int left = p.nstore - n2, la = ra.ok ? left : 0, lb = rb.ok ? left : 0;
@@ -607,7 +609,7 @@ __device__ __forceinline__ void c2r_a(const GenRowPass &p, const TprSmem &m, int
             gc += t;
             t = keep * (t + bk * k0);
             t = EPI == C2R_UPDATE ? t * us + dval : t * us;
-            if (EPI == C2R_UPDATE) zero(dst + d, dval);
+            if (EPI == C2R_UPDATE) zero(dst + d);
             go += t;
         }
         dst[d] = t;
