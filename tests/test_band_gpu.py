@@ -175,3 +175,112 @@ def test_batch_results_do_not_depend_on_neighbours(gpu):
                 v.close()
     finally:
         vfd.autotune_clear()
+
+
+# Fields of a wide range.  What an output may be off by is relative to the
+# values its blocks hold: the sum of |weight x value| and the mean of a block of
+# 64 that holds it (the offset), 14 * 2^-24 of each a group.  A window of blocks
+# reaches at most 192 positions from an output.
+REACH = 192
+LONG = 520
+GRIDS = [(LONG, 6, 5), (7, LONG, 4), (5, 6, LONG)]
+
+
+def along(axis, n):
+    """Positions along `axis` as a (nz, ny, nx) array that broadcasts."""
+    return np.arange(n).reshape([-1 if a == 2 - axis else 1 for a in range(3)])
+
+
+def run_once(grid, u, sig, substeps, dec=0.0):
+    with vfd.World(*grid, [vfd.field_params(sig, dec)]) as w:
+        w.upload(0, u)
+        w.tick(substeps)
+        out, mass = w.download(0), w.mass()[0]
+    ref = oracle.tick(u, sig, dec, substeps, np.zeros(0, np.int32), np.zeros(0, np.float32))
+    return out.astype(np.float64), ref, mass
+
+
+# half-widths of 8 (one substep of sigma 2.6), 32 and 48 (ten of 1.3 and of 2.6)
+WIDE = [(2.6, 1), (1.3, 10), (2.6, 10)]
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("sigma,substeps", WIDE)
+def test_single_voxel_in_the_middle(gpu, axis, sigma, substeps):
+    """One voxel of 1 at the middle of every axis, nothing else: the result is
+    as accurate as a dense field's, and zero where no block sees the voxel."""
+    grid = GRIDS[axis]
+    u = np.zeros(grid[::-1], np.float32)
+    u[grid[2] // 2, grid[1] // 2, grid[0] // 2] = 1.0
+    out, ref, mass = run_once(grid, u, sigma, substeps)
+    assert rel_l2(out, ref) <= 2 * PER_GROUP  # its own products' and the offset's
+    assert abs(out.sum() - ref.sum()) <= 1e-6 * ref.sum()
+    far = np.broadcast_to(np.abs(along(axis, LONG) - LONG // 2) > REACH, out.shape)
+    assert far.any() and not out[far].any()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("sigma,substeps", WIDE)
+@pytest.mark.parametrize("at", [0, LONG // 2 - 30, LONG - 60])
+def test_plume_leaves_zeros_alone(gpu, axis, sigma, substeps, at):
+    """60 voxels of about 1 at either end or in the middle, zeros elsewhere."""
+    grid = GRIDS[axis]
+    p = along(axis, LONG)
+    u = np.where((p >= at) & (p < at + 60), 0.5 + vfd.synth_field(4, 0, 0, grid[::-1]), 0.0).astype(np.float32)
+    out, ref, mass = run_once(grid, u, sigma, substeps)
+    assert rel_l2(out, ref) <= PER_GROUP
+    assert abs(out.sum() - ref.sum()) <= 1e-6 * ref.sum()
+    far = np.broadcast_to((p < at - REACH) | (p >= at + 60 + REACH), out.shape)
+    assert far.any() and not out[far].any()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("sigma,substeps", WIDE)
+@pytest.mark.parametrize("at", [3, LONG // 2])
+def test_large_value_spoils_no_small_ones(gpu, axis, sigma, substeps, at):
+    """A voxel of 1 (at the low end, at the middle) on a background of 5e-7:
+    away from it the error is relative to the background."""
+    grid = GRIDS[axis]
+    back = np.float32(5e-7)
+    u = (back * (0.5 + vfd.synth_field(5, 0, 0, grid[::-1]))).astype(np.float32)
+    u[(grid[2] // 2, grid[1] // 2, at) if axis == 0 else (grid[2] // 2, at, grid[0] // 2) if axis == 1 else
+      (at, grid[1] // 2, grid[0] // 2)] = 1.0
+    out, ref, mass = run_once(grid, u, sigma, substeps)
+    assert rel_l2(out, ref) <= 2 * PER_GROUP
+    far = np.broadcast_to(np.abs(along(axis, LONG) - at) > REACH, out.shape)
+    assert far.any() and np.abs(out[far] - ref[far]).max() <= PER_GROUP * 1.5 * back
+
+
+@pytest.mark.parametrize("sigma,substeps", [(1.4, 4), (2.6, 10)])
+@pytest.mark.parametrize("kind", ["sparse", "signed"])
+def test_sparse_and_signed_fields(gpu, sigma, substeps, kind):
+    """Errors relative to what the products add up, sum |weight x value|: for
+    a sparse field of positive values that is the output itself."""
+    grid = (300, 70, 36)
+    rng = np.random.default_rng(8)
+    u = rng.standard_normal(grid[::-1])
+    if kind == "sparse":
+        u = np.where(rng.random(u.shape) < 0.02, np.exp(2.0 * u - 6.0), 0.0)
+    u = u.astype(np.float32)
+    out, ref, mass = run_once(grid, u, sigma, substeps)
+    scale = oracle.tick(np.abs(u), sigma, 0.0, substeps, np.zeros(0, np.int32), np.zeros(0, np.float32))
+    # the other axes' passes smooth |values| as far as values: the scale of the worst is the x pass'
+    assert np.sqrt(((out - ref) ** 2).sum()) <= PER_GROUP * np.sqrt((scale ** 2).sum())
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_non_finite_values_reach_their_blocks_only(gpu, axis):
+    grid = GRIDS[axis]
+    u = vfd.synth_field(2, 0, 0, grid[::-1])
+    bad = u.copy()
+    bad[tuple(20 if a == 2 - axis else 1 for a in range(3))] = np.inf
+    outs = []
+    for v in (u, bad):
+        with vfd.World(*grid, [vfd.field_params(0.6, 0.0)]) as w:
+            w.upload(0, v)
+            w.tick(1)
+            outs.append(w.download(0))
+    hit = ~np.isfinite(outs[1])
+    assert hit[tuple(20 if a == 2 - axis else 1 for a in range(3))]
+    assert not hit[np.broadcast_to(along(axis, LONG) > 20 + REACH, hit.shape)].any()
+    np.testing.assert_array_equal(outs[0][~hit], outs[1][~hit])

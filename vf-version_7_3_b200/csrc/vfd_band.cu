@@ -11,11 +11,18 @@
 // blocks; the parts w0, w1, w2 of W_b come from shared memory.  Six
 // tensor-core products of FP32 accumulation a k-step -- x_i w_j for i + j <= 2,
 // the five small ones of every k-step first -- give the FP32 product.  The
-// tensor cores truncate when they accumulate, so a line's values are taken
-// relative to an offset near them, whose own product (offset times the row
-// sum of B^m) is added in FP32: what is truncated is then small and of either
-// sign (one substep of positive values, relative L2 against FP64: 1.1e-7
-// without the offset, 4.5e-8 with it; the FFT passes 8e-8).
+// tensor cores truncate when they accumulate, so values are taken relative to
+// an offset, whose own product (offset times a row sum of B^m) is added in
+// FP32: what is truncated is then small and of either sign.  The offset of a
+// line is that of its input block, the block's mean: the mean is the value
+// that leaves least (its sum of squares is never above that of the values
+// themselves), and what a block holds cannot cost bits in blocks that do not
+// see it.  One offset for the whole line did: a voxel of 1 in the middle of a
+// line of zeros left 2e-5 of the result's L2 and 8e-5 of its sum (ten substeps,
+// sigma 2.6), a plume residues over all of its lines.  Relative L2 against
+// FP64, one substep of positive values: 1.1e-7 without offsets, 3.7e-8 with
+// them, the FFT passes 1e-7; ten substeps, sigma 2.6: 3.6e-8 and 1.2e-6; the
+// voxel of 1: 9.7e-8 and 1.3e-6.
 //
 // In place: outputs of block b are stored once its product is complete; all
 // input blocks that hold those positions are in tensor memory by then, and
@@ -24,7 +31,8 @@
 // Roles (one CTA per SM, persistent): warps 0..7 read the accumulators back
 // and store the outputs (four warps an accumulator), warps 8..15 convert input
 // blocks and store them to tensor memory, warps 16..19 copy input blocks to
-// shared memory (cp.async, nstage blocks deep), warps 20 and 21 issue the
+// shared memory (bulk tensor copies, or cp.async where the layout does not
+// allow them; nstage blocks deep), warps 20 and 21 issue the
 // products of even and of odd blocks, warp 22 fetches weight images (bulk
 // copies).
 #include <cuda_bf16.h>
@@ -56,9 +64,9 @@ constexpr int BD_ACC_COL = 3 * BD_PART_RING;          // two accumulators of 64 
 constexpr int BD_HALF_BYTES = BD_STEP_BYTES / 2;      // 8 positions of a k-step: 64 outputs of each part
 constexpr int BD_STAGE_BYTES = BD_LINES * BD_BLK * 4;
 constexpr int BD_XOUT_BYTES = BD_EPI_WARPS * 32 * 16 * 4;
-constexpr int BD_TILES = 8;          // tiles the loaders can be ahead of the epilogue by, at most (6), and more
+constexpr int BD_OFFS = 8;           // input blocks' offsets kept: the loaders are ahead of the epilogue by 7 at most
 constexpr int BD_MAXSTAGE = 4, BD_MAXSLOT = 4;
-constexpr size_t BD_SMEM_MAX = 214 * 1024;  // beside the 12 KB of BandShared
+constexpr size_t BD_SMEM_MAX = 213 * 1024;  // beside BandShared
 constexpr size_t BD_SMEM_MIN = 120 * 1024;  // one CTA per SM: each takes all of tensor memory
 
 // D FP32, A and B bf16, both K-major, M 128, N 64
@@ -73,7 +81,8 @@ struct BandShared {
     uint64_t dfull[2], dempty[2]; // accumulator complete / read back
     uint64_t wfull[2];            // weight image of the next even / odd block landed
     int wslot[2];                 // its slot
-    alignas(16) float off[BD_TILES][BD_LINES];  // each line's offset, by tile
+    alignas(16) float off[BD_OFFS][BD_LINES];   // each line's offset in an input block
+    float half[2][2][BD_LINES];   // sums of a block's halves, in turn
     alignas(16) float fn[BD_CONV_WARPS][2][32];  // a block's functional weights, alpha and lambda
     uint32_t tmem;
     int dead;                     // a wait gave up: nothing waits or stores any more
@@ -227,6 +236,7 @@ struct BandTiles {
     }
 };
 static_assert(sizeof(BandJob) / 16 <= 32, "one piece a lane");
+static_assert(sizeof(BandShared) + BD_SMEM_MAX <= 227 * 1024, "shared memory of a block");
 
 // Byte offset of (line, position) in a stage, as the bulk copies leave it.  x
 // pass: two boxes of 32 positions, a row of 128 bytes per line, its 16-byte
@@ -241,13 +251,14 @@ __device__ __forceinline__ int band_at(int line, int pos)
 }
 
 // ---------------------------------------------------------------------------
-// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.70-0.72 ms a pass for
-// ten folded substeps (4.5 TB/s of the 8 bytes a voxel it moves; without its
-// products 0.60), so a tick of ten substeps and its deposit takes 2.3 ms alone
-// and 2.6 ms back to back (power-limited), against 19.0 ms on 30 register-FFT
-// passes of 0.58-0.66 ms; 0.57-0.58 ms (y, z; x 0.76) for one substep.  768x384x576: 9.3 against 60 ms.  What bounds it: HBM,
-// with the products (48 cycles each, two issuing threads together) and the
-// ring of four input blocks limiting how far its stages overlap.
+// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.71-0.75 ms a pass for
+// ten folded substeps (4.3-4.5 TB/s of the 8 bytes a voxel it moves; without its
+// products 0.60; with one offset a line instead of one a block 0.69-0.70), so a
+// tick of ten substeps and its deposit takes 2.7 ms back to back against 19.0 ms
+// on 30 register-FFT passes of 0.58-0.66 ms.  768x384x576: 9.7 against 60 ms.
+// What bounds it: HBM, with the products (48 cycles each, two issuing threads
+// together), the read-back of the accumulators and the ring of four input
+// blocks limiting how far its stages overlap.
 // ---------------------------------------------------------------------------
 // Copies input blocks to the stages.
 template <bool XP>
@@ -378,11 +389,12 @@ __device__ __forceinline__ double dot32(const float2 (&v)[16], const float *w)
 }
 
 // Converts input blocks: the padding rule, the accounting's input terms, the
-// three bf16 parts of value minus line offset, into tensor memory.
-template <bool XP>
+// three bf16 parts of value minus the block's offset, into tensor memory.
+template <int AXIS>
 __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int nstage, unsigned char *stages,
                                              BandShared &S, uint32_t tmem)
 {
+    constexpr bool XP = AXIS == PASS_X;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quad = warp & 3, half = (warp - BD_CONV0) >> 2;
     const int ln = quad * 32 + lane;  // line of the tile = lane of tensor memory
@@ -395,13 +407,12 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
         const double sp = XP ? band_warp_sum(accP) : 0.0;
         if (lane == 0 && !S.dead) {
             if (XP) atomicAdd(J.mass + MS_INPUT, sp);
-            if (sl != 0.0) atomicAdd(J.mass + (XP ? MS_LEAK_X : J.kind == PASS_Y ? MS_LEAK_Y : MS_LEAK_Z), sl);
+            if (sl != 0.0) atomicAdd(J.mass + (XP ? MS_LEAK_X : AXIS == PASS_Y ? MS_LEAK_Y : MS_LEAK_Z), sl);
         }
         accP = accL = 0.0;
     };
-    int tile = 0;
     int jn = T.job(T.first());
-    for (int t = T.first(); t < T.end; t += gridDim.x, ++tile) {
+    for (int t = T.first(); t < T.end; t += gridDim.x) {
         const int j = jn;
         jn = T.job(t + gridDim.x);
         if (j != job) {
@@ -413,9 +424,8 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
         const bool mask = XP && J.mask;
         const float b = J.b;
         const int l = (t - J.tile0) * BD_LINES + ln;
-        float off = 0.0f;
         float lw1 = 1.0f, lw2 = 1.0f;  // the line's weights, read long before they are used
-        int lo = 0, hi = 0;
+        int lo = 0, hi = mask ? 0 : n;  // the positions that count
         const bool acc = sums && J.sums;
         if (l < J.nlines && (mask || acc)) {
             if (XP) {
@@ -428,18 +438,9 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
                     lo = J.box_lo[0];
                     hi = J.box_hi[0];
                 }
-            } else if (J.kind == PASS_Y) {
+            } else if (AXIS == PASS_Y) {
                 lw2 = __ldg(J.lw2 + l / J.n0);
             }
-        }
-        // A wide band has its first block near the boundary only: the line's
-        // offset is then the middle sample, read while that block is under way.
-        const bool far = H > BD_BLK / 2;
-        if (far && l < J.nlines && (!mask || lo < hi)) {
-            const int mid = mask ? (lo + hi) >> 1 : n >> 1, o = XP ? 0 : l / J.n0;
-            off = __ldcg(XP ? J.data + (int64_t)l * n + mid
-                            : J.data + (int64_t)o * J.outer_stride + (l - o * J.n0) + mid * J.pos_stride);
-            if (mask) off -= b;
         }
         double tP = 0.0, tL = 0.0;  // the line's sums
         // a block's functional weights, one position a lane, read a block ahead
@@ -466,22 +467,6 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = make_float2(f[2 * i * 32], f[(2 * i + 1) * 32]);
             }
-            if (k == 0) {
-                if (!far) {
-                    // the line's offset: of two samples of its first block, the
-                    // one nearer to zero
-                    const int i1 = min(BD_BLK - 1, n - 1 + H), i0 = (H + i1) >> 1;
-                    float s0 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i0));
-                    float s1 = *reinterpret_cast<const float *>(sp + band_at<XP>(ln, i1));
-                    if (mask) {
-                        s0 = (i0 - H >= lo && i0 - H < hi) ? s0 - b : 0.0f;
-                        s1 = (i1 - H >= lo && i1 - H < hi) ? s1 - b : 0.0f;
-                    }
-                    off = fabsf(s0) < fabsf(s1) ? s0 : s1;
-                }
-                if (!(fabsf(off) < 1e30f)) off = 0.0f;
-                S.off[tile % BD_TILES][ln] = off;  // both halves store the same
-            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.sempty[st]);
             if (++st == nstage) {
@@ -503,9 +488,11 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
                     }
                 }
             }
+            const float vs = sum32(v);
+            S.half[done & 1][half][ln] = vs;
             if (acc) {
                 if ((J.plain >> k) & 1ull) {
-                    if (XP) tP += (double)(sum32(v) * J.fscale);
+                    if (XP) tP += (double)(vs * J.fscale);
                 } else {
                     float(*f)[32] = S.fn[warp - BD_CONV0];
                     __syncwarp();
@@ -522,7 +509,13 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
             }
             if (done >= BD_RING) band_wait(&S.aempty[slot], ((done / BD_RING) - 1) & 1, &S.dead);
             tc_fence_after();
-            __syncwarp();
+            // the block's offset: the mean of its positions that count (those in
+            // the line and inside the padding box; the others have weight 0)
+            asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quad) : "memory");
+            const int count = min(BD_BLK * (k + 1) - H, hi) - max(BD_BLK * k - H, lo);
+            float off = count > 0 ? __fdividef(vs + S.half[done & 1][half ^ 1][ln], (float)count) : 0.0f;
+            if (!(fabsf(off) < 1e30f)) off = 0.0f;
+            if (half == 0) S.off[done % BD_OFFS][ln] = off;
             const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(slot * BD_PART_COLS + half * 16);
             const float2 noff = make_float2(-off, -off), neg = make_float2(-1.0f, -1.0f);
             uint32_t w[16];
@@ -699,10 +692,11 @@ __device__ __forceinline__ void band_issuer(const BandTiles &T, int par, int slo
 }
 
 // Stores the outputs: 32 positions of the warp's 32 lines at a time.
-template <bool XP>
+template <int AXIS>
 __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsigned char *xout, BandShared &S,
                                               uint32_t tmem)
 {
+    constexpr bool XP = AXIS == PASS_X, zl = AXIS == PASS_Z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quad = warp & 3, team = warp >> 2;  // team: the accumulator (every other block) this warp reads
     const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + BD_ACC_COL + team * BD_BLK;
@@ -710,7 +704,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
     double acc_ot = 0.0;
     const BandJob &J = S.job[warp];
     auto flush = [&]() {
-        if (XP || !sums || job < 0 || !J.sums || J.kind != PASS_Z) return;
+        if (!zl || !sums || job < 0 || !J.sums) return;
         const double so = band_warp_sum(acc_ot), c = band_warp_sum((double)count);
         if (lane == 0 && !S.dead) {
             // the convolution's sum from the stored values: out = keep (t + b)
@@ -720,9 +714,9 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
         acc_ot = 0.0;
         count = 0;
     };
-    int tile = 0;
+    int ein = 0;  // input blocks of the tiles before
     int jn = T.job(T.first());
-    for (int t_ = T.first(); t_ < T.end; t_ += gridDim.x, ++tile) {
+    for (int t_ = T.first(); t_ < T.end; t_ += gridDim.x) {
         const int j = jn;
         jn = T.job(t_ + gridDim.x);
         if (j != job) {
@@ -730,37 +724,36 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
             job = j;
             T.load(j, &S.job[warp], lane);
         }
-        const int n = J.n, nb = J.nb, nlines = J.nlines;
-        const bool zl = !XP && J.kind == PASS_Z;
-        const int64_t ps = J.pos_stride;
+        // (what is read from the job where it is used need not stay in a register)
+        const int n = J.n;
         const int l0 = (t_ - J.tile0) * BD_LINES + quad * 32, l = l0 + lane;
-        const bool lok = l < nlines;
+        const bool lok = l < J.nlines;
         float *dst = J.data;
-        int naff = 0, ly = 0, lx = 0;
         if (!XP) {
             const int o = lok ? l / J.n0 : 0;
             dst += lok ? (int64_t)o * J.outer_stride + (l - o * J.n0) : 0;
-            if (zl) {
-                naff = J.naff;
-                if (naff) {
-                    ly = l / J.nx;
-                    lx = l - ly * J.nx;
-                }
-            }
         }
-        float off = 0.0f;
-        bool have = false;
-        for (int b = 0; b < nb; ++b, ++i) {
+        for (int b = 0; b < J.nb; ++b, ++i) {
             if ((i & 1) != team) continue;
             band_wait(&S.dfull[team], phase, &S.dead);
             phase ^= 1;
             tc_fence_after();
-            if (!have) off = S.off[tile % BD_TILES][quad * 32 + lane];
-            have = true;
             const bool live = !*(volatile int *)&S.dead;
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
                 float2 t[16];  // positions 2 c, 2 c + 1 of this half
+                // the offsets of the window's blocks (two, or three where it spans as
+                // many): the last one's, the steps to it from the first (d0) and
+                // from the second (d1)
+                const bool three = J.ksteps > 2 * BD_BLK / 16;
+                auto offset = [&](int k) { return S.off[(ein + min(k, J.nin - 1)) % BD_OFFS][quad * 32 + lane]; };
+                float off = offset(b + 1), d1 = 0.0f;
+                const float d0 = offset(b) - off;
+                if (three) {
+                    const float last = offset(b + 2);
+                    d1 = off - last;
+                    off = last;
+                }
                 __syncwarp();
                 tc_ld32(ta + 32 * half, t);
                 if (half == 1) {
@@ -768,39 +761,34 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&S.dempty[team]);
                 }
-                // the offset's share, its product with the operator's row sums;
-                // last pass: out = keep (t + baseline)
-                const float2 k2 = make_float2(zl ? J.keep : 1.0f, zl ? J.keep : 1.0f);
-                const float base = zl ? J.b : 0.0f;
-                if (b >= J.b0 && b < J.b1) {
-                    const float o = fmaf(off, J.fscale, base);
-                    const float2 o2 = make_float2(o, o);
-                    if (zl) {
-                        const float2 q2 = __fmul2_rn(k2, o2);
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) t[c] = __ffma2_rn(k2, t[c], q2);
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
-                    }
-                } else {
-                    const float4 *rho = reinterpret_cast<const float4 *>(J.rho + J.image(b) * BD_BLK + 32 * half);
-                    const float2 off2 = make_float2(off, off), b2 = make_float2(base, base);
+                // the offsets' share: the weights' sums over the window's first
+                // block, its first two and all of it; last pass: out = keep (t +
+                // baseline), keep being part of the operator
+                const float base = zl ? J.keep * J.b : 0.0f;
+                const float4 *rho = reinterpret_cast<const float4 *>(J.rho + J.image(b) * (3 * BD_BLK) + 32 * half);
+                auto add = [&](float d, const float4 *r) {
+                    const float2 d2 = make_float2(d, d);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
-                        const float4 r = __ldg(rho + c);
-                        t[2 * c] = __fmul2_rn(
-                            k2, __fadd2_rn(__ffma2_rn(off2, make_float2(r.x, r.y), t[2 * c]), b2));
-                        t[2 * c + 1] = __fmul2_rn(
-                            k2, __fadd2_rn(__ffma2_rn(off2, make_float2(r.z, r.w), t[2 * c + 1]), b2));
+                        const float4 q = __ldg(r + c);
+                        t[2 * c] = __ffma2_rn(d2, make_float2(q.x, q.y), t[2 * c]);
+                        t[2 * c + 1] = __ffma2_rn(d2, make_float2(q.z, q.w), t[2 * c + 1]);
                     }
-                }
+                };
+                add(d0, rho);
+                if (three) add(d1, rho + BD_BLK / 4);
+                const bool inner = b >= J.b0 && b < J.b1;  // the sums over all of a window are all the same
+                if (!inner) add(off, rho + 2 * (BD_BLK / 4));
+                const float o = inner ? fmaf(off, J.fscale, base) : base;
+                const float2 o2 = make_float2(o, o);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
                 const int p0 = BD_BLK * b + 32 * half;
                 if (XP) {
                     // 32 rows x 16 positions at a time through shared memory,
                     // 64-byte row segments out
                     unsigned char *o = xout + warp * 2048;
-                    const int rmax = live ? nlines - l0 : 0;
+                    const int rmax = live ? J.nlines - l0 : 0;
 #pragma unroll
                     for (int g = 0; g < 2; ++g) {
                         __syncwarp();
@@ -835,6 +823,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                         }
                     }
                 } else {
+                    const int naff = zl ? J.naff : 0, ly = naff ? l / J.nx : 0, lx = l - ly * J.nx;
                     for (int g = 0; g < naff; ++g) {
                         // the affine rows, decayed like the rest
                         const float q = lok ? J.keep * J.affc[g] * J.aff[0][(int64_t)g * J.affs[0] + lx] *
@@ -861,6 +850,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                         acc_ot += (double)sum32(t);
                         count += m;
                     }
+                    const int64_t ps = J.pos_stride;
                     float *q = dst + (int64_t)p0 * ps;
                     if (m == 32 && live) {
 #pragma unroll
@@ -880,11 +870,12 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                 }
             }
         }
+        ein += J.nin;
     }
     flush();
 }
 
-template <bool XP>
+template <int AXIS>
 __global__ void __launch_bounds__(BD_THREADS, 1)
     band_kernel(const BandJob *__restrict__ jobs, const unsigned short *__restrict__ tjob, int tile_begin, int tile_end,
                 int sums, int nstage, int nslots, int slot_bytes)
@@ -926,22 +917,20 @@ __global__ void __launch_bounds__(BD_THREADS, 1)
     // the weights do not depend on the kernel before; the fields do
     if (warp != BD_FETCH) grid_dep_wait();
     const BandTiles T{jobs, tjob, tile_begin, tile_end};
-    // registers: 80 a thread at launch; 256 x (104 + 88 + 48) = 256 x (96 + 96 + 48) = 768 x 80
+    // registers: 80 a thread at launch; 256 x (104 + 88 + 48) = 768 x 80
     if (warp < BD_CONV0) {
-        if (XP) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;\n");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
     } else if (warp < BD_COPY0) {
-        if (XP) asm volatile("setmaxnreg.inc.sync.aligned.u32 96;\n");
-        else asm volatile("setmaxnreg.inc.sync.aligned.u32 88;\n");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 88;\n");
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;\n");
     }
     if (warp < BD_CONV0) {
-        band_epilogue<XP>(T, sums, xout, S, tmem);
+        band_epilogue<AXIS>(T, sums, xout, S, tmem);
     } else if (warp < BD_COPY0) {
-        band_convert<XP>(T, sums, nstage, stages, S, tmem);
+        band_convert<AXIS>(T, sums, nstage, stages, S, tmem);
     } else if (warp < BD_ISSUE) {
-        band_copy<XP>(T, nstage, stages, S);
+        band_copy<AXIS == PASS_X>(T, nstage, stages, S);
     } else if ((threadIdx.x & 31) == 0) {
         if (warp < BD_FETCH) band_issuer(T, warp - BD_ISSUE, slot_bytes, wsm, S, tmem);
         else if (warp == BD_FETCH) band_fetch(T, nslots, slot_bytes, wsm, S);
@@ -1010,12 +999,12 @@ __global__ void __launch_bounds__(128) band_image_kernel(const BandAxis *axes)
     }
     __syncwarp();
     unsigned char *img = X.img + (size_t)im * X.ksteps * BD_STEP_BYTES;
-    double sum = 0.0;
+    double sum[3] = {0.0, 0.0, 0.0};  // over the window's first input block, its first two, all of it
     for (int kk = lane; kk < X.ksteps * 16; kk += 32) {
         const int j = BD_BLK * b - X.H + kk, q = j - i + hw;
         double w = 0.0;
         if (j >= 0 && j < n && abs(i - j) <= X.H && q >= 0 && q < wd) w = cur[q] * X.scale;
-        sum += w;
+        for (int k = kk / BD_BLK; k < 3; ++k) sum[k] += w;
         const size_t at = (size_t)(kk >> 4) * BD_STEP_BYTES + ((kk >> 3) & 1) * BD_HALF_BYTES + (o >> 3) * 128 +
                           (o & 7) * 16 + (kk & 7) * 2;
 #pragma unroll
@@ -1025,8 +1014,10 @@ __global__ void __launch_bounds__(128) band_image_kernel(const BandAxis *axes)
             *reinterpret_cast<__nv_bfloat16 *>(img + at + part * (BD_HALF_BYTES / 3)) = h;
         }
     }
-    sum = band_warp_sum(sum);
-    if (lane == 0) X.rho[row] = (float)sum;
+    for (int k = 0; k < 3; ++k) {
+        const double r = band_warp_sum(sum[k]);
+        if (lane == 0) X.rho[(im * 3 + k) * BD_BLK + o] = (float)r;
+    }
 }
 
 // y(j) = sum_i x(i) g(i - j) over [0, n): A is symmetric
@@ -1132,7 +1123,7 @@ __global__ void band_init_kernel(const BandInit *init, int nfields)
     }
 }
 
-template <bool XP>
+template <int AXIS>
 cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int tile_begin, int ntiles, BandGeom geo,
                           bool sums, cudaStream_t st)
 {
@@ -1140,7 +1131,7 @@ cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int t
     static thread_local int sms = 148;
     const unsigned long long ctx = current_context_id();
     if (ctx == 0 || ctx != ctx_done) {
-        cudaError_t e = cudaFuncSetAttribute(band_kernel<XP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(band_kernel<AXIS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)BD_SMEM_MAX);
         if (e != cudaSuccess) return e;
         int dev = 0;
@@ -1149,7 +1140,7 @@ cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int t
         ctx_done = ctx;
     }
     const int slot = geo.ksteps * BD_STEP_BYTES;
-    const size_t xo = XP ? BD_XOUT_BYTES : 0;
+    const size_t xo = AXIS == PASS_X ? BD_XOUT_BYTES : 0;
     // two images, then stages up to three, then more images, then a fourth stage
     int nstage = 2, nslots = 2;
     auto bytes = [&]() { return (size_t)nslots * slot + (size_t)nstage * BD_STAGE_BYTES + xo + 1024; };
@@ -1164,7 +1155,7 @@ cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int t
     grow(nstage, BD_MAXSTAGE);
     grow(nslots, BD_MAXSLOT);
     const size_t sm = std::max(bytes(), BD_SMEM_MIN);
-    const cudaError_t e = launch_overlapped(ntiles <= 8 * sms, band_kernel<XP>, dim3((unsigned)std::min(ntiles, sms)), BD_THREADS, sm, st, jobs,
+    const cudaError_t e = launch_overlapped(ntiles <= 8 * sms, band_kernel<AXIS>, dim3((unsigned)std::min(ntiles, sms)), BD_THREADS, sm, st, jobs,
                                             tjob, tile_begin, tile_begin + ntiles, sums ? 1 : 0, nstage, nslots, slot);
     note_launch();
     return e == cudaSuccess ? cudaGetLastError() : e;
@@ -1223,8 +1214,9 @@ cudaError_t launch_band(const BandJob *jobs, const unsigned short *tjob, int til
                         BandGeom geo, bool sums, cudaStream_t st)
 {
     if (ntiles <= 0) return cudaSuccess;
-    return axis == PASS_X ? launch_band_t<true>(jobs, tjob, tile_begin, ntiles, geo, sums, st)
-                          : launch_band_t<false>(jobs, tjob, tile_begin, ntiles, geo, sums, st);
+    return axis == PASS_X   ? launch_band_t<PASS_X>(jobs, tjob, tile_begin, ntiles, geo, sums, st)
+           : axis == PASS_Y ? launch_band_t<PASS_Y>(jobs, tjob, tile_begin, ntiles, geo, sums, st)
+                            : launch_band_t<PASS_Z>(jobs, tjob, tile_begin, ntiles, geo, sums, st);
 }
 
 bool band_take_timeout()

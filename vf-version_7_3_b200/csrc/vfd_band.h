@@ -32,7 +32,7 @@ struct alignas(16) BandJob {
     double *mass;
     const unsigned char *img;  // this axis' weight images (BandAxis)
     const CUtensorMap *map;    // tensor map of the input blocks, or NULL (copied by cp.async)
-    const float *rho;          // row sums of the images, 64 each
+    const float *rho;          // row sums of the images, 64 each: over the window's first input block, its first two, all
     const float *fn;           // functional weights by input position: alpha[nin * 64], then lambda[nin * 64]
     const float *lw1, *lw2;    // line weights: x pass alpha_y, alpha_z; y pass (lw2) alpha_z
     const float *aff[3];       // affine rows X_j, Y_j, Z_j (z pass, naff > 0), row stride affs[a]
@@ -48,7 +48,7 @@ struct alignas(16) BandJob {
     int b0, b1;                // output blocks b0 .. b1 - 1 see no boundary: they share image b0
     int mask;                  // x pass: apply the padding rule
     int sums;                  // form the accounting (a launch may turn it off for all)
-    float b, keep, fscale;     // fscale: factor folded into the operator (x pass: keep^(m-1), else 1)
+    float b, keep, fscale;     // fscale: factor folded into the operator (x pass: keep^(m-1), z pass: keep, y pass: 1)
     int nx, ny;
     int box_lo[3], box_hi[3];
     // image of output block b
@@ -60,7 +60,7 @@ static_assert(sizeof(BandJob) % 16 == 0, "BandJob is copied in 16-byte pieces");
 struct BandAxis {
     const double *taps;     // 2 r + 1
     unsigned char *img;     // nimg images of ksteps * BD_STEP_BYTES
-    float *rho;             // row sums of the images, 64 each
+    float *rho;             // row sums of the images (as BandJob::rho)
     float *fn;              // alpha, lambda (as BandJob::fn)
     float *aff;             // naff rows of affs floats (X_1 .. X_naff)
     double *dots;           // [3][BD_MMAX]: sum M X_j, sum lambda_0 X_j, sum X_j

@@ -748,8 +748,10 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
                 J.box_hi[c] = A.box_hi[c];
             }
             const double keep = 1.0 - p.decay_rate;
-            const double fold = a == PASS_X ? std::pow(keep, m - 1) : 1.0;
-            J.fscale = (float)fold;
+            // the substeps' decays: all but the last in the x pass (and its
+            // sums), the last in the z pass
+            const double fold = a == PASS_X ? std::pow(keep, m - 1) : 1.0, scale = a == PASS_Z ? keep : fold;
+            J.fscale = (float)scale;
             const int naff = A.b != 0.0f ? m - 1 : 0;
             const int lo = A.box_lo[a], hi = std::max(A.box_hi[a], A.box_lo[a]);
             // one image for the blocks that see no boundary (adjacent ones), one
@@ -771,7 +773,8 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
             X.nin = J.nin;
             X.lo = lo;
             X.hi = hi;
-            X.scale = X.fscale = fold;
+            X.scale = scale;
+            X.fscale = fold;
             X.naff = naff;
             X.affs = J.nb * BD_BLK;
             max_rows = std::max(max_rows, X.nimg * BD_BLK);
@@ -780,7 +783,7 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
             o_taps[i] = taps.size();
             taps.insert(taps.end(), g.begin(), g.end());
             o_img[i] = take((size_t)X.nimg * J.ksteps * BD_STEP_BYTES);
-            o_rho[i] = take(sizeof(float) * X.nimg * BD_BLK);
+            o_rho[i] = take(sizeof(float) * 3 * X.nimg * BD_BLK);
             o_fn[i] = take(sizeof(float) * 2 * J.nin * BD_BLK);
             o_aff[i] = take(sizeof(float) * (size_t)naff * X.affs);
         }
