@@ -223,7 +223,7 @@ def test_single_voxel_in_the_middle(gpu, axis, sigma, substeps):
 @pytest.mark.parametrize("sigma,substeps", WIDE)
 @pytest.mark.parametrize("at", [0, LONG // 2 - 30, LONG - 60])
 def test_plume_leaves_zeros_alone(gpu, axis, sigma, substeps, at):
-    """60 voxels of about 1 at either end or in the middle, zeros elsewhere."""
+    """60 voxels of about 0.5 at either end or in the middle, zeros elsewhere."""
     grid = GRIDS[axis]
     p = along(axis, LONG)
     u = np.where((p >= at) & (p < at + 60), 0.5 + vfd.synth_field(4, 0, 0, grid[::-1]), 0.0).astype(np.float32)
@@ -284,3 +284,24 @@ def test_non_finite_values_reach_their_blocks_only(gpu, axis):
     assert hit[tuple(20 if a == 2 - axis else 1 for a in range(3))]
     assert not hit[np.broadcast_to(along(axis, LONG) > 20 + REACH, hit.shape)].any()
     np.testing.assert_array_equal(outs[0][~hit], outs[1][~hit])
+
+
+@pytest.mark.parametrize("substeps", [1, 7])
+def test_convolution_sum_next_to_a_baseline(gpu, substeps):
+    """The accounting identity where the values hardly differ from the
+    baseline: input, convolved and leaked sums are of the differences, so
+    rounding the stored values (about the baseline) must not reach them."""
+    nx, ny, nz, base = 132, 70, 35, 3e-4
+    b = np.float32(base)
+    u = (b * (1 + 1e-4 * np.random.default_rng(1).random((nz, ny, nx)))).astype(np.float32)
+    with vfd.World(nx, ny, nz, [vfd.field_params(1.1, 0.0371, baseline=base)], pad_mode=vfd.PAD_CONSTANT_VF,
+                   epi_boundary=125) as w:
+        w.upload(0, u)
+        w.tick(substeps)
+        m, out = w.mass()[0], w.download(0)
+    if substeps == 1:  # later substeps start from the decayed baseline, whose differences are not small
+        v = np.zeros(u.shape)
+        v[1:-1, 1:-1, 1:125] = u[1:-1, 1:-1, 1:125].astype(np.float64) - float(b)
+        assert abs(m["input_sum"] - v.sum()) <= 1e-6 * v.sum()
+    assert abs(m["input_sum"] - m["conv_sum"] - sum(m["leaked"])) <= 1e-6 * abs(m["input_sum"])
+    assert abs(m["total"] - out.astype(np.float64).sum()) <= 1e-6 * abs(m["total"])

@@ -700,19 +700,17 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quad = warp & 3, team = warp >> 2;  // team: the accumulator (every other block) this warp reads
     const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + BD_ACC_COL + team * BD_BLK;
-    int i = 0, phase = 0, job = -1, count = 0;  // count: positions summed
-    double acc_ot = 0.0;
+    int i = 0, phase = 0, job = -1;
+    double acc_ot = 0.0, acc_ct = 0.0;  // of the values stored, and (where there is a baseline) before it is added
     const BandJob &J = S.job[warp];
     auto flush = [&]() {
         if (!zl || !sums || job < 0 || !J.sums) return;
-        const double so = band_warp_sum(acc_ot), c = band_warp_sum((double)count);
+        const double so = band_warp_sum(acc_ot), sc = J.b != 0.0f ? band_warp_sum(acc_ct) : so;
         if (lane == 0 && !S.dead) {
-            // the convolution's sum from the stored values: out = keep (t + b)
-            atomicAdd(J.mass + MS_CONV, so / (double)J.keep - (double)J.b * c);
+            atomicAdd(J.mass + MS_CONV, sc / (double)J.keep);
             atomicAdd(J.mass + MS_OUT, so);
         }
-        acc_ot = 0.0;
-        count = 0;
+        acc_ot = acc_ct = 0.0;
     };
     int ein = 0;  // input blocks of the tiles before
     int jn = T.job(T.first());
@@ -762,9 +760,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                     if (lane == 0) mbar_arrive(&S.dempty[team]);
                 }
                 // the offsets' share: the weights' sums over the window's first
-                // block, its first two and all of it; last pass: out = keep (t +
-                // baseline), keep being part of the operator
-                const float base = zl ? J.keep * J.b : 0.0f;
+                // block, its first two and all of it
                 const float4 *rho = reinterpret_cast<const float4 *>(J.rho + J.image(b) * (3 * BD_BLK) + 32 * half);
                 auto add = [&](float d, const float4 *r) {
                     const float2 d2 = make_float2(d, d);
@@ -779,10 +775,12 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                 if (three) add(d1, rho + BD_BLK / 4);
                 const bool inner = b >= J.b0 && b < J.b1;  // the sums over all of a window are all the same
                 if (!inner) add(off, rho + 2 * (BD_BLK / 4));
-                const float o = inner ? fmaf(off, J.fscale, base) : base;
-                const float2 o2 = make_float2(o, o);
+                auto shift = [&](float o) {
+                    const float2 o2 = make_float2(o, o);
 #pragma unroll
-                for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
+                    for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
+                };
+                if (inner) shift(off * J.fscale);
                 const int p0 = BD_BLK * b + 32 * half;
                 if (XP) {
                     // 32 rows x 16 positions at a time through shared memory,
@@ -839,7 +837,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                         }
                     }
                     const int m = lok ? min(32, n - p0) : 0;
-                    if (zl && sums && J.sums && m > 0) {
+                    auto sum = [&]() {  // over the line's positions
                         if (m < 32) {
 #pragma unroll
                             for (int x = 0; x < 16; ++x) {
@@ -847,9 +845,15 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
                                 if (2 * x + 1 >= m) t[x].y = 0.0f;
                             }
                         }
-                        acc_ot += (double)sum32(t);
-                        count += m;
+                        return (double)sum32(t);
+                    };
+                    const bool acc = zl && sums && J.sums && m > 0;
+                    if (zl && J.b != 0.0f) {
+                        // out = keep (t + baseline), keep being part of the operator
+                        if (acc) acc_ct += sum();
+                        shift(J.keep * J.b);
                     }
+                    if (acc) acc_ot += sum();
                     const int64_t ps = J.pos_stride;
                     float *q = dst + (int64_t)p0 * ps;
                     if (m == 32 && live) {
