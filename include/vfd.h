@@ -457,6 +457,11 @@ vfd_status vfd_write_csv(const float *field, int nx, int ny, int nz, const char 
  * call returns VFD_ERR_TIMEOUT -- the status vfd_read_mass reports after a
  * pass's wait gave up.  Any other status means the mechanism is broken. */
 vfd_status vfd_check_wait_timeout(int device, long long limit_cycles);
+/* The banded passes' wait given up on purpose in the same way, in the flag of
+ * world w (asynchronous on `stream`): the next of vfd_read_mass,
+ * vfd_diffuse_host and vfd_diffuse_update_host on w returns VFD_ERR_TIMEOUT,
+ * once; other worlds' calls do not. */
+vfd_status vfd_world_check_wait(vfd_world *w, long long limit_cycles, void *stream);
 
 const char *vfd_status_string(vfd_status s);
 /* Last error message of this world (or of the last failed create when

@@ -305,3 +305,31 @@ def test_convolution_sum_next_to_a_baseline(gpu, substeps):
         assert abs(m["input_sum"] - v.sum()) <= 1e-6 * v.sum()
     assert abs(m["input_sum"] - m["conv_sum"] - sum(m["leaked"])) <= 1e-6 * abs(m["input_sum"])
     assert abs(m["total"] - out.astype(np.float64).sum()) <= 1e-6 * abs(m["total"])
+
+
+def test_wait_that_gave_up_reaches_its_own_world(gpu):
+    """A banded pass's wait that gave up (run on purpose against a barrier that
+    nothing completes, about 1 ms) is told once, by whichever synchronous call
+    on its world comes next, and by no other world's; then the world ticks on."""
+    grid, params = (40, 24, 16), [vfd.field_params(1.0, 0.1)]
+    u = vfd.synth_field(1, 0, 0, grid[::-1])
+
+    def gave_up(call):
+        assert vfd.lib().vfd_world_check_wait(w._h, 2_000_000, None) == 0
+        w.tick(2)  # later ticks do not clear the flag
+        v.tick(2)
+        assert v.mass()[0]["total"] > 0
+        with pytest.raises(vfd.VfdError) as e:
+            call()
+        assert e.value.status == 5
+        v.tick(2)
+        call()
+
+    with vfd.World(*grid, params) as w, vfd.World(*grid, params) as v:
+        for x in (w, v):
+            x.upload(0, u)
+        out, d = [np.empty_like(u)], [np.zeros_like(u)]
+        gave_up(w.mass)
+        gave_up(lambda: w.diffuse_host([u], out, 2))
+        gave_up(lambda: w.diffuse_update_host(out, d, np.ones(1, np.float32), 2))
+        assert w.mass()[0]["total"] > 0

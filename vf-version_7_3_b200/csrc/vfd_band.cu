@@ -48,9 +48,6 @@
 
 namespace vfd {
 
-// Set when a pass's bounded wait gave up (read and cleared by band_take_timeout).
-__device__ int g_band_timeout = 0;
-
 namespace {
 
 constexpr int BD_EPI_WARPS = 8, BD_CONV_WARPS = 8, BD_COPY_WARPS = 4;
@@ -107,15 +104,15 @@ __device__ __forceinline__ bool band_try(uint64_t *bar, uint32_t parity)
 // Waits for phase `parity`, about 1 s at most; after a wait gave up every
 // wait returns at once, so all roles run out their loops (in bounds, storing
 // nothing) and the CTA ends.
-__device__ __forceinline__ bool band_wait(uint64_t *bar, uint32_t parity, volatile int *dead)
+__device__ __forceinline__ bool band_wait(uint64_t *bar, uint32_t parity, volatile int *dead,
+                                          long long limit = kTmaWaitCycles)
 {
     if (band_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!band_try(bar, parity)) {
         if (*dead) return false;
-        if (clock64() - t0 > kTmaWaitCycles) {
+        if (clock64() - t0 > limit) {
             *dead = 1;
-            atomicExch(&g_band_timeout, 1);
             return false;
         }
     }
@@ -942,8 +939,26 @@ __global__ void __launch_bounds__(BD_THREADS, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // every world this CTA had a tile of learns that a wait gave up
+    if (S.dead && threadIdx.x == 0)
+        for (int t = T.first(); t < T.end; t += gridDim.x) atomicExch(jobs[tjob[t]].gave_up, 1);
     if (warp == BD_ISSUE)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(tmem) : "memory");
+}
+
+__global__ void band_wait_probe_kernel(long long limit, int *gave_up)
+{
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ int dead;
+    if (threadIdx.x == 0) {
+        dead = 0;
+        mbar_init(&bar, 1);
+        mbar_fence_init();
+    }
+    __syncwarp();
+    band_wait(&bar, 0, &dead, limit);
+    __syncwarp();
+    if (dead && threadIdx.x == 0) atomicExch(gave_up, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1223,13 +1238,11 @@ cudaError_t launch_band(const BandJob *jobs, const unsigned short *tjob, int til
                             : launch_band_t<PASS_Z>(jobs, tjob, tile_begin, ntiles, geo, sums, st);
 }
 
-bool band_take_timeout()
+cudaError_t band_wait_probe(long long limit, int *gave_up, cudaStream_t st)
 {
-    int h = 0;
-    if (cudaMemcpyFromSymbol(&h, g_band_timeout, sizeof(int)) != cudaSuccess || h == 0) return false;
-    const int z = 0;
-    cudaMemcpyToSymbol(g_band_timeout, &z, sizeof(int));
-    return true;
+    band_wait_probe_kernel<<<1, 32, 0, st>>>(limit, gave_up);
+    note_launch();
+    return cudaGetLastError();
 }
 
 }  // namespace vfd

@@ -37,17 +37,18 @@ struct alignas(16) BandJob {
     const float *lw1, *lw2;    // line weights: x pass alpha_y, alpha_z; y pass (lw2) alpha_z
     const float *aff[3];       // affine rows X_j, Y_j, Z_j (z pass, naff > 0), row stride affs[a]
     const float *affc;         // their coefficients
+    int *gave_up;              // set where a wait gave up (the world's)
     int64_t outer_stride, pos_stride;
     unsigned long long plain;  // bit k: input block k has alpha = 1 and lambda = 0 everywhere
     int affs[3];
     int naff;
     int n, n0, nlines, ntiles, tile0;
     int H, ksteps, nb, nin;    // half-width, k-steps of an image, output and input blocks
-    int kind;                  // PassKind
-    int vec;                   // 16-byte accesses apply
     int b0, b1;                // output blocks b0 .. b1 - 1 see no boundary: they share image b0
-    int mask;                  // x pass: apply the padding rule
-    int sums;                  // form the accounting (a launch may turn it off for all)
+    unsigned char kind;        // PassKind
+    bool vec;                  // 16-byte accesses apply
+    bool mask;                 // x pass: apply the padding rule
+    bool sums;                 // form the accounting (a launch may turn it off for all)
     float b, keep, fscale;     // fscale: factor folded into the operator (x pass: keep^(m-1), z pass: keep, y pass: 1)
     int nx, ny;
     int box_lo[3], box_hi[3];
@@ -104,7 +105,8 @@ struct BandGeom {
 cudaError_t launch_band(const BandJob *jobs, const unsigned short *tjob, int tile_begin, int ntiles, int axis,
                         BandGeom geo, bool sums, cudaStream_t st);
 
-// Reads and clears the flag a pass sets when a bounded wait gave up.
-bool band_take_timeout();
+// The passes' bounded wait on a barrier that nothing completes: it gives up
+// after `limit` cycles, which *gave_up tells as a pass would.
+cudaError_t band_wait_probe(long long limit, int *gave_up, cudaStream_t st);
 
 }  // namespace vfd

@@ -3,9 +3,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "vfd.h"
 #include "vfd_axis.cuh"
 
 namespace vfd {
+
+// What went wrong in the world's passes up to here on `st` (waits for it):
+// VFD_ERR_DEVICE_FAULT, or VFD_ERR_TIMEOUT (told once).
+vfd_status world_status(vfd_world *w, cudaStream_t st);
 
 // One field's share of a source-deposit launch.
 struct DepositJob {

@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "vfd.h"
+#include "vfd_internal.h"
 
 namespace {
 
@@ -246,6 +247,7 @@ int retire(vfd_server *s, const std::shared_ptr<Request> &r, std::string &msg)
 {
     int st = VFD_OK;
     if (r->mass) st = vfd_read_mass(r->world, r->mass, s->rstream);
+    else st = vfd::world_status(r->world, s->rstream);
     for (int f = 0; f < r->nf && st == VFD_OK && !r->result.empty(); ++f)
         if (r->result[f]) st = vfd_download_field(r->world, f, r->result[f], s->rstream);
     if (st != VFD_OK) msg = vfd_last_error(r->world);

@@ -395,7 +395,7 @@ struct vfd_world {
     int Fmax = 0;
     double *d_mass = nullptr;  // [f][MS_COUNT]
     AxisJob *d_jobs = nullptr; // [pass][nf] all-field jobs, then [pass][nf] single-field jobs
-    int *d_err = nullptr;
+    int *d_err = nullptr;      // [0]: a kernel met a bad index; [1]: a banded pass's wait gave up
 
     // sources
     std::vector<std::vector<int32_t>> src_idx;
@@ -723,7 +723,8 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
             const int n = dims[a], H = hw[m - 1];
             J.data = A.data;
             J.mass = A.mass;
-            J.kind = a;
+            J.gave_up = w->d_err + 1;
+            J.kind = (unsigned char)a;
             J.n = n;
             J.H = H;
             J.ksteps = (BD_BLK + 2 * H + 15) / 16;
@@ -1024,6 +1025,18 @@ static cudaError_t build_fft(vfd_world *w)
     return cudaSuccess;
 }
 
+vfd_status vfd::world_status(vfd_world *w, cudaStream_t st)
+{
+    int h[2] = {0, 0};
+    VFD_CUDA(w, cudaMemcpyAsync(h, w->d_err, sizeof(h), cudaMemcpyDeviceToHost, st));
+    VFD_CUDA(w, cudaStreamSynchronize(st));
+    const bool late = w->method == VFD_METHOD_SEPARABLE && rf_take_timeout();
+    if (h[1]) VFD_CUDA(w, cudaMemsetAsync(w->d_err + 1, 0, sizeof(int), st));
+    if (h[0]) return fail(w, VFD_ERR_DEVICE_FAULT, "a kernel rejected an out-of-range index");
+    if (h[1] || late) return fail(w, VFD_ERR_TIMEOUT, "an axis pass gave up waiting for a bulk copy");
+    return VFD_OK;
+}
+
 extern "C" {
 
 const char *vfd_status_string(vfd_status s)
@@ -1263,8 +1276,8 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
     if (general && (e = build_axis_tables(w)) != cudaSuccess) return bail(e, "twiddles and spectra");
     if ((e = cudaMalloc(&w->d_mass, sizeof(double) * MS_COUNT * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc mass");
     if ((e = cudaMemset(w->d_mass, 0, sizeof(double) * MS_COUNT * w->nf)) != cudaSuccess) return bail(e, "cudaMemset mass");
-    if ((e = cudaMalloc(&w->d_err, sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc err");
-    if ((e = cudaMemset(w->d_err, 0, sizeof(int))) != cudaSuccess) return bail(e, "cudaMemset err");
+    if ((e = cudaMalloc(&w->d_err, 2 * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc err");
+    if ((e = cudaMemset(w->d_err, 0, 2 * sizeof(int))) != cudaSuccess) return bail(e, "cudaMemset err");
     if ((e = cudaMalloc(&w->d_dep, sizeof(DepositJob) * 2 * w->nf)) != cudaSuccess) return bail(e, "cudaMalloc deposit jobs");
     if (general) {
         const int64_t nk = (int64_t)w->Fxs * w->F[1] * w->F[2];
@@ -1518,11 +1531,24 @@ vfd_status vfd_check_wait_timeout(int device, long long limit_cycles)
     if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof(int));
     if (e == cudaSuccess) e = rf_wait_probe(limit_cycles, d, nullptr);
     if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(int), cudaMemcpyDeviceToHost);
+    int hb = 0;  // and the banded passes'
+    if (e == cudaSuccess) e = cudaMemset(d, 0, sizeof(int));
+    if (e == cudaSuccess) e = band_wait_probe(limit_cycles, d, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(&hb, d, sizeof(int), cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return fail(nullptr, VFD_ERR_CUDA, std::string("wait probe: ") + cudaGetErrorString(e));
     const bool flagged = rf_take_timeout();
-    if (h && flagged) return fail(nullptr, VFD_ERR_TIMEOUT, "the bounded wait gave up and reported it");
+    if (h && hb && flagged) return fail(nullptr, VFD_ERR_TIMEOUT, "the bounded wait gave up and reported it");
     return fail(nullptr, VFD_ERR_CUDA, "the bounded wait did not report giving up");
+}
+
+vfd_status vfd_world_check_wait(vfd_world *w, long long limit_cycles, void *stream)
+{
+    if (!w) return VFD_ERR_INVALID_ARG;
+    if (limit_cycles < 1 || limit_cycles > 4000000000ll) return fail(w, VFD_ERR_INVALID_ARG, "bad wait limit");
+    DeviceGuard g(w->device);
+    VFD_CUDA(w, band_wait_probe(limit_cycles, w->d_err + 1, (cudaStream_t)stream));
+    return VFD_OK;
 }
 
 vfd_status vfd_window_spectrum(const float *window, int kw, int kh, int kd, int cx, int cy, int cz, int fx, int fy,
@@ -2085,11 +2111,10 @@ vfd_status vfd_read_mass(vfd_world *w, vfd_mass *out, void *stream)
     if (!w || !out) return VFD_ERR_INVALID_ARG;
     DeviceGuard g(w->device);
     std::vector<double> h((size_t)MS_COUNT * w->nf);
-    int herr = 0;
     VFD_CUDA(w, cudaMemcpyAsync(h.data(), w->d_mass, sizeof(double) * h.size(), cudaMemcpyDeviceToHost,
                                 (cudaStream_t)stream));
-    VFD_CUDA(w, cudaMemcpyAsync(&herr, w->d_err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
-    VFD_CUDA(w, cudaStreamSynchronize((cudaStream_t)stream));
+    const vfd_status st = world_status(w, (cudaStream_t)stream);
+    if (st == VFD_ERR_CUDA) return st;
     for (int f = 0; f < w->nf; ++f) {
         const double *m = h.data() + (size_t)f * MS_COUNT;
         out[f].input_sum = m[MS_INPUT];
@@ -2111,10 +2136,7 @@ vfd_status vfd_read_mass(vfd_world *w, vfd_mass *out, void *stream)
         out[f].total = m[MS_OUT] + m[MS_SOURCES];
         out[f].reserved = 0.0;
     }
-    if (herr) return fail(w, VFD_ERR_DEVICE_FAULT, "a kernel rejected an out-of-range index");
-    if (rf_take_timeout() || band_take_timeout())
-        return fail(w, VFD_ERR_TIMEOUT, "an axis pass gave up waiting for a bulk copy");
-    return VFD_OK;
+    return st;
 }
 
 vfd_status vfd_update_gradients(vfd_world *w, const float *collagen, const float *elastin, float *fib, float *neu,
@@ -2456,11 +2478,7 @@ vfd_status vfd_diffuse_host(vfd_world *w, const float *const *host_in, float *co
         VFD_CUDA(w, cudaMemcpyAsync(host_out[f], dev, bytes, cudaMemcpyDeviceToHost, w->s_out));
     }
     VFD_CUDA(w, cudaStreamSynchronize(w->s_out));
-    VFD_CUDA(w, cudaStreamSynchronize(w->s_cmp));
-    int herr = 0;
-    VFD_CUDA(w, cudaMemcpy(&herr, w->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) return fail(w, VFD_ERR_DEVICE_FAULT, "a kernel rejected an out-of-range index");
-    return VFD_OK;
+    return world_status(w, w->s_cmp);
 }
 
 vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *const *host_d, const float *decay,
@@ -2516,11 +2534,7 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
     for (int f = 0; f < w->nf; ++f)
         if (dptr[f] && !pinned[f]) std::memset(host_d[f], 0, bytes);
     VFD_CUDA(w, cudaStreamSynchronize(w->s_out));
-    VFD_CUDA(w, cudaStreamSynchronize(w->s_cmp));
-    int herr = 0;
-    VFD_CUDA(w, cudaMemcpy(&herr, w->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (herr) return fail(w, VFD_ERR_DEVICE_FAULT, "a kernel rejected an out-of-range index");
-    return VFD_OK;
+    return world_status(w, w->s_cmp);
 }
 
 // ---------------------------------------------------------------------------

@@ -47,7 +47,7 @@ EXPORTED = [
     "vfd_autotune", "vfd_world_tuning", "vfd_autotune_set", "vfd_autotune_clear",
     "vfd_set_spectrum", "vfd_set_boundary", "vfd_tick_update", "vfd_diffuse_update_host",
     "vfd_batch_autotune", "vfd_window_spectrum", "vfd_write_raw_normalized", "vfd_write_csv",
-    "vfd_check_wait_timeout", "vfd_spectrum_window",
+    "vfd_check_wait_timeout", "vfd_world_check_wait", "vfd_spectrum_window",
 ]
 
 PASS_METHODS = {0: "register_fft", 1: "overlap_save", 2: "full_line"}
@@ -160,6 +160,7 @@ def load(path=LIB_PATH):
     lib.vfd_write_raw_normalized.argtypes = [P, C.c_int, C.c_int, C.c_int, C.c_char_p, C.c_int]
     lib.vfd_write_csv.argtypes = [P, C.c_int, C.c_int, C.c_int, C.c_char_p]
     lib.vfd_check_wait_timeout.argtypes = [C.c_int, C.c_longlong]
+    lib.vfd_world_check_wait.argtypes = [P, C.c_longlong, P]
     lib.vfd_stencil_window.argtypes = [C.c_double, C.c_double, C.c_int, C.c_int, P, C.c_int]
     lib.vfd_synth_field_device.argtypes = [C.c_uint64, C.c_int, C.c_int, C.c_float, C.c_float, P,
                                            C.c_size_t, P]
