@@ -333,3 +333,70 @@ def test_wait_that_gave_up_reaches_its_own_world(gpu):
         gave_up(lambda: w.diffuse_host([u], out, 2))
         gave_up(lambda: w.diffuse_update_host(out, d, np.ones(1, np.float32), 2))
         assert w.mass()[0]["total"] > 0
+
+
+@pytest.mark.parametrize("what", ["world", "batch"])
+@pytest.mark.parametrize("grid,sigma", [((90, 44, 31), 1.3), ((176, 160, 96), 0.9)])
+def test_first_tick_captured(gpu, what, grid, sigma):
+    """A fresh world's first tick of ten substeps under stream capture is the
+    folded one (its operators are built beside the capture), and a replay
+    gives what a direct tick gives."""
+    import torch
+    params = [vfd.field_params(sigma, 0.02)] * 2
+    us = [vfd.synth_field(5, 0, f, grid[::-1]) for f in range(2)]
+    with vfd.World(*grid, params) as w, vfd.World(*grid, params) as v:
+        for f, u in enumerate(us):
+            w.upload(f, u)
+            v.upload(f, u)
+        v.tick(10)
+        v.tick(10)
+        torch.cuda.synchronize()
+        t = vfd.Batch([w]) if what == "batch" else w
+        graph = torch.cuda.CUDAGraph()
+        before = vfd.launch_count()
+        with torch.cuda.graph(graph):
+            t.tick(10, stream=torch.cuda.current_stream().cuda_stream)
+        # three operators' set-up kernels, three passes, and a batch's accounting reset
+        assert vfd.launch_count() - before <= 7
+        torch.cuda.synchronize()
+        for f, u in enumerate(us):
+            np.testing.assert_array_equal(w.download(f), u)
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        for f in range(2):
+            np.testing.assert_array_equal(w.download(f), v.download(f))
+        del graph
+        if what == "batch":
+            t.close()
+
+
+def test_operators_are_ready_on_every_stream(gpu):
+    """Operators are built on a stream of their own: a first tick on one stream
+    and the next on another, right after, use them complete."""
+    import torch
+    grid, params = (200, 60, 50), [vfd.field_params(1.3 + 0.1 * f, 0.02) for f in range(4)]
+    us = [vfd.synth_field(6, 0, f, grid[::-1]) for f in range(4)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = []
+    for k in range(3):
+        with vfd.World(*grid, params) as w, vfd.World(*grid, params) as v:
+            for x in (w, v):
+                for f, u in enumerate(us):
+                    x.upload(f, u)
+            torch.cuda.synchronize()
+            if k < 2:
+                for m in (2 + k, 9):
+                    w.tick(m, stream=streams[0].cuda_stream)
+                    v.tick(m, stream=streams[1].cuda_stream)
+            else:
+                with vfd.Batch([w, v]) as b:
+                    b.tick(2, stream=streams[0].cuda_stream)
+                    b.tick(9, stream=streams[1].cuda_stream)
+                    torch.cuda.synchronize()
+            torch.cuda.synchronize()
+            outs.append([x.download(f) for x in (w, v) for f in range(4)])
+    for f in range(4):
+        np.testing.assert_array_equal(outs[0][f], outs[0][4 + f])
+        np.testing.assert_array_equal(outs[0][f], outs[2][f])
+        np.testing.assert_array_equal(outs[1][f], outs[1][4 + f])

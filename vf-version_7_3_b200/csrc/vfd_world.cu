@@ -362,6 +362,25 @@ struct BandPlan {
     int ntiles[3] = {0, 0, 0};
     const double *d_init = nullptr;     // [field][MS_COUNT] accounting start
     bool affine = false;                // d_init is not all zero
+    cudaEvent_t ready = nullptr;        // the operators are built (on the world's own stream) ...
+    bool done = false;                  // ... and known to be
+};
+
+static bool stream_capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+}
+
+// Set-up while a stream is being captured: allocations and waits on streams
+// that are not, which the capture need not know of, are allowed in its scope.
+class CaptureRelaxed {
+  public:
+    CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+  private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
 };
 
 struct vfd_world {
@@ -488,7 +507,10 @@ static void release(vfd_world *w)
     cudaFree(w->d_C);
     cudaFree(w->d_P);
     cudaFree(w->d_upd);
-    for (auto &kv : w->band_plans) cudaFree(kv.second.d);
+    for (auto &kv : w->band_plans) {
+        cudaFree(kv.second.d);
+        cudaEventDestroy(kv.second.ready);
+    }
     for (auto &t : w->timed) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -690,8 +712,8 @@ static int band_fold_limit(const vfd_world *w, int mmax)
     return top;
 }
 
-// Builds the operators of m substeps on the world's own stream and waits for
-// that stream only.
+// Builds the operators of m substeps on the world's own stream, without
+// waiting: passes that use them wait for P.ready (band_plan).
 static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
 {
     const int nf = w->nf, dims[3] = {w->nx, w->ny, w->nz};
@@ -856,32 +878,45 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
     if ((e = cudaMemcpyAsync(d + o_host, host.data(), host.size(), cudaMemcpyHostToDevice, w->s_in)) == cudaSuccess &&
         (e = launch_band_setup(reinterpret_cast<BandAxis *>(d + o_axes), 3 * nf, max_rows,
                                reinterpret_cast<BandInit *>(d + o_in), nf, w->s_in)) == cudaSuccess)
-        e = cudaStreamSynchronize(w->s_in);
+        if ((e = cudaEventCreateWithFlags(&P.ready, cudaEventDisableTiming)) == cudaSuccess)
+            e = cudaEventRecord(P.ready, w->s_in);
     if (e != cudaSuccess) {
         cudaFree(P.d);
+        if (P.ready) cudaEventDestroy(P.ready);
         P.d = nullptr;
+        P.ready = nullptr;
     }
     return e;
 }
 
-// The plan of m substeps, built on first use.
-static cudaError_t band_plan(vfd_world *w, int m, const BandPlan **out)
+// The plan of m substeps, built on first use; what follows on `st` may use it
+// (a capture takes in no wait for it: it is complete then).
+static cudaError_t band_plan(vfd_world *w, int m, cudaStream_t st, const BandPlan **out)
 {
     auto it = w->band_plans.find(m);
-    if (it == w->band_plans.end()) {
-        BandPlan P;
-        cudaError_t e = build_band_plan(w, m, P);
-        if (e != cudaSuccess) return e;
-        it = w->band_plans.emplace(m, std::move(P)).first;
+    if (it == w->band_plans.end() || !it->second.done) {
+        CaptureRelaxed scope;
+        cudaError_t e;
+        if (it == w->band_plans.end()) {
+            BandPlan P;
+            if ((e = build_band_plan(w, m, P)) != cudaSuccess) return e;
+            it = w->band_plans.emplace(m, std::move(P)).first;
+        }
+        BandPlan &P = it->second;
+        if (stream_capturing(st)) {
+            if ((e = cudaEventSynchronize(P.ready)) != cudaSuccess) return e;
+            P.done = true;
+        } else if ((e = cudaEventQuery(P.ready)) == cudaErrorNotReady) {
+            cudaGetLastError();
+            if ((e = cudaStreamWaitEvent(st, P.ready, 0)) != cudaSuccess) return e;
+        } else if (e != cudaSuccess) {
+            return e;
+        } else {
+            P.done = true;
+        }
     }
     *out = &it->second;
     return cudaSuccess;
-}
-
-static bool stream_capturing(cudaStream_t st)
-{
-    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
 }
 
 // The sizes of the groups a tick's substeps are folded into: as few as
@@ -914,16 +949,11 @@ static bool runs_band(const vfd_world *w, int n_substeps)
     return 2 * radii > 11 * 3 * w->nf;  // mean radius above 5.5
 }
 
-// What band_groups may fold for a tick of this world.  Operators that are
-// not built yet cannot be while `st` is being captured: then the
-// single-substep ones, which every world has, run the tick.
-static int band_limit(vfd_world *w, int n_substeps, cudaStream_t st)
+// What band_groups may fold for a tick of this world.
+static int band_limit(vfd_world *w, int n_substeps)
 {
     if (n_substeps == 1) return 1;
     if (w->band_mmax == 0) w->band_mmax = band_fold_limit(w, BD_MMAX);
-    if (stream_capturing(st))
-        for (int m : band_groups(n_substeps, w->band_mmax))
-            if (!w->band_plans.count(m)) return 1;
     return w->band_mmax;
 }
 
@@ -1306,7 +1336,7 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         }
         if (band_enabled() && !(ch && ch->pinned) && band_fold_limit(w, 1) >= 1) {
             const BandPlan *P = nullptr;
-            if ((e = band_plan(w, 1, &P)) != cudaSuccess) return bail(e, "banded operators");
+            if ((e = band_plan(w, 1, w->s_in, &P)) != cudaSuccess) return bail(e, "banded operators");
             w->band = true;
         }
         if (!runs_band(w, 1) && (e = build_fft(w)) != cudaSuccess) return bail(e, "FFT passes");
@@ -2031,12 +2061,12 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
     }
     const bool band = runs_band(w, n_substeps);
     if (band) {
-        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps, st));
+        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps));
         double *mass = w->d_mass + (field < 0 ? 0 : (int64_t)field * MS_COUNT);
         const size_t mbytes = sizeof(double) * MS_COUNT * (field < 0 ? w->nf : 1);
         for (size_t g = 0; g < groups.size(); ++g) {
             const BandPlan *P = nullptr;
-            VFD_CUDA(w, band_plan(w, groups[g], &P));
+            VFD_CUDA(w, band_plan(w, groups[g], st, &P));
             const bool last = g + 1 == groups.size();  // the accounting is the last group's
             if (last && P->affine)
                 VFD_CUDA(w, cudaMemcpyAsync(mass, P->d_init + (field < 0 ? 0 : (int64_t)field * MS_COUNT), mbytes,
@@ -2955,7 +2985,7 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
     if ((!oj.empty() && (e = os_prepare()) != cudaSuccess) ||
         ((rfh[0].tiles.size() + rfh[1].tiles.size() + rfh[2].tiles.size()) > 0 && (e = rf_prepare()) != cudaSuccess) ||
         (e = take_arena(b->device, ar.host.size(), &b->d_fft_arena)) != cudaSuccess ||
-        (e = cudaMemcpy(b->d_fft_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
+        (e = cudaMemcpyAsync(b->d_fft_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, b->st)) != cudaSuccess)
         return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
                      std::string("batch setup: ") + cudaGetErrorString(e));
     b->d_fft_mass_ptrs = reinterpret_cast<double **>(b->d_fft_arena + o_mp);
@@ -3001,14 +3031,14 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     std::vector<Host> host;
     for (auto *w : b->worlds) {
         if (!runs_band(w, n_substeps)) continue;
-        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps, b->st));
+        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps));
         if (host.size() < groups.size()) {
             host.resize(groups.size());
             B.launches.resize(groups.size());
         }
         for (size_t g = 0; g < groups.size(); ++g) {
             const BandPlan *P = nullptr;
-            const cudaError_t e = band_plan(w, groups[g], &P);
+            const cudaError_t e = band_plan(w, groups[g], b->st, &P);
             if (e != cudaSuccess)
                 return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
                              std::string("banded operators: ") + cudaGetErrorString(e));
@@ -3034,7 +3064,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
         }
     if (!host.empty()) {
         VFD_BCUDA(b, take_arena(b->device, ar.host.size(), &B.d));
-        const cudaError_t e = cudaMemcpy(B.d, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice);
+        const cudaError_t e = cudaMemcpyAsync(B.d, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, b->st);
         if (e != cudaSuccess) {
             give_arena(b->device, B.d);
             return bfail(b, VFD_ERR_CUDA, std::string("batch setup: ") + cudaGetErrorString(e));
@@ -3050,12 +3080,15 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     return VFD_OK;
 }
 
-// Sets up what a tick of n_substeps needs, outside any capture.
-static vfd_status batch_prepare(vfd_batch *b, int n_substeps)
+// Sets up what a tick of n_substeps needs, outside any capture: complete when
+// it returns if the tick's stream is being captured.
+static vfd_status batch_prepare(vfd_batch *b, int n_substeps, cudaStream_t stream)
 {
-    const vfd_status st = batch_prepare_band(b, n_substeps);
-    if (st != VFD_OK) return st;
-    return batch_prepare_fft(b, batch_fft_worlds(b, n_substeps));
+    CaptureRelaxed scope;
+    vfd_status st = batch_prepare_band(b, n_substeps);
+    if (st == VFD_OK) st = batch_prepare_fft(b, batch_fft_worlds(b, n_substeps));
+    if (st == VFD_OK && stream_capturing(stream)) VFD_BCUDA(b, cudaStreamSynchronize(b->st));
+    return st;
 }
 
 // Times one axis pass of the whole batch as configured now (one warm-up,
@@ -3254,8 +3287,8 @@ vfd_status vfd_batch_tick(vfd_batch *b, int n_substeps, void *stream)
         b->same_ticks = 0;
     }
     ++b->same_ticks;
-    {
-        const vfd_status st = batch_prepare(b, n_substeps);
+    if (!b->exec) {
+        const vfd_status st = batch_prepare(b, n_substeps, (cudaStream_t)stream);
         if (st != VFD_OK) return st;
     }
     VFD_BCUDA(b, cudaEventRecord(b->ev_in, (cudaStream_t)stream));
