@@ -400,3 +400,22 @@ def test_operators_are_ready_on_every_stream(gpu):
         np.testing.assert_array_equal(outs[0][f], outs[0][4 + f])
         np.testing.assert_array_equal(outs[0][f], outs[2][f])
         np.testing.assert_array_equal(outs[1][f], outs[1][4 + f])
+
+
+def test_operators_are_built_for_ticks_that_use_them(gpu):
+    """A large world of narrow kernels runs single substeps on the FFT passes:
+    it holds no banded operators until a tick of several substeps."""
+    grid, params = (256, 160, 128), [vfd.field_params(0.9, 0.02)] * 2
+    vfd.autotune_clear()
+    try:
+        with vfd.World(*grid, params) as w:
+            w.tick(1)
+            single = w.device_bytes()
+            w.tick(10)
+            assert w.device_bytes() > single
+        vfd.autotune_set(*grid, params, [{"method": "register_fft"}] * 3)
+        with vfd.World(*grid, params) as w:  # no banded products at all
+            w.tick(1)
+            assert w.device_bytes() == single
+    finally:
+        vfd.autotune_clear()

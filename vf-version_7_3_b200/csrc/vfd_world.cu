@@ -1334,12 +1334,12 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
             for (int f = 0; f < w->nf && ok; ++f) ok = rf_eligible(make_os_job(w, f, a, 0, false));
             w->use_rf[a] = ok;
         }
-        if (band_enabled() && !(ch && ch->pinned) && band_fold_limit(w, 1) >= 1) {
-            const BandPlan *P = nullptr;
-            if ((e = band_plan(w, 1, w->s_in, &P)) != cudaSuccess) return bail(e, "banded operators");
-            w->band = true;
-        }
-        if (!runs_band(w, 1) && (e = build_fft(w)) != cudaSuccess) return bail(e, "FFT passes");
+        w->band = band_enabled() && !(ch && ch->pinned) && band_fold_limit(w, 1) >= 1;
+        // what a single substep takes is set up now, the rest where a tick needs it
+        const BandPlan *P = nullptr;
+        if (runs_band(w, 1)) e = band_plan(w, 1, w->s_in, &P);
+        else e = build_fft(w);
+        if (e != cudaSuccess) return bail(e, "the passes' operators");
     }
     if ((e = cudaStreamCreateWithFlags(&w->s_cmp, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
     if ((e = cudaStreamCreateWithFlags(&w->s_out, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
