@@ -419,3 +419,31 @@ def test_operators_are_built_for_ticks_that_use_them(gpu):
             assert w.device_bytes() == single
     finally:
         vfd.autotune_clear()
+
+
+def test_batch_alternates_substep_counts(gpu):
+    """Ticks of one and of several substeps in turn, over worlds that take the
+    FFT passes always (pinned), for single substeps (large, narrow kernels) and
+    never: every tick equals the world's own."""
+    vfd.autotune_clear()
+    try:
+        vfd.autotune_set(44, 40, 36, [vfd.field_params(1.0, 0.02)] * 2, [{"method": "register_fft"}] * 3)
+        specs = [((44, 40, 36), 1.0), ((176, 160, 96), 0.9), ((90, 33, 70), 2.6)]
+        worlds, singles = [], []
+        for i, (g, sig) in enumerate(specs):
+            for out in (worlds, singles):
+                w = vfd.World(*g, [vfd.field_params(sig, 0.02)] * 2)
+                for f in range(2):
+                    w.upload(f, vfd.synth_field(3, i, f, g[::-1]))
+                out.append(w)
+        with vfd.Batch(worlds) as b:
+            for n in (1, 4, 1, 4, 4, 4, 1, 1, 1, 6, 1):
+                b.tick(n)
+                for w, v in zip(worlds, singles):
+                    v.tick(n)
+                    for f in range(2):
+                        np.testing.assert_array_equal(w.download(f), v.download(f))
+        for w in worlds + singles:
+            w.close()
+    finally:
+        vfd.autotune_clear()

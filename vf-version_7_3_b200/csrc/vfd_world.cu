@@ -2591,33 +2591,40 @@ struct BatchBand {
 };
 constexpr size_t BATCH_BANDS = 4;  // substep counts whose arrays a batch keeps
 
+// The FFT passes of some of a batch's worlds.
+struct BatchFft {
+    std::vector<vfd_world *> worlds;
+    bool ready = false;
+    bool each = false;                // they take different passes: each world launches its own
+    unsigned char *d_arena = nullptr;
+    double **d_mass_ptrs = nullptr;   // the worlds' accounting blocks
+    int *d_mass_counts = nullptr;
+    int njobs = 0;
+    int tiles[3] = {0, 0, 0};
+    AxisJob *d_jobs = nullptr;        // [3][njobs]
+    bool use_os[3] = {false, false, false};
+    OsJob *d_osjobs = nullptr;        // [3][njobs]
+    int os_tiles[3] = {0, 0, 0};
+    OsTileInfo *d_os_tiles[3] = {nullptr, nullptr, nullptr};
+    bool os_tiles_owned[3] = {true, true, true};
+    bool use_rf[3] = {false, false, false};
+    std::vector<RfGroup> rf[3];
+    std::vector<OsJob> oj;            // host copy of the overlap-save jobs ([axis][njobs])
+};
+
 // A world's tick runs on banded products or on FFT passes whatever else is in
 // the batch (a request's result does not depend on its neighbours): a batch
 // launches each axis pass for the worlds of either kind.
 struct vfd_batch {
     std::map<int, BatchBand> bands;                   // by a tick's substeps
-    std::vector<vfd_world *> fft_worlds;              // the worlds whose FFT passes the arrays below hold
-    bool fft_ready = false;
-    bool fft_each = false;                            // they take different passes: each world launches its own
+    BatchFft fft[2];                                  // of a tick of one substep / of several
     int tuned_method[3] = {PASS_METHOD_AUTO, PASS_METHOD_AUTO, PASS_METHOD_AUTO};
-    unsigned char *d_fft_arena = nullptr;
-    double **d_fft_mass_ptrs = nullptr;               // their accounting blocks
-    int *d_fft_mass_counts = nullptr;
     int device = 0;
     std::vector<vfd_world *> worlds;
     int variant[3] = {0, 0, 0};
-    int tiles[3] = {0, 0, 0};
     int Fmax[3] = {0, 0, 0};
-    int njobs = 0;
-    AxisJob *d_jobs = nullptr;  // [3][njobs]
-    bool use_os[3] = {false, false, false};
     int rmin[3] = {0, 0, 0};
-    OsJob *d_osjobs = nullptr;  // [3][njobs]
-    int os_tiles[3] = {0, 0, 0};
-    OsTileInfo *d_os_tiles[3] = {nullptr, nullptr, nullptr};
     int os_minb[3] = {0, 0, 0};
-    bool use_rf[3] = {false, false, false};
-    std::vector<RfGroup> rf[3];
     cudaStream_t st = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;
     cudaGraph_t graph = nullptr;
@@ -2629,8 +2636,6 @@ struct vfd_batch {
     double **d_mass_ptrs = nullptr;  // every world's accounting block, zeroed per substep in one launch
     int *d_mass_counts = nullptr;
     unsigned char *d_arena = nullptr;  // the arrays set up at creation, in one allocation
-    bool os_tiles_owned[3] = {true, true, true};
-    std::vector<OsJob> oj;       // host copy of the overlap-save jobs ([axis][njobs])
     bool can_os[3] = {false, false, false};
     float tuned_ms[3] = {0.0f, 0.0f, 0.0f};
     std::string err;
@@ -2719,6 +2724,16 @@ static void give_arena(int dev, unsigned char *p)
     g_bcache.arenas[dev].insert({it->second.first, p});
 }
 
+static void free_batch_fft(int device, BatchFft &F)
+{
+    for (int a = 0; a < 3; ++a) {
+        if (F.os_tiles_owned[a]) cudaFree(F.d_os_tiles[a]);
+        free_rf_groups(F.rf[a]);
+    }
+    give_arena(device, F.d_arena);
+    F = BatchFft();
+}
+
 static void batch_release(vfd_batch *b)
 {
     int prev = 0;
@@ -2726,16 +2741,11 @@ static void batch_release(vfd_batch *b)
     cudaSetDevice(b->device);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
-    for (int a = 0; a < 3; ++a) {
-        if (b->os_tiles_owned[a]) cudaFree(b->d_os_tiles[a]);
-        free_rf_groups(b->rf[a]);
-    }
-    // d_jobs, d_osjobs, the mass arrays and the arena-placed tiles: the
-    // arena is kept for the next batch on this device (the batch's work is
+    // arenas are kept for the next batch on this device (the batch's work is
     // complete when it is destroyed)
     if (b->d_arena) cudaStreamSynchronize(b->st);
+    for (auto &F : b->fft) free_batch_fft(b->device, F);
     give_arena(b->device, b->d_arena);
-    give_arena(b->device, b->d_fft_arena);
     for (auto &kv : b->bands) give_arena(b->device, kv.second.d);
     bool kept = false;
     if (b->st && b->ev_in && b->ev_out && b->device >= 0 && b->device < 64) {
@@ -2758,13 +2768,13 @@ extern "C" {
 
 // Whether every job of axis a (oj: [axis][njobs]) can take the register-FFT
 // pass and every world allows it there.
-static bool batch_rf_possible(const vfd_batch *b, const std::vector<OsJob> &oj, int a)
+static bool batch_rf_possible(const BatchFft &F, const std::vector<OsJob> &oj, int a)
 {
-    if (!rf_enabled() || !b->use_os[a]) return false;
-    for (auto *w : b->fft_worlds)
+    if (!rf_enabled() || !F.use_os[a]) return false;
+    for (auto *w : F.worlds)
         if (!w->allow_rf[a]) return false;
-    for (int i = 0; i < b->njobs; ++i)
-        if (!rf_eligible(oj[(size_t)a * b->njobs + i])) return false;
+    for (int i = 0; i < F.njobs; ++i)
+        if (!rf_eligible(oj[(size_t)a * F.njobs + i])) return false;
     return true;
 }
 
@@ -2801,7 +2811,7 @@ static std::vector<vfd_world *> batch_fft_worlds(const vfd_batch *b, int n_subst
         if (!runs_band(w, n_substeps)) out.push_back(w);
     return out;
 }
-static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *> &ws);
+static vfd_status batch_prepare_fft(vfd_batch *b, BatchFft &F, const std::vector<vfd_world *> &ws);
 
 vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **out)
 {
@@ -2843,7 +2853,6 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
             all = all && w->use_os[a];
             for (int f = 0; f < w->nf; ++f) rmn = std::min(rmn, w->params[f].radius[a]);
         }
-        b->use_os[a] = all;
         b->can_os[a] = all;
         b->rmin[a] = rmn;
         b->os_minb[a] = b->worlds[0]->os_minb[a];
@@ -2873,7 +2882,7 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
     b->d_mass_counts = reinterpret_cast<int *>(b->d_arena + o_mc);
     b->gens.assign(n_worlds, ~0ull);
     // the FFT passes of single-substep ticks: set up now rather than in the first
-    const vfd_status st = batch_prepare_fft(b, batch_fft_worlds(b, 1));
+    const vfd_status st = batch_prepare_fft(b, b->fft[0], batch_fft_worlds(b, 1));
     if (st != VFD_OK) {
         const std::string msg = b->err;
         batch_release(b);
@@ -2887,39 +2896,25 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
 // The arrays of the FFT passes, set up when a tick or the tuner needs them (a
 // server rebuilds its batch whenever the active set changes, and its batches
 // may never need them).
-static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *> &ws)
+static vfd_status batch_prepare_fft(vfd_batch *b, BatchFft &F, const std::vector<vfd_world *> &ws)
 {
-    if (b->fft_ready && ws == b->fft_worlds) return VFD_OK;
-    if (b->fft_ready) {
-        // another set of worlds than the arrays hold
-        VFD_BCUDA(b, cudaStreamSynchronize(b->st));
-        for (int a = 0; a < 3; ++a) {
-            if (b->os_tiles_owned[a]) cudaFree(b->d_os_tiles[a]);
-            b->d_os_tiles[a] = nullptr;
-            b->os_tiles_owned[a] = true;
-            free_rf_groups(b->rf[a]);
-            b->use_rf[a] = false;
-        }
-        give_arena(b->device, b->d_fft_arena);
-        b->d_fft_arena = nullptr;
-        b->fft_ready = false;
-    }
-    b->fft_worlds = ws;
-    b->njobs = 0;
-    for (auto *w : ws) b->njobs += w->nf;
-    if (b->njobs == 0) {
-        b->fft_ready = true;
+    if (F.ready) return VFD_OK;
+    free_batch_fft(b->device, F);  // what an attempt that failed left
+    F.worlds = ws;
+    for (auto *w : ws) F.njobs += w->nf;
+    if (F.njobs == 0) {
+        F.ready = true;
         return VFD_OK;
     }
     for (auto *w : ws) VFD_BCUDA(b, build_fft(w));
-    b->fft_each = false;
+    F.each = false;
     for (int a = 0; a < 3; ++a)
         for (auto *w : ws)
             if (b->tuned_method[a] == PASS_METHOD_AUTO &&
                 (w->use_rf[a] != ws[0]->use_rf[a] || w->use_os[a] != b->can_os[a]))
-                b->fft_each = true;
+                F.each = true;
     for (int a = 0; a < 3; ++a)  // a tuned axis keeps its pass
-        if (b->tuned_method[a] != PASS_METHOD_AUTO) b->use_os[a] = b->can_os[a] && b->tuned_method[a] != PASS_METHOD_FULL;
+        F.use_os[a] = b->can_os[a] && b->tuned_method[a] != PASS_METHOD_FULL;
     std::vector<AxisJob> jobs;
     for (int a = 0; a < 3; ++a) {
         const int nl = kAxisVariants[b->variant[a]].nl;
@@ -2929,11 +2924,11 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
                 jobs.push_back(make_job(w, f, a, tb, nl));
                 tb += field_tiles(w, a, nl);
             }
-        b->tiles[a] = tb;
+        F.tiles[a] = tb;
     }
     std::vector<OsJob> oj;
     std::vector<OsTileInfo> tile_info[3];
-    if (b->use_os[0] || b->use_os[1] || b->use_os[2]) {
+    if (F.use_os[0] || F.use_os[1] || F.use_os[2]) {
         for (int a = 0; a < 3; ++a) {
             int tb = 0;
             for (auto *w : ws)
@@ -2946,7 +2941,7 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
                     }
                     tb += os_field_tiles(oj.back());
                 }
-            b->os_tiles[a] = tb;
+            F.os_tiles[a] = tb;
         }
     }
     // Per axis: the register-FFT pass when every job and world allows it,
@@ -2957,12 +2952,12 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
     for (int a = 0; a < 3 && !oj.empty(); ++a) {
         const int want = b->tuned_method[a];
         if (want == PASS_METHOD_FULL) continue;
-        if (want != PASS_METHOD_OS && batch_rf_possible(b, oj, a)) {
-            rf_group_host(&oj[(size_t)a * b->njobs], b->njobs, rfh[a]);
+        if (want != PASS_METHOD_OS && batch_rf_possible(F, oj, a)) {
+            rf_group_host(&oj[(size_t)a * F.njobs], F.njobs, rfh[a]);
             if (!rfh[a].tiles.empty()) continue;
         }
-        if (b->use_os[a])
-            for (int i = 0; i < b->njobs; ++i) os_append_tiles(oj[(size_t)a * b->njobs + i], i, tile_info[a]);
+        if (F.use_os[a])
+            for (int i = 0; i < F.njobs; ++i) os_append_tiles(oj[(size_t)a * F.njobs + i], i, tile_info[a]);
     }
     std::vector<double *> mp;
     std::vector<int> mc;
@@ -2984,19 +2979,19 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
     cudaError_t e = cudaSuccess;
     if ((!oj.empty() && (e = os_prepare()) != cudaSuccess) ||
         ((rfh[0].tiles.size() + rfh[1].tiles.size() + rfh[2].tiles.size()) > 0 && (e = rf_prepare()) != cudaSuccess) ||
-        (e = take_arena(b->device, ar.host.size(), &b->d_fft_arena)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(b->d_fft_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, b->st)) != cudaSuccess)
+        (e = take_arena(b->device, ar.host.size(), &F.d_arena)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(F.d_arena, ar.host.data(), ar.host.size(), cudaMemcpyHostToDevice, b->st)) != cudaSuccess)
         return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
                      std::string("batch setup: ") + cudaGetErrorString(e));
-    b->d_fft_mass_ptrs = reinterpret_cast<double **>(b->d_fft_arena + o_mp);
-    b->d_fft_mass_counts = reinterpret_cast<int *>(b->d_fft_arena + o_mc);
-    unsigned char *base = b->d_fft_arena;
-    b->d_jobs = reinterpret_cast<AxisJob *>(base + o_jobs);
-    b->d_osjobs = oj.empty() ? nullptr : reinterpret_cast<OsJob *>(base + o_oj);
+    F.d_mass_ptrs = reinterpret_cast<double **>(F.d_arena + o_mp);
+    F.d_mass_counts = reinterpret_cast<int *>(F.d_arena + o_mc);
+    unsigned char *base = F.d_arena;
+    F.d_jobs = reinterpret_cast<AxisJob *>(base + o_jobs);
+    F.d_osjobs = oj.empty() ? nullptr : reinterpret_cast<OsJob *>(base + o_oj);
     for (int a = 0; a < 3; ++a) {
         if (!tile_info[a].empty()) {
-            b->d_os_tiles[a] = reinterpret_cast<OsTileInfo *>(base + o_ost[a]);
-            b->os_tiles_owned[a] = false;
+            F.d_os_tiles[a] = reinterpret_cast<OsTileInfo *>(base + o_ost[a]);
+            F.os_tiles_owned[a] = false;
         }
         if (!rfh[a].tiles.empty()) {
             RfGroup rg;
@@ -3004,12 +2999,12 @@ static vfd_status batch_prepare_fft(vfd_batch *b, const std::vector<vfd_world *>
             rg.d_tiles = reinterpret_cast<OsTileInfo *>(base + o_rft[a]);
             rg.d_maps = rfh[a].maps.empty() ? nullptr : reinterpret_cast<CUtensorMap *>(base + o_rfm[a]);
             rg.owned = false;
-            b->rf[a].push_back(rg);
-            b->use_rf[a] = true;
+            F.rf[a].push_back(rg);
+            F.use_rf[a] = true;
         }
     }
-    b->oj.swap(oj);
-    b->fft_ready = true;
+    F.oj.swap(oj);
+    F.ready = true;
     return VFD_OK;
 }
 
@@ -3086,24 +3081,24 @@ static vfd_status batch_prepare(vfd_batch *b, int n_substeps, cudaStream_t strea
 {
     CaptureRelaxed scope;
     vfd_status st = batch_prepare_band(b, n_substeps);
-    if (st == VFD_OK) st = batch_prepare_fft(b, batch_fft_worlds(b, n_substeps));
+    if (st == VFD_OK) st = batch_prepare_fft(b, b->fft[n_substeps > 1], batch_fft_worlds(b, n_substeps));
     if (st == VFD_OK && stream_capturing(stream)) VFD_BCUDA(b, cudaStreamSynchronize(b->st));
     return st;
 }
 
 // Times one axis pass of the whole batch as configured now (one warm-up,
 // `reps` timed launches, CUDA events on the batch stream).
-static vfd_status batch_time_axis(vfd_batch *b, int a, int reps, cudaEvent_t e0, cudaEvent_t e1, float *ms)
+static vfd_status batch_time_axis(vfd_batch *b, const BatchFft &F, int a, int reps, cudaEvent_t e0, cudaEvent_t e1, float *ms)
 {
     for (int it = -1; it < reps; ++it) {
         if (it == 0) VFD_BCUDA(b, cudaEventRecord(e0, b->st));
-        if (b->use_rf[a])
-            VFD_BCUDA(b, launch_rf_groups(b->d_osjobs + a * b->njobs, b->rf[a], a, b->st));
-        else if (b->use_os[a])
-            VFD_BCUDA(b, launch_os(b->d_osjobs + a * b->njobs, b->d_os_tiles[a], b->os_tiles[a], b->rmin[a], a, b->st,
+        if (F.use_rf[a])
+            VFD_BCUDA(b, launch_rf_groups(F.d_osjobs + a * F.njobs, F.rf[a], a, b->st));
+        else if (F.use_os[a])
+            VFD_BCUDA(b, launch_os(F.d_osjobs + a * F.njobs, F.d_os_tiles[a], F.os_tiles[a], b->rmin[a], a, b->st,
                                    b->os_minb[a]));
         else
-            VFD_BCUDA(b, launch_axis(b->variant[a], b->d_jobs + a * b->njobs, b->njobs, b->tiles[a], b->Fmax[a],
+            VFD_BCUDA(b, launch_axis(b->variant[a], F.d_jobs + a * F.njobs, F.njobs, F.tiles[a], b->Fmax[a],
                                      b->st));
     }
     VFD_BCUDA(b, cudaEventRecord(e1, b->st));
@@ -3120,8 +3115,13 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
     DeviceGuard g(b->device);
     VFD_BCUDA(b, cudaStreamSynchronize(b->st));
     // the tuner times every world, and one pass an axis for all of them
-    const vfd_status ready = batch_prepare_fft(b, b->worlds);
-    if (ready != VFD_OK) return ready;
+    for (int a = 0; a < 3; ++a) b->tuned_method[a] = PASS_METHOD_AUTO;
+    BatchFft F;
+    const vfd_status ready = batch_prepare_fft(b, F, b->worlds);
+    if (ready != VFD_OK) {
+        free_batch_fft(b->device, F);
+        return ready;
+    }
     // the passes run on the worlds' own fields: save them, restore after
     std::vector<float *> saved(b->worlds.size(), nullptr);
     auto restore = [&](bool copy) {
@@ -3140,6 +3140,7 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
             e = cudaMemcpyAsync(saved[i], w->d_fields, sizeof(float) * w->V * w->nf, cudaMemcpyDeviceToDevice, b->st);
         if (e != cudaSuccess) {
             restore(false);
+            free_batch_fft(b->device, F);
             return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
                          std::string("autotune backup: ") + cudaGetErrorString(e));
         }
@@ -3150,26 +3151,26 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
     vfd_status st = VFD_OK;
     for (int a = 0; a < 3 && st == VFD_OK; ++a) {
         // register-FFT groups for this axis if every job allows them
-        bool rf_ok = !b->rf[a].empty();
-        if (!rf_ok && b->can_os[a] && rf_enabled() && !b->oj.empty()) {
+        bool rf_ok = !F.rf[a].empty();
+        if (!rf_ok && b->can_os[a] && rf_enabled() && !F.oj.empty()) {
             bool ok = true;
-            for (int i = 0; i < b->njobs; ++i) ok = ok && rf_eligible(b->oj[(size_t)a * b->njobs + i]);
+            for (int i = 0; i < F.njobs; ++i) ok = ok && rf_eligible(F.oj[(size_t)a * F.njobs + i]);
             if (ok && rf_prepare() == cudaSuccess &&
-                build_rf_groups(&b->oj[(size_t)a * b->njobs], b->njobs, b->rf[a]) == cudaSuccess)
-                rf_ok = !b->rf[a].empty();
+                build_rf_groups(&F.oj[(size_t)a * F.njobs], F.njobs, F.rf[a]) == cudaSuccess)
+                rf_ok = !F.rf[a].empty();
         }
         struct Cand {
             int method, minb;
         };
-        if (b->can_os[a] && !b->d_os_tiles[a] && !b->oj.empty()) {
+        if (b->can_os[a] && !F.d_os_tiles[a] && !F.oj.empty()) {
             std::vector<OsTileInfo> ti;
-            for (int i = 0; i < b->njobs; ++i) os_append_tiles(b->oj[(size_t)a * b->njobs + i], i, ti);
-            if (upload_vec(&b->d_os_tiles[a], ti) != cudaSuccess) b->d_os_tiles[a] = nullptr;
-            b->os_tiles_owned[a] = true;
+            for (int i = 0; i < F.njobs; ++i) os_append_tiles(F.oj[(size_t)a * F.njobs + i], i, ti);
+            if (upload_vec(&F.d_os_tiles[a], ti) != cudaSuccess) F.d_os_tiles[a] = nullptr;
+            F.os_tiles_owned[a] = true;
         }
         std::vector<Cand> cands;
         if (rf_ok) cands.push_back({PASS_METHOD_RF, 0});
-        if (b->can_os[a] && b->d_os_tiles[a]) {
+        if (b->can_os[a] && F.d_os_tiles[a]) {
             cands.push_back({PASS_METHOD_OS, 3});
             cands.push_back({PASS_METHOD_OS, 4});
         }
@@ -3177,19 +3178,17 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
         float best = 0.0f;
         Cand bc = cands.back();
         for (const Cand &c : cands) {
-            b->use_rf[a] = c.method == PASS_METHOD_RF;
-            b->use_os[a] = c.method == PASS_METHOD_OS;
+            F.use_rf[a] = c.method == PASS_METHOD_RF;
+            F.use_os[a] = c.method == PASS_METHOD_OS;
             b->os_minb[a] = c.minb;
             float ms = 0.0f;
-            st = batch_time_axis(b, a, reps, e0, e1, &ms);
+            st = batch_time_axis(b, F, a, reps, e0, e1, &ms);
             if (st != VFD_OK) break;
             if (best == 0.0f || ms < best) {
                 best = ms;
                 bc = c;
             }
         }
-        b->use_rf[a] = bc.method == PASS_METHOD_RF;
-        b->use_os[a] = bc.method == PASS_METHOD_OS;
         b->os_minb[a] = bc.minb;
         b->tuned_ms[a] = best;
         b->tuned_method[a] = bc.method;
@@ -3207,7 +3206,8 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     restore(true);
-    b->fft_each = false;
+    free_batch_fft(b->device, F);
+    for (auto &G : b->fft) free_batch_fft(b->device, G);  // set up anew with the chosen passes
     // the next tick runs directly and re-captures its graph with the chosen passes
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -3230,28 +3230,29 @@ static vfd_status batch_enqueue(vfd_batch *b, int n_substeps)
 {
     VFD_BCUDA(b, launch_zero_blocks(b->d_mass_ptrs, b->d_mass_counts, (int)b->worlds.size(), b->st));
     const BatchBand &B = b->bands.at(n_substeps);
+    const BatchFft &F = b->fft[n_substeps > 1];
     for (const auto &x : B.affine)
         VFD_BCUDA(b, cudaMemcpyAsync(x.first->d_mass, x.second, sizeof(double) * MS_COUNT * x.first->nf,
                                      cudaMemcpyDeviceToDevice, b->st));
     for (const auto &L : B.launches)
         for (int a = 0; a < 3; ++a)
             VFD_BCUDA(b, launch_band(L.d_jobs[a], L.d_tjob[a], 0, L.ntiles[a], a, L.geo[a], true, b->st));
-    for (size_t i = 0; b->fft_each && i < b->fft_worlds.size(); ++i) {
-        const vfd_status st = enqueue_fft_substeps(b->fft_worlds[i], -1, n_substeps, b->st);
-        if (st != VFD_OK) return bfail(b, st, b->fft_worlds[i]->err);
+    for (size_t i = 0; F.each && i < F.worlds.size(); ++i) {
+        const vfd_status st = enqueue_fft_substeps(F.worlds[i], -1, n_substeps, b->st);
+        if (st != VFD_OK) return bfail(b, st, F.worlds[i]->err);
     }
-    for (int s = 0; s < n_substeps && b->njobs > 0 && !b->fft_each; ++s) {
+    for (int s = 0; s < n_substeps && F.njobs > 0 && !F.each; ++s) {
         if (s > 0)
-            VFD_BCUDA(b, launch_zero_blocks(b->d_fft_mass_ptrs, b->d_fft_mass_counts, (int)b->fft_worlds.size(),
+            VFD_BCUDA(b, launch_zero_blocks(F.d_mass_ptrs, F.d_mass_counts, (int)F.worlds.size(),
                                             b->st));
         for (int a = 0; a < 3; ++a) {
-            if (b->use_rf[a])
-                VFD_BCUDA(b, launch_rf_groups(b->d_osjobs + a * b->njobs, b->rf[a], a, b->st));
-            else if (b->use_os[a])
-                VFD_BCUDA(b, launch_os(b->d_osjobs + a * b->njobs, b->d_os_tiles[a], b->os_tiles[a], b->rmin[a], a,
+            if (F.use_rf[a])
+                VFD_BCUDA(b, launch_rf_groups(F.d_osjobs + a * F.njobs, F.rf[a], a, b->st));
+            else if (F.use_os[a])
+                VFD_BCUDA(b, launch_os(F.d_osjobs + a * F.njobs, F.d_os_tiles[a], F.os_tiles[a], b->rmin[a], a,
                                        b->st, b->os_minb[a]));
             else
-                VFD_BCUDA(b, launch_axis(b->variant[a], b->d_jobs + a * b->njobs, b->njobs, b->tiles[a],
+                VFD_BCUDA(b, launch_axis(b->variant[a], F.d_jobs + a * F.njobs, F.njobs, F.tiles[a],
                                          b->Fmax[a], b->st));
         }
     }
