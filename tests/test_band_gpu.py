@@ -447,3 +447,22 @@ def test_batch_alternates_substep_counts(gpu):
             w.close()
     finally:
         vfd.autotune_clear()
+
+
+def test_batch_of_many_fields(gpu):
+    """More than 65535 fields in one batch."""
+    grid, nf, n = (4, 3, 2), 1200, 56
+    params = [vfd.field_params(0.5, 0.02)] * nf
+    worlds = [vfd.World(*grid, params) for _ in range(n)]
+    u = [vfd.synth_field(7, 0, f, grid[::-1]) for f in range(4)]
+    probe = [(0, 0), (n // 2, 5), (n - 1, nf - 1), (n - 2, 17)]
+    for k, (i, f) in enumerate(probe):
+        worlds[i].upload(f, u[k])
+    with vfd.Batch(worlds) as b:
+        b.tick(2)
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    for k, (i, f) in enumerate(probe):
+        assert rel_l2(worlds[i].download(f), oracle.tick(u[k], 0.5, 0.02, 2, *none)) <= PER_GROUP
+    assert not worlds[1].download(3).any()
+    for w in worlds:
+        w.close()

@@ -218,11 +218,11 @@ __device__ __forceinline__ double band_warp_sum(double v)
 // A launch's tiles: tile t belongs to job jobs[tjob[t]].
 struct BandTiles {
     const BandJob *jobs;
-    const unsigned short *tjob;
+    const int *tjob;
     int begin, end;
     __device__ __forceinline__ int first() const { return begin + (int)blockIdx.x; }
     // tile t's job, or -1
-    __device__ __forceinline__ int job(int t) const { return t < end ? (int)__ldg(tjob + t) : -1; }
+    __device__ __forceinline__ int job(int t) const { return t < end ? __ldg(tjob + t) : -1; }
     // copies a job to the warp's place in shared memory
     __device__ __forceinline__ void load(int j, BandJob *to, int lane) const
     {
@@ -878,7 +878,7 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
 
 template <int AXIS>
 __global__ void __launch_bounds__(BD_THREADS, 1)
-    band_kernel(const BandJob *__restrict__ jobs, const unsigned short *__restrict__ tjob, int tile_begin, int tile_end,
+    band_kernel(const BandJob *__restrict__ jobs, const int *__restrict__ tjob, int tile_begin, int tile_end,
                 int sums, int nstage, int nslots, int slot_bytes)
 {
     extern __shared__ unsigned char dyn_[];
@@ -1143,7 +1143,7 @@ __global__ void band_init_kernel(const BandInit *init, int nfields)
 }
 
 template <int AXIS>
-cudaError_t launch_band_t(const BandJob *jobs, const unsigned short *tjob, int tile_begin, int ntiles, BandGeom geo,
+cudaError_t launch_band_t(const BandJob *jobs, const int *tjob, int tile_begin, int ntiles, BandGeom geo,
                           bool sums, cudaStream_t st)
 {
     static thread_local unsigned long long ctx_done = 0;
@@ -1229,7 +1229,7 @@ cudaError_t launch_band_setup(const BandAxis *axes, int naxes, int max_rows, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_band(const BandJob *jobs, const unsigned short *tjob, int tile_begin, int ntiles, int axis,
+cudaError_t launch_band(const BandJob *jobs, const int *tjob, int tile_begin, int ntiles, int axis,
                         BandGeom geo, bool sums, cudaStream_t st)
 {
     if (ntiles <= 0) return cudaSuccess;

@@ -102,7 +102,7 @@ cudaError_t launch_band_setup(const BandAxis *axes, int naxes, int max_rows, con
 struct BandGeom {
     int ksteps = 0;  // largest of the jobs
 };
-cudaError_t launch_band(const BandJob *jobs, const unsigned short *tjob, int tile_begin, int ntiles, int axis,
+cudaError_t launch_band(const BandJob *jobs, const int *tjob, int tile_begin, int ntiles, int axis,
                         BandGeom geo, bool sums, cudaStream_t st);
 
 // The passes' bounded wait on a barrier that nothing completes: it gives up

@@ -357,7 +357,7 @@ struct BandPlan {
     size_t bytes = 0;
     std::vector<BandJob> jobs;          // [axis][field]
     BandJob *d_jobs[3] = {nullptr, nullptr, nullptr};
-    unsigned short *d_tjob[3] = {nullptr, nullptr, nullptr};
+    int *d_tjob[3] = {nullptr, nullptr, nullptr};
     BandGeom geo[3];
     int ntiles[3] = {0, 0, 0};
     const double *d_init = nullptr;     // [field][MS_COUNT] accounting start
@@ -820,7 +820,7 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
                  o_in = take(sizeof(BandInit) * nf), o_tp = take(sizeof(double) * taps.size());
     const size_t o_maps = take(sizeof(CUtensorMap) * P.jobs.size());
     size_t o_tj[3];
-    for (int a = 0; a < 3; ++a) o_tj[a] = take(sizeof(unsigned short) * P.ntiles[a]);
+    for (int a = 0; a < 3; ++a) o_tj[a] = take(sizeof(int) * P.ntiles[a]);
     cudaError_t e = cudaMalloc(&P.d, off);
     if (e != cudaSuccess) {
         P.d = nullptr;
@@ -871,9 +871,9 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
     memcpy(host.data() + (o_in - o_host), in.data(), sizeof(BandInit) * nf);
     memcpy(host.data() + (o_tp - o_host), taps.data(), sizeof(double) * taps.size());
     for (int a = 0; a < 3; ++a) {
-        P.d_tjob[a] = reinterpret_cast<unsigned short *>(d + o_tj[a]);
-        unsigned short *t = reinterpret_cast<unsigned short *>(host.data() + (o_tj[a] - o_host));
-        for (int f = 0; f < nf; ++f) t = std::fill_n(t, P.jobs[(size_t)a * nf + f].ntiles, (unsigned short)f);
+        P.d_tjob[a] = reinterpret_cast<int *>(d + o_tj[a]);
+        int *t = reinterpret_cast<int *>(host.data() + (o_tj[a] - o_host));
+        for (int f = 0; f < nf; ++f) t = std::fill_n(t, P.jobs[(size_t)a * nf + f].ntiles, f);
     }
     if ((e = cudaMemcpyAsync(d + o_host, host.data(), host.size(), cudaMemcpyHostToDevice, w->s_in)) == cudaSuccess &&
         (e = launch_band_setup(reinterpret_cast<BandAxis *>(d + o_axes), 3 * nf, max_rows,
@@ -2581,7 +2581,7 @@ vfd_status vfd_diffuse_update_host(vfd_world *w, float *const *host_p, float *co
 struct BatchBand {
     struct Launch {
         BandJob *d_jobs[3] = {nullptr, nullptr, nullptr};
-        unsigned short *d_tjob[3] = {nullptr, nullptr, nullptr};
+        int *d_tjob[3] = {nullptr, nullptr, nullptr};
         BandGeom geo[3];
         int ntiles[3] = {0, 0, 0};
     };
@@ -2840,12 +2840,6 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
             return bfail(nullptr, VFD_ERR_NOT_SUPPORTED, "no kernel variant fits every world's FFT plan");
         }
     }
-    int64_t njobs = 0;
-    for (auto *w : b->worlds) njobs += w->nf;
-    if (njobs > 65535) {
-        delete b;
-        return bfail(nullptr, VFD_ERR_NOT_SUPPORTED, "more than 65535 fields in a batch");
-    }
     for (int a = 0; a < 3; ++a) {
         bool all = true;
         int rmn = 1 << 30;
@@ -3020,7 +3014,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     BatchBand B;
     struct Host {
         std::vector<BandJob> jobs[3];
-        std::vector<unsigned short> tjob[3];
+        std::vector<int> tjob[3];
         size_t o_j[3], o_t[3];
     };
     std::vector<Host> host;
@@ -3043,7 +3037,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
                     BandJob j = P->jobs[(size_t)a * w->nf + f];
                     j.tile0 = (int)host[g].tjob[a].size();
                     j.sums = last;
-                    host[g].tjob[a].insert(host[g].tjob[a].end(), j.ntiles, (unsigned short)host[g].jobs[a].size());
+                    host[g].tjob[a].insert(host[g].tjob[a].end(), j.ntiles, (int)host[g].jobs[a].size());
                     host[g].jobs[a].push_back(j);
                 }
                 B.launches[g].geo[a].ksteps = std::max(B.launches[g].geo[a].ksteps, P->geo[a].ksteps);
@@ -3055,7 +3049,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     for (auto &h : host)
         for (int a = 0; a < 3; ++a) {
             h.o_j[a] = ar.add(h.jobs[a].data(), sizeof(BandJob) * h.jobs[a].size());
-            h.o_t[a] = ar.add(h.tjob[a].data(), sizeof(unsigned short) * h.tjob[a].size());
+            h.o_t[a] = ar.add(h.tjob[a].data(), sizeof(int) * h.tjob[a].size());
         }
     if (!host.empty()) {
         VFD_BCUDA(b, take_arena(b->device, ar.host.size(), &B.d));
@@ -3068,7 +3062,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     for (size_t g = 0; g < host.size(); ++g)
         for (int a = 0; a < 3; ++a) {
             B.launches[g].d_jobs[a] = reinterpret_cast<BandJob *>(B.d + host[g].o_j[a]);
-            B.launches[g].d_tjob[a] = reinterpret_cast<unsigned short *>(B.d + host[g].o_t[a]);
+            B.launches[g].d_tjob[a] = reinterpret_cast<int *>(B.d + host[g].o_t[a]);
             B.launches[g].ntiles[a] = (int)host[g].tjob[a].size();
         }
     b->bands.emplace(n_substeps, std::move(B));
