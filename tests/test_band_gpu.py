@@ -466,3 +466,32 @@ def test_batch_of_many_fields(gpu):
     assert not worlds[1].download(3).any()
     for w in worlds:
         w.close()
+
+
+@pytest.mark.parametrize("what", ["world", "batch"])
+@pytest.mark.parametrize("when", ["before", "after"])
+@pytest.mark.parametrize("grid,sigma", [((90, 44, 31), 1.3), ((176, 160, 96), 0.9)])
+def test_no_memory_for_operators(gpu, monkeypatch, what, when, grid, sigma):
+    """Operators that find no memory (a bound of one byte, before or after the
+    world is created) leave ticks on what the world was created with."""
+    nf = 2
+    params = [vfd.field_params(sigma, 0.02)] * nf
+    us = [vfd.synth_field(5, 0, f, grid[::-1]) for f in range(nf)]
+    if when == "before":
+        monkeypatch.setenv("VFD_BAND_BYTES", "1")
+    with vfd.World(*grid, params) as w:
+        monkeypatch.setenv("VFD_BAND_BYTES", "1")
+        for f, u in enumerate(us):
+            w.upload(f, u)
+        t = vfd.Batch([w]) if what == "batch" else w
+        for n in (4, 1, 4):
+            t.tick(n)
+        got = [w.download(f) for f in range(nf)]
+        mass = w.mass()
+        if what == "batch":
+            t.close()
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    for f, u in enumerate(us):
+        ref = oracle.tick(u, sigma, 0.02, 9, *none)
+        assert rel_l2(got[f], ref) <= 1e-5
+        assert abs(mass[f]["total"] - ref.sum()) <= 1e-5 * ref.sum()

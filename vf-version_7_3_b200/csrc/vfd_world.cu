@@ -459,6 +459,7 @@ struct vfd_world {
     bool band = false;
     bool fft_ready = false;          // the FFT passes' arrays are set up (build_fft)
     int band_mmax = 0;               // most substeps one operator folds (0: not known yet)
+    bool band_full = false;          // no memory for further operators
     std::map<int, BandPlan> band_plans;
 
     std::string err;
@@ -712,6 +713,16 @@ static int band_fold_limit(const vfd_world *w, int mmax)
     return top;
 }
 
+// Most device memory a world's operators take together: what its fields take,
+// or 256 MB where that is more (VFD_BAND_BYTES: another bound).  Eight fields'
+// operators of one number of substeps are 1 to 8 MB; tens of thousands of
+// fields of a few voxels would take gigabytes.
+static size_t band_bytes_limit(const vfd_world *w)
+{
+    const char *e = getenv("VFD_BAND_BYTES");
+    return e ? (size_t)strtoull(e, nullptr, 10) : std::max(sizeof(float) * w->V * w->nf, (size_t)256 << 20);
+}
+
 // Builds the operators of m substeps on the world's own stream, without
 // waiting: passes that use them wait for P.ready (band_plan).
 static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
@@ -821,6 +832,9 @@ static cudaError_t build_band_plan(vfd_world *w, int m, BandPlan &P)
     const size_t o_maps = take(sizeof(CUtensorMap) * P.jobs.size());
     size_t o_tj[3];
     for (int a = 0; a < 3; ++a) o_tj[a] = take(sizeof(int) * P.ntiles[a]);
+    size_t held = off;
+    for (const auto &kv : w->band_plans) held += kv.second.bytes;
+    if (held > band_bytes_limit(w)) return cudaErrorMemoryAllocation;
     cudaError_t e = cudaMalloc(&P.d, off);
     if (e != cudaSuccess) {
         P.d = nullptr;
@@ -955,6 +969,32 @@ static int band_limit(vfd_world *w, int n_substeps)
     if (n_substeps == 1) return 1;
     if (w->band_mmax == 0) w->band_mmax = band_fold_limit(w, BD_MMAX);
     return w->band_mmax;
+}
+
+// The operators of a tick's groups of substeps, in order, for use on `st`;
+// none where the tick runs on the FFT passes.  A tick whose operators find no
+// memory runs on what the world was created with: single-substep operators or
+// the FFT passes.
+static cudaError_t band_tick(vfd_world *w, int n_substeps, cudaStream_t st, std::vector<const BandPlan *> &plans)
+{
+    plans.clear();
+    if (!runs_band(w, n_substeps)) return cudaSuccess;
+    int limit = band_limit(w, n_substeps);
+    for (;;) {
+        cudaError_t e = cudaSuccess;
+        for (int m : band_groups(n_substeps, limit)) {
+            const BandPlan *P = nullptr;
+            e = w->band_full && !w->band_plans.count(m) ? cudaErrorMemoryAllocation : band_plan(w, m, st, &P);
+            if (e != cudaSuccess) break;
+            plans.push_back(P);
+        }
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+        w->band_full = true;
+        plans.clear();
+        if (limit == 1 || !w->band_plans.count(1)) return cudaSuccess;
+        limit = 1;
+    }
 }
 
 // True when the pass stages samples unchanged (no padding-rule transform).
@@ -1337,8 +1377,11 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         w->band = band_enabled() && !(ch && ch->pinned) && band_fold_limit(w, 1) >= 1;
         // what a single substep takes is set up now, the rest where a tick needs it
         const BandPlan *P = nullptr;
-        if (runs_band(w, 1)) e = band_plan(w, 1, w->s_in, &P);
-        else e = build_fft(w);
+        if (runs_band(w, 1) && (e = band_plan(w, 1, w->s_in, &P)) == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            w->band = false;
+        }
+        if (!runs_band(w, 1)) e = build_fft(w);
         if (e != cudaSuccess) return bail(e, "the passes' operators");
     }
     if ((e = cudaStreamCreateWithFlags(&w->s_cmp, cudaStreamNonBlocking)) != cudaSuccess) return bail(e, "stream");
@@ -2059,15 +2102,14 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
         }
         return VFD_OK;
     }
-    const bool band = runs_band(w, n_substeps);
-    if (band) {
-        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps));
+    std::vector<const BandPlan *> plans;
+    VFD_CUDA(w, band_tick(w, n_substeps, st, plans));
+    if (!plans.empty()) {
         double *mass = w->d_mass + (field < 0 ? 0 : (int64_t)field * MS_COUNT);
         const size_t mbytes = sizeof(double) * MS_COUNT * (field < 0 ? w->nf : 1);
-        for (size_t g = 0; g < groups.size(); ++g) {
-            const BandPlan *P = nullptr;
-            VFD_CUDA(w, band_plan(w, groups[g], st, &P));
-            const bool last = g + 1 == groups.size();  // the accounting is the last group's
+        for (size_t g = 0; g < plans.size(); ++g) {
+            const BandPlan *P = plans[g];
+            const bool last = g + 1 == plans.size();  // the accounting is the last group's
             if (last && P->affine)
                 VFD_CUDA(w, cudaMemcpyAsync(mass, P->d_init + (field < 0 ? 0 : (int64_t)field * MS_COUNT), mbytes,
                                             cudaMemcpyDeviceToDevice, st));
@@ -2082,7 +2124,7 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
             }
         }
     }
-    if (!band) {
+    if (plans.empty()) {
         const vfd_status r = enqueue_fft_substeps(w, field, n_substeps, st);
         if (r != VFD_OK) return r;
     }
@@ -2588,6 +2630,7 @@ struct BatchBand {
     unsigned char *d = nullptr;  // arena
     std::vector<Launch> launches;
     std::vector<std::pair<vfd_world *, const double *>> affine;  // accounting starts that are not zero
+    std::vector<vfd_world *> fft_worlds;  // the worlds whose ticks run on FFT passes
 };
 constexpr size_t BATCH_BANDS = 4;  // substep counts whose arrays a batch keeps
 
@@ -2803,14 +2846,6 @@ static cudaError_t take_stream(vfd_batch *b)
     return cudaSuccess;
 }
 
-// The worlds whose ticks of n_substeps run on FFT passes.
-static std::vector<vfd_world *> batch_fft_worlds(const vfd_batch *b, int n_substeps)
-{
-    std::vector<vfd_world *> out;
-    for (auto *w : b->worlds)
-        if (!runs_band(w, n_substeps)) out.push_back(w);
-    return out;
-}
 static vfd_status batch_prepare_fft(vfd_batch *b, BatchFft &F, const std::vector<vfd_world *> &ws);
 
 vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **out)
@@ -2876,7 +2911,10 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
     b->d_mass_counts = reinterpret_cast<int *>(b->d_arena + o_mc);
     b->gens.assign(n_worlds, ~0ull);
     // the FFT passes of single-substep ticks: set up now rather than in the first
-    const vfd_status st = batch_prepare_fft(b, b->fft[0], batch_fft_worlds(b, 1));
+    std::vector<vfd_world *> ws;
+    for (auto *w : b->worlds)
+        if (!runs_band(w, 1)) ws.push_back(w);
+    const vfd_status st = batch_prepare_fft(b, b->fft[0], ws);
     if (st != VFD_OK) {
         const std::string msg = b->err;
         batch_release(b);
@@ -2892,8 +2930,10 @@ vfd_status vfd_batch_create(vfd_world *const *worlds, int n_worlds, vfd_batch **
 // may never need them).
 static vfd_status batch_prepare_fft(vfd_batch *b, BatchFft &F, const std::vector<vfd_world *> &ws)
 {
-    if (F.ready) return VFD_OK;
-    free_batch_fft(b->device, F);  // what an attempt that failed left
+    if (F.ready && F.worlds == ws) return VFD_OK;
+    // other worlds (one found no memory for operators), or what an attempt that failed left
+    if (F.ready) VFD_BCUDA(b, cudaStreamSynchronize(b->st));
+    free_batch_fft(b->device, F);
     F.worlds = ws;
     for (auto *w : ws) F.njobs += w->nf;
     if (F.njobs == 0) {
@@ -3019,19 +3059,18 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     };
     std::vector<Host> host;
     for (auto *w : b->worlds) {
-        if (!runs_band(w, n_substeps)) continue;
-        const std::vector<int> groups = band_groups(n_substeps, band_limit(w, n_substeps));
-        if (host.size() < groups.size()) {
-            host.resize(groups.size());
-            B.launches.resize(groups.size());
+        std::vector<const BandPlan *> plans;
+        const cudaError_t e = band_tick(w, n_substeps, b->st, plans);
+        if (e != cudaSuccess)
+            return bfail(b, VFD_ERR_CUDA, std::string("banded operators: ") + cudaGetErrorString(e));
+        if (plans.empty()) B.fft_worlds.push_back(w);
+        if (host.size() < plans.size()) {
+            host.resize(plans.size());
+            B.launches.resize(plans.size());
         }
-        for (size_t g = 0; g < groups.size(); ++g) {
-            const BandPlan *P = nullptr;
-            const cudaError_t e = band_plan(w, groups[g], b->st, &P);
-            if (e != cudaSuccess)
-                return bfail(b, e == cudaErrorMemoryAllocation ? VFD_ERR_OUT_OF_MEMORY : VFD_ERR_CUDA,
-                             std::string("banded operators: ") + cudaGetErrorString(e));
-            const bool last = g + 1 == groups.size();  // the accounting is the last group's
+        for (size_t g = 0; g < plans.size(); ++g) {
+            const BandPlan *P = plans[g];
+            const bool last = g + 1 == plans.size();  // the accounting is the last group's
             for (int a = 0; a < 3; ++a) {
                 for (int f = 0; f < w->nf; ++f) {
                     BandJob j = P->jobs[(size_t)a * w->nf + f];
@@ -3075,7 +3114,7 @@ static vfd_status batch_prepare(vfd_batch *b, int n_substeps, cudaStream_t strea
 {
     CaptureRelaxed scope;
     vfd_status st = batch_prepare_band(b, n_substeps);
-    if (st == VFD_OK) st = batch_prepare_fft(b, b->fft[n_substeps > 1], batch_fft_worlds(b, n_substeps));
+    if (st == VFD_OK) st = batch_prepare_fft(b, b->fft[n_substeps > 1], b->bands.at(n_substeps).fft_worlds);
     if (st == VFD_OK && stream_capturing(stream)) VFD_BCUDA(b, cudaStreamSynchronize(b->st));
     return st;
 }
