@@ -1361,7 +1361,13 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
         w->k0.assign(w->nf, 1.0f);
         const int64_t nc = (w->method == VFD_METHOD_PLAIN) ? nk : (int64_t)w->Fxs * w->F[1] * w->nz;
         if (w->method == VFD_METHOD_FFT3D) w->gen_group = general_group(w);
-        if ((e = cudaMalloc(&w->d_C, sizeof(float2) * nc * w->gen_group)) != cudaSuccess) return bail(e, "cudaMalloc spectrum scratch");
+        e = cudaMalloc(&w->d_C, sizeof(float2) * nc * w->gen_group);
+        if (e == cudaErrorMemoryAllocation && w->gen_group > 1) {
+            cudaGetLastError();
+            w->gen_group = 1;  // one field a launch needs no more than one field's
+            e = cudaMalloc(&w->d_C, sizeof(float2) * nc);
+        }
+        if (e != cudaSuccess) return bail(e, "cudaMalloc spectrum scratch");
         if (w->method == VFD_METHOD_PLAIN) {
             if ((e = cudaMalloc(&w->d_P, sizeof(float) * (int64_t)w->F[0] * w->F[1] * w->F[2])) != cudaSuccess)
                 return bail(e, "cudaMalloc padded grid");
