@@ -495,3 +495,27 @@ def test_no_memory_for_operators(gpu, monkeypatch, what, when, grid, sigma):
         ref = oracle.tick(u, sigma, 0.02, 9, *none)
         assert rel_l2(got[f], ref) <= 1e-5
         assert abs(mass[f]["total"] - ref.sum()) <= 1e-5 * ref.sum()
+
+
+def test_device_memory_is_accounted(gpu):
+    """vfd_world_device_bytes tells what a world's passes hold by then, and a
+    server counts the operators of its ticks' substeps against its budget."""
+    grid, params, nf = (176, 160, 96), [vfd.field_params(0.9, 0.02)] * 4, 4
+    fields = 4 * nf * int(np.prod(grid))
+    with vfd.World(*grid, params) as w:  # FFT passes: jobs, tiles, tensor maps
+        fft = w.device_bytes() - fields
+        w.tick(10)
+        both = w.device_bytes() - fields
+    small = (64, 64, 32)
+    with vfd.World(*small, params) as w:  # banded products alone
+        one = w.device_bytes() - 4 * nf * int(np.prod(small))
+        w.tick(10)
+        ten = w.device_bytes()
+    # an axis' operator holds at least one image of 5 (one substep of radius 3) or
+    # 8 (ten) k-steps of 6 KB, the tiles of the FFT passes 16 bytes each
+    assert one >= 3 * nf * 5 * 6144 and both - fft >= 3 * nf * 8 * 6144
+    assert fft >= sum(16 * nf * (np.prod(grid) // n // 32) for n in grid) // 4
+    with vfd.Server(8 << 30, max_active=2, substeps_per_tick=10) as s:
+        rid = s.submit(small, params, 3, synth=(7, 0, 0.0, 1e-3))
+        assert s.wait(rid)["status"] == 0
+        assert s.stats()["hbm_peak"] >= ten

@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -37,6 +38,7 @@
 #include <vector>
 
 #include "vfd.h"
+#include "vfd_band.h"
 #include "vfd_internal.h"
 
 namespace {
@@ -126,11 +128,19 @@ struct vfd_server {
 
 namespace {
 
-size_t estimate_bytes(const Request &r)
+size_t estimate_bytes(const Request &r, int substeps)
 {
-    // fields + per-axis tables (generous) + banded operators + sources
+    // fields + per-axis tables (generous) + banded operators (up to four images
+    // an axis, of 64 outputs by the folded kernel's width, and vectors) + sources
     size_t b = sizeof(float) * (size_t)r.nx * r.ny * r.nz * r.nf;
-    for (int n : {r.nx, r.ny, r.nz}) b += (size_t)r.nf * 32 * 1024 * std::min((n + 63) / 64, 4);
+    for (int a = 0; a < 3; ++a) {
+        const int n = a == 0 ? r.nx : a == 1 ? r.ny : r.nz;
+        for (const auto &p : r.params) {
+            const double radius = p.radius[a] > 0 ? p.radius[a] : std::ceil(3.0 * p.sigma[a]);
+            const size_t half = (size_t)std::min(radius * substeps + 4.0, (double)vfd::BD_HMAX);
+            b += std::min((n + 63) / 64, 4) * (vfd::BD_STEP_BYTES * ((64 + 2 * half + 15) / 16)) + 32 * (size_t)n + 4096;
+        }
+    }
     b += (size_t)r.nf * 3 * 4096 * sizeof(float) + 3 * 4096 * 8 + 64 * 1024;
     for (const auto &v : r.src_idx) b += v.size() * 8;
     return b;
@@ -328,7 +338,7 @@ std::vector<std::shared_ptr<Request>> select_admissions(vfd_server *s, int occup
     size_t used = s->in_use;
     while (!s->pending.empty() && slots > 0) {
         auto r = s->pending.front();
-        const size_t est = estimate_bytes(*r);
+        const size_t est = estimate_bytes(*r, s->substeps);
         if (est > s->budget) {
             s->pending.pop_front();
             s->st.queued = (int64_t)s->pending.size();
@@ -346,7 +356,7 @@ std::vector<std::shared_ptr<Request>> select_admissions(vfd_server *s, int occup
             lk.lock();
             taken.clear();
             used = s->in_use;
-            for (auto &q : out) used += estimate_bytes(*q);
+            for (auto &q : out) used += estimate_bytes(*q, s->substeps);
             if (used + est > s->budget) break;
         }
         if (pooled) taken[key]++;
@@ -483,6 +493,13 @@ void scheduler(vfd_server *s)
             s->batch = nullptr;
             s->set_changed = true;
             continue;
+        }
+        // a world's first tick sets up what its passes need
+        for (auto &r : s->active) {
+            size_t bytes = r->bytes;
+            if (vfd_world_device_bytes(r->world, &bytes) != VFD_OK) continue;
+            s->in_use += bytes - r->bytes;
+            r->bytes = bytes;
         }
         std::vector<std::shared_ptr<Request>> survivors;
         for (auto &r : s->active) {

@@ -305,7 +305,7 @@ static void rf_group_host(const OsJob *jobs, int n, RfGroupHost &h)
 }
 
 // rf_group_host, uploaded to arrays of its own.
-static cudaError_t build_rf_groups(const OsJob *jobs, int n, std::vector<RfGroup> &out)
+static cudaError_t build_rf_groups(const OsJob *jobs, int n, std::vector<RfGroup> &out, size_t *bytes = nullptr)
 {
     RfGroupHost h;
     rf_group_host(jobs, n, h);
@@ -328,6 +328,7 @@ static cudaError_t build_rf_groups(const OsJob *jobs, int n, std::vector<RfGroup
         return e;
     }
     out.push_back(g);
+    if (bytes) *bytes += sizeof(OsTileInfo) * t.size() + sizeof(CUtensorMap) * maps.size();
     return cudaSuccess;
 }
 
@@ -458,6 +459,7 @@ struct vfd_world {
     // pinned tuning or a kernel too wide for them keeps it on the FFT passes
     bool band = false;
     bool fft_ready = false;          // the FFT passes' arrays are set up (build_fft)
+    size_t fft_bytes = 0;            // what they (and the general methods' tables) take on the device
     int band_mmax = 0;               // most substeps one operator folds (0: not known yet)
     bool band_full = false;          // no memory for further operators
     std::map<int, BandPlan> band_plans;
@@ -1015,6 +1017,7 @@ static cudaError_t build_axis_tables(vfd_world *w)
         if ((e = cudaMalloc(&w->d_tw[a], sizeof(float2) * w->F[a])) != cudaSuccess) return e;
         if ((e = cudaMemcpy(w->d_tw[a], tw.data(), sizeof(float2) * w->F[a], cudaMemcpyHostToDevice)) != cudaSuccess)
             return e;
+        w->fft_bytes += sizeof(float2) * w->F[a];
     }
     {
         std::vector<float> spec((size_t)w->nf * 3 * w->Fmax, 0.0f), tmp;
@@ -1026,6 +1029,7 @@ static cudaError_t build_axis_tables(vfd_world *w)
         if ((e = cudaMalloc(&w->d_spec, sizeof(float) * spec.size())) != cudaSuccess) return e;
         if ((e = cudaMemcpy(w->d_spec, spec.data(), sizeof(float) * spec.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return e;
+        w->fft_bytes += sizeof(float) * spec.size();
     }
     return cudaSuccess;
 }
@@ -1052,6 +1056,7 @@ static cudaError_t build_fft(vfd_world *w)
         if ((e = cudaMalloc(&w->d_jobs, sizeof(AxisJob) * jobs.size())) != cudaSuccess) return e;
         if ((e = cudaMemcpy(w->d_jobs, jobs.data(), sizeof(AxisJob) * jobs.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return e;
+        w->fft_bytes += sizeof(AxisJob) * jobs.size();
     }
     if (w->use_os[0] || w->use_os[1] || w->use_os[2]) {
         std::vector<OsJob> oj;
@@ -1071,6 +1076,7 @@ static cudaError_t build_fft(vfd_world *w)
         if ((e = cudaMalloc(&w->d_osjobs, sizeof(OsJob) * oj.size())) != cudaSuccess) return e;
         if ((e = cudaMemcpy(w->d_osjobs, oj.data(), sizeof(OsJob) * oj.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
             return e;
+        w->fft_bytes += sizeof(OsJob) * oj.size();
         for (int a = 0; a < 3; ++a) {
             std::vector<OsTileInfo> all, one;
             for (int f = 0; f < w->nf; ++f) {
@@ -1080,14 +1086,15 @@ static cudaError_t build_fft(vfd_world *w)
             if ((e = upload_vec(&w->d_os_tiles[a], all)) != cudaSuccess ||
                 (e = upload_vec(&w->d_os_ftiles[a], one)) != cudaSuccess)
                 return e;
+            w->fft_bytes += sizeof(OsTileInfo) * (all.size() + one.size());
         }
         for (int a = 0; a < 3; ++a) {
             if (!w->use_rf[a]) continue;
             if ((e = rf_prepare()) != cudaSuccess) return e;
-            if ((e = build_rf_groups(&oj[(size_t)a * w->nf], w->nf, w->rf[a])) != cudaSuccess) return e;
+            if ((e = build_rf_groups(&oj[(size_t)a * w->nf], w->nf, w->rf[a], &w->fft_bytes)) != cudaSuccess) return e;
             w->rf_field[a].resize(w->nf);
             for (int f = 0; f < w->nf; ++f)
-                if ((e = build_rf_groups(&oj[(size_t)(3 + a) * w->nf + f], 1, w->rf_field[a][f])) != cudaSuccess)
+                if ((e = build_rf_groups(&oj[(size_t)(3 + a) * w->nf + f], 1, w->rf_field[a][f], &w->fft_bytes)) != cudaSuccess)
                     return e;
         }
     }
@@ -1428,10 +1435,8 @@ vfd_status vfd_world_fft_dims(const vfd_world *w, int *fft3)
 vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes)
 {
     if (!w || !bytes) return VFD_ERR_INVALID_ARG;
-    size_t b = sizeof(float) * (size_t)w->V * w->nf;
-    for (int a = 0; a < 3; ++a) b += sizeof(float2) * w->F[a];
-    b += sizeof(float) * (size_t)w->nf * 3 * w->Fmax + sizeof(double) * MS_COUNT * w->nf;
-    b += sizeof(AxisJob) * 6 * w->nf + sizeof(DepositJob) * 2 * w->nf;
+    size_t b = sizeof(float) * (size_t)w->V * w->nf * (w->d_upd ? 2 : 1);
+    b += w->fft_bytes + sizeof(double) * MS_COUNT * w->nf + 2 * sizeof(int) + sizeof(DepositJob) * 2 * w->nf;
     b += (sizeof(int32_t) + sizeof(float)) * (size_t)w->src_cap;
     for (const auto &kv : w->band_plans) b += kv.second.bytes;
     if (w->method != VFD_METHOD_SEPARABLE) {
