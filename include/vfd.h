@@ -135,7 +135,8 @@ vfd_status vfd_world_device_bytes(const vfd_world *w, size_t *bytes);
  * are the faster form (kernels up to 56 voxels of half-width after folding; a
  * single substep of narrow kernels on large fields stays on the FFT passes),
  * unless vfd_autotune_set pinned their FFT passes.  What follows chooses
- * among the FFT passes.
+ * among the FFT passes, and (vfd_autotune, vfd_batch_autotune) between them
+ * and the banded products for single substeps.
  * Per axis, the FFT pass: the register FFT (kernel radius <= 8),
  * overlap-save FFT-64 blocks (radius <= 16) at 3 or 4 resident CTAs per SM,
  * or a full-line FFT with a chosen padded length (the three cheapest
@@ -160,7 +161,9 @@ typedef struct vfd_axis_tuning {
 /* Times every candidate of each axis on temporary worlds of desc's shape
  * (zero fields, `reps` timed launches each after one warm-up; the device
  * needs room for one extra world), caches the fastest per shape (device,
- * grid, padding rule, per-field radii) and writes it to out[3].  Later
+ * grid, padding rule, per-field radii) and writes it to out[3].  Single
+ * substeps of the shape then run on these passes or on the banded products,
+ * which are timed too, whichever was faster.  Later
  * vfd_world_create calls with that shape use the cached choice; with the
  * environment variable VFD_AUTOTUNE=1 they tune an uncached shape first. */
 vfd_status vfd_autotune(const vfd_world_desc *desc, int device, int reps, vfd_axis_tuning *out3);
@@ -168,8 +171,8 @@ vfd_status vfd_autotune(const vfd_world_desc *desc, int device, int reps, vfd_ax
  * world was not created from a tuned choice). */
 vfd_status vfd_world_tuning(const vfd_world *w, vfd_axis_tuning *out3);
 /* Stores a choice for desc's shape in the cache (a saved tuning, or a pinned
- * pass): later worlds of the shape run it, and no banded products.  An axis whose world cannot run
- * the stored method (register FFT beyond radius 8 or on an unaligned x
+ * pass): later worlds of the shape run it, and no banded products.  An axis
+ * whose world cannot run the stored method (register FFT beyond radius 8 or on an unaligned x
  * line, overlap-save beyond radius 16) falls back to the default pass. */
 vfd_status vfd_autotune_set(const vfd_world_desc *desc, int device, const vfd_axis_tuning *in3);
 /* Empties the per-shape cache. */
@@ -311,6 +314,8 @@ vfd_status vfd_batch_tick(vfd_batch *b, int n_substeps, void *stream);
  * (register FFT, overlap-save at 3 and at 4 resident CTAs per SM, full-line
  * FFT) over all the batch's fields -- one warm-up and `reps` timed launches
  * each, CUDA events -- and keeps the fastest per axis (out3, may be NULL).
+ * Single-substep ticks then take the fastest of: these passes for every
+ * world, banded products for every world, each world's own choice.
  * The passes run on the worlds' own fields, which are saved to temporary
  * device buffers and restored.  The next tick re-captures the graph. */
 vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3);

@@ -154,3 +154,33 @@ def test_batch_of_pinned_worlds_matches_single_worlds(gpu, clean_cache):
             assert rel_l2(got, oracle.tick(u, SIGMAS[f], DECAY[f], 2, idx, amt)) <= REL_L2
     for w in worlds + singles:
         w.close()
+
+
+@pytest.mark.parametrize("grid", [GRID, (176, 160, 96)])
+def test_tuned_single_substeps(gpu, clean_cache, grid):
+    """Single substeps of tuned worlds and batches run on the form that was
+    timed to be faster (FFT passes or banded products), set up at creation;
+    ticks of several substeps as untuned ones."""
+    vfd.autotune(*grid, params(), reps=2)
+    none = (np.zeros(0, np.int32), np.zeros(0, np.float32))
+    us = [vfd.synth_field(5, 0, f, grid[::-1]) for f in range(len(SIGMAS))]
+    refs = [oracle.tick(oracle.tick(u, SIGMAS[f], DECAY[f], 1, *none).astype(np.float32), SIGMAS[f], DECAY[f], 4, *none)
+            for f, u in enumerate(us)]
+    worlds = [vfd.World(*grid, params()) for _ in range(3)]
+    for w in worlds:
+        for f, u in enumerate(us):
+            w.upload(f, u)
+    held = worlds[0].device_bytes()
+    worlds[0].tick(1)
+    assert worlds[0].device_bytes() == held
+    worlds[0].tick(4)
+    with vfd.Batch(worlds[1:]) as b:
+        b.autotune(reps=2)
+        for f, u in enumerate(us):
+            np.testing.assert_array_equal(worlds[1].download(f), u)
+        b.tick(1)
+        b.tick(4)
+    for w in worlds:
+        for f, ref in enumerate(refs):
+            assert rel_l2(w.download(f), ref) <= REL_L2
+        w.close()

@@ -462,6 +462,7 @@ struct vfd_world {
     size_t fft_bytes = 0;            // what they (and the general methods' tables) take on the device
     int band_mmax = 0;               // most substeps one operator folds (0: not known yet)
     bool band_full = false;          // no memory for further operators
+    int single_band = -1;            // single substeps on them: 1 yes, 0 no (tuned), -1 by the rule of runs_band
     std::map<int, BandPlan> band_plans;
 
     std::string err;
@@ -955,9 +956,12 @@ static std::vector<int> band_groups(int n_substeps, int limit)
 // 304, 512x256x256 1236 / 1168; mean radius 5.1: 512x256x384 2094 / 2067; mean
 // radius 6.5: 35 / 46, 53 / 68, 96 / 116, 307 / 378, 1226 / 1318.
 constexpr int64_t BAND_SMALL = (int64_t)4 << 20;  // voxels x fields
-static bool runs_band(const vfd_world *w, int n_substeps)
+// single: what was timed for the batch the tick is of (-1: nothing).
+static bool runs_band(const vfd_world *w, int n_substeps, int single = -1)
 {
     if (!w->band) return false;
+    if (single < 0) single = w->single_band;
+    if (n_substeps == 1 && single >= 0) return single == 1;
     if (n_substeps > 1 || !(w->use_rf[0] && w->use_rf[1] && w->use_rf[2]) || w->V * w->nf <= BAND_SMALL) return true;
     int radii = 0;
     for (int f = 0; f < w->nf; ++f)
@@ -977,10 +981,11 @@ static int band_limit(vfd_world *w, int n_substeps)
 // none where the tick runs on the FFT passes.  A tick whose operators find no
 // memory runs on what the world was created with: single-substep operators or
 // the FFT passes.
-static cudaError_t band_tick(vfd_world *w, int n_substeps, cudaStream_t st, std::vector<const BandPlan *> &plans)
+static cudaError_t band_tick(vfd_world *w, int n_substeps, cudaStream_t st, std::vector<const BandPlan *> &plans,
+                             int single = -1)
 {
     plans.clear();
-    if (!runs_band(w, n_substeps)) return cudaSuccess;
+    if (!runs_band(w, n_substeps, single)) return cudaSuccess;
     int limit = band_limit(w, n_substeps);
     for (;;) {
         cudaError_t e = cudaSuccess;
@@ -1158,6 +1163,7 @@ struct AxisChoice {
 struct ShapeChoice {
     AxisChoice ax[3];
     bool pinned = false;  // the FFT passes of ax run whatever else would (vfd_autotune_set, timing)
+    int single = -1;      // single substeps on banded products (vfd_world::single_band)
 };
 
 static std::mutex g_tune_mu;
@@ -1324,6 +1330,7 @@ static vfd_status world_create(const vfd_world_desc *d, int device, const ShapeC
             w->os_minb[a] = ch->ax[a].minb;
             w->tuned_ms[a] = ch->ax[a].ms;
         }
+    if (ch) w->single_band = ch->single;
     if (general) {
         w->Fxh = w->F[0] / 2 + 1;
         w->Fxs = spectrum_stride(w->method, w->Fxh);
@@ -2065,6 +2072,20 @@ static vfd_status enqueue_fft_substeps(vfd_world *w, int field, int n_substeps, 
     return VFD_OK;
 }
 
+// The banded passes of one group of substeps, of all fields (field < 0) or of one.
+static cudaError_t enqueue_band(vfd_world *w, const BandPlan *P, int field, bool sums, cudaStream_t st)
+{
+    for (int a = 0; a < 3; ++a) {
+        LaunchTimer lt(w, a, st);
+        const BandJob *J = field < 0 ? nullptr : &P->jobs[(size_t)a * w->nf + field];
+        const cudaError_t e = launch_band(P->d_jobs[a], P->d_tjob[a], J ? J->tile0 : 0, J ? J->ntiles : P->ntiles[a], a,
+                                          P->geo[a], sums, st);
+        if (e != cudaSuccess) return e;
+        lt.done();
+    }
+    return cudaSuccess;
+}
+
 // Whether an update of field f may run in one launch with one of field g: an
 // update reads and zeroes its dChem, so neither field's dChem may be the
 // other's, nor the other's values.  (Fields of separate launches run in
@@ -2126,13 +2147,7 @@ static vfd_status enqueue_tick(vfd_world *w, int field, int n_substeps, cudaStre
                                             cudaMemcpyDeviceToDevice, st));
             else if (last)
                 VFD_CUDA(w, cudaMemsetAsync(mass, 0, mbytes, st));
-            for (int a = 0; a < 3; ++a) {
-                LaunchTimer lt(w, a, st);
-                const BandJob *J = field < 0 ? nullptr : &P->jobs[(size_t)a * w->nf + field];
-                VFD_CUDA(w, launch_band(P->d_jobs[a], P->d_tjob[a], J ? J->tile0 : 0, J ? J->ntiles : P->ntiles[a], a,
-                                        P->geo[a], last, st));
-                lt.done();
-            }
+            VFD_CUDA(w, enqueue_band(w, P, field, last, st));
         }
     }
     if (plans.empty()) {
@@ -2331,6 +2346,33 @@ static vfd_status tune_candidate(TuneRun &T, ShapeChoice proto, const bool *axes
     return s;
 }
 
+// Times the banded products on a single substep against the best FFT passes.
+static vfd_status tune_single(TuneRun &T)
+{
+    ShapeChoice c;
+    c.single = 1;
+    vfd_world *w = nullptr;
+    const vfd_status s = world_create(T.d, T.device, &c, &w);
+    if (s != VFD_OK) return s == VFD_ERR_OUT_OF_MEMORY ? VFD_OK : s;
+    std::vector<const BandPlan *> plans;
+    float ms = 0.0f;
+    cudaError_t e = band_tick(w, 1, T.st, plans);
+    if (e == cudaSuccess && !plans.empty()) {
+        for (int i = -1; i < T.reps && e == cudaSuccess; ++i) {
+            if (i == 0) e = cudaEventRecord(T.e0, T.st);
+            if (e == cudaSuccess) e = enqueue_band(w, plans[0], -1, true, T.st);
+        }
+        if (e == cudaSuccess) e = cudaEventRecord(T.e1, T.st);
+        if (e == cudaSuccess) e = cudaEventSynchronize(T.e1);
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, T.e0, T.e1);
+        float fft = 0.0f;
+        for (int a = 0; a < 3; ++a) fft += T.best.ax[a].ms;
+        T.best.single = ms / T.reps < fft ? 1 : 0;
+    }
+    vfd_world_destroy(w);
+    return e == cudaSuccess ? VFD_OK : fail(nullptr, VFD_ERR_CUDA, std::string("autotune: ") + cudaGetErrorString(e));
+}
+
 static vfd_status tune_shape(const vfd_world_desc *d, int device, int reps, ShapeChoice *out)
 {
     if (!d || !d->fields || d->n_fields < 1 || d->nx < 1 || d->ny < 1 || d->nz < 1)
@@ -2398,6 +2440,7 @@ static vfd_status tune_shape(const vfd_world_desc *d, int device, int reps, Shap
                 }
                 if (any) s = tune_candidate(T, c, axes);
             }
+    if (s == VFD_OK && T.have[0] && T.have[1] && T.have[2]) s = tune_single(T);
     cudaEventDestroy(T.e0);
     cudaEventDestroy(T.e1);
     cudaStreamDestroy(T.st);
@@ -2672,6 +2715,7 @@ struct BatchFft {
 struct vfd_batch {
     std::map<int, BatchBand> bands;                   // by a tick's substeps
     BatchFft fft[2];                                  // of a tick of one substep / of several
+    int single = -1;                                  // tuned: single substeps on banded products (runs_band)
     int tuned_method[3] = {PASS_METHOD_AUTO, PASS_METHOD_AUTO, PASS_METHOD_AUTO};
     int device = 0;
     std::vector<vfd_world *> worlds;
@@ -3071,7 +3115,7 @@ static vfd_status batch_prepare_band(vfd_batch *b, int n_substeps)
     std::vector<Host> host;
     for (auto *w : b->worlds) {
         std::vector<const BandPlan *> plans;
-        const cudaError_t e = band_tick(w, n_substeps, b->st, plans);
+        const cudaError_t e = band_tick(w, n_substeps, b->st, plans, b->single);
         if (e != cudaSuccess)
             return bfail(b, VFD_ERR_CUDA, std::string("banded operators: ") + cudaGetErrorString(e));
         if (plans.empty()) B.fft_worlds.push_back(w);
@@ -3128,6 +3172,76 @@ static vfd_status batch_prepare(vfd_batch *b, int n_substeps, cudaStream_t strea
     if (st == VFD_OK) st = batch_prepare_fft(b, b->fft[n_substeps > 1], b->bands.at(n_substeps).fft_worlds);
     if (st == VFD_OK && stream_capturing(stream)) VFD_BCUDA(b, cudaStreamSynchronize(b->st));
     return st;
+}
+
+// The passes of a tick, without the deposit.
+static vfd_status batch_passes(vfd_batch *b, int n_substeps)
+{
+    VFD_BCUDA(b, launch_zero_blocks(b->d_mass_ptrs, b->d_mass_counts, (int)b->worlds.size(), b->st));
+    const BatchBand &B = b->bands.at(n_substeps);
+    const BatchFft &F = b->fft[n_substeps > 1];
+    for (const auto &x : B.affine)
+        VFD_BCUDA(b, cudaMemcpyAsync(x.first->d_mass, x.second, sizeof(double) * MS_COUNT * x.first->nf,
+                                     cudaMemcpyDeviceToDevice, b->st));
+    for (const auto &L : B.launches)
+        for (int a = 0; a < 3; ++a)
+            VFD_BCUDA(b, launch_band(L.d_jobs[a], L.d_tjob[a], 0, L.ntiles[a], a, L.geo[a], true, b->st));
+    for (size_t i = 0; F.each && i < F.worlds.size(); ++i) {
+        const vfd_status st = enqueue_fft_substeps(F.worlds[i], -1, n_substeps, b->st);
+        if (st != VFD_OK) return bfail(b, st, F.worlds[i]->err);
+    }
+    for (int s = 0; s < n_substeps && F.njobs > 0 && !F.each; ++s) {
+        if (s > 0)
+            VFD_BCUDA(b, launch_zero_blocks(F.d_mass_ptrs, F.d_mass_counts, (int)F.worlds.size(),
+                                            b->st));
+        for (int a = 0; a < 3; ++a) {
+            if (F.use_rf[a])
+                VFD_BCUDA(b, launch_rf_groups(F.d_osjobs + a * F.njobs, F.rf[a], a, b->st));
+            else if (F.use_os[a])
+                VFD_BCUDA(b, launch_os(F.d_osjobs + a * F.njobs, F.d_os_tiles[a], F.os_tiles[a], b->rmin[a], a,
+                                       b->st, b->os_minb[a]));
+            else
+                VFD_BCUDA(b, launch_axis(b->variant[a], F.d_jobs + a * F.njobs, F.njobs, F.tiles[a],
+                                         b->Fmax[a], b->st));
+        }
+    }
+    return VFD_OK;
+}
+
+// Drops what ticks' passes have been set up with (the stream is idle).
+static void batch_reset(vfd_batch *b)
+{
+    for (auto &F : b->fft) free_batch_fft(b->device, F);
+    for (auto &kv : b->bands) give_arena(b->device, kv.second.d);
+    b->bands.clear();
+}
+
+// Times a single-substep tick's passes with its worlds' own choice between
+// banded products and the (tuned) FFT passes, and with either for all that can.
+static vfd_status batch_tune_single(vfd_batch *b, int reps, cudaEvent_t e0, cudaEvent_t e1)
+{
+    float best = 0.0f;
+    int choice = -1;
+    for (int c = -1; c <= 1; ++c) {
+        b->single = c;
+        batch_reset(b);
+        vfd_status st = batch_prepare(b, 1, b->st);
+        for (int i = -1; i < reps && st == VFD_OK; ++i) {
+            if (i == 0) VFD_BCUDA(b, cudaEventRecord(e0, b->st));
+            st = batch_passes(b, 1);
+        }
+        if (st != VFD_OK) return st;
+        float ms = 0.0f;
+        VFD_BCUDA(b, cudaEventRecord(e1, b->st));
+        VFD_BCUDA(b, cudaEventSynchronize(e1));
+        VFD_BCUDA(b, cudaEventElapsedTime(&ms, e0, e1));
+        if (best == 0.0f || ms < best) {
+            best = ms;
+            choice = c;
+        }
+    }
+    b->single = choice;
+    return VFD_OK;
 }
 
 // Times one axis pass of the whole batch as configured now (one warm-up,
@@ -3247,11 +3361,13 @@ vfd_status vfd_batch_autotune(vfd_batch *b, int reps, vfd_axis_tuning *out3)
             out3[a].ms = best;
         }
     }
+    free_batch_fft(b->device, F);
+    if (st == VFD_OK) st = batch_tune_single(b, reps, e0, e1);
+    if (st != VFD_OK) b->single = -1;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     restore(true);
-    free_batch_fft(b->device, F);
-    for (auto &G : b->fft) free_batch_fft(b->device, G);  // set up anew with the chosen passes
+    batch_reset(b);  // set up anew with the chosen passes
     // the next tick runs directly and re-captures its graph with the chosen passes
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -3272,34 +3388,8 @@ vfd_status vfd_batch_destroy(vfd_batch *b)
 
 static vfd_status batch_enqueue(vfd_batch *b, int n_substeps)
 {
-    VFD_BCUDA(b, launch_zero_blocks(b->d_mass_ptrs, b->d_mass_counts, (int)b->worlds.size(), b->st));
-    const BatchBand &B = b->bands.at(n_substeps);
-    const BatchFft &F = b->fft[n_substeps > 1];
-    for (const auto &x : B.affine)
-        VFD_BCUDA(b, cudaMemcpyAsync(x.first->d_mass, x.second, sizeof(double) * MS_COUNT * x.first->nf,
-                                     cudaMemcpyDeviceToDevice, b->st));
-    for (const auto &L : B.launches)
-        for (int a = 0; a < 3; ++a)
-            VFD_BCUDA(b, launch_band(L.d_jobs[a], L.d_tjob[a], 0, L.ntiles[a], a, L.geo[a], true, b->st));
-    for (size_t i = 0; F.each && i < F.worlds.size(); ++i) {
-        const vfd_status st = enqueue_fft_substeps(F.worlds[i], -1, n_substeps, b->st);
-        if (st != VFD_OK) return bfail(b, st, F.worlds[i]->err);
-    }
-    for (int s = 0; s < n_substeps && F.njobs > 0 && !F.each; ++s) {
-        if (s > 0)
-            VFD_BCUDA(b, launch_zero_blocks(F.d_mass_ptrs, F.d_mass_counts, (int)F.worlds.size(),
-                                            b->st));
-        for (int a = 0; a < 3; ++a) {
-            if (F.use_rf[a])
-                VFD_BCUDA(b, launch_rf_groups(F.d_osjobs + a * F.njobs, F.rf[a], a, b->st));
-            else if (F.use_os[a])
-                VFD_BCUDA(b, launch_os(F.d_osjobs + a * F.njobs, F.d_os_tiles[a], F.os_tiles[a], b->rmin[a], a,
-                                       b->st, b->os_minb[a]));
-            else
-                VFD_BCUDA(b, launch_axis(b->variant[a], F.d_jobs + a * F.njobs, F.njobs, F.tiles[a],
-                                         b->Fmax[a], b->st));
-        }
-    }
+    const vfd_status st = batch_passes(b, n_substeps);
+    if (st != VFD_OK) return st;
     for (auto *w : b->worlds)
         if (w->dep_njobs > 0)
             VFD_BCUDA(b, launch_deposit(w->d_dep, w->dep_njobs, w->d_src_idx, w->d_src_amt, w->src_total,
