@@ -508,11 +508,13 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
             tc_fence_after();
             // the block's offset: the mean of its positions that count (those in
             // the line and inside the padding box; the others have weight 0)
+            __syncwarp();
             asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quad) : "memory");
             const int count = min(BD_BLK * (k + 1) - H, hi) - max(BD_BLK * k - H, lo);
             float off = count > 0 ? __fdividef(vs + S.half[done & 1][half ^ 1][ln], (float)count) : 0.0f;
             if (!(fabsf(off) < 1e30f)) off = 0.0f;
             if (half == 0) S.off[done % BD_OFFS][ln] = off;
+            __syncwarp();
             const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(slot * BD_PART_COLS + half * 16);
             const float2 noff = make_float2(-off, -off), neg = make_float2(-1.0f, -1.0f);
             uint32_t w[16];
