@@ -519,3 +519,14 @@ def test_device_memory_is_accounted(gpu):
         rid = s.submit(small, params, 3, synth=(7, 0, 0.0, 1e-3))
         assert s.wait(rid)["status"] == 0
         assert s.stats()["hbm_peak"] >= ten
+
+
+@pytest.mark.parametrize("scale", [1e-33, 1e-20, 1.0, 1e20, 1e36])
+@pytest.mark.parametrize("substeps", [1, 6])
+def test_scales(gpu, scale, substeps):
+    """Positive fields over FP32's range (from 2^-110 on, where the third part
+    of a value underflows, to where a block's sum overflows)."""
+    grid = (140, 33, 41)
+    u = ((0.2 + np.random.default_rng(3).random(grid[::-1])) * scale).astype(np.float32)
+    out, ref, mass = run_once(grid, u, 1.4, substeps)
+    assert rel_l2(out / scale, ref / scale) <= PER_GROUP

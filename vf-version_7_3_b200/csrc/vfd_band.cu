@@ -22,7 +22,8 @@
 // sigma 2.6), a plume residues over all of its lines.  Relative L2 against
 // FP64, one substep of positive values: 1.1e-7 without offsets, 3.7e-8 with
 // them, the FFT passes 1e-7; ten substeps, sigma 2.6: 3.6e-8 and 1.2e-6; the
-// voxel of 1: 9.7e-8 and 1.3e-6.
+// voxel of 1: 9.7e-8 and 1.3e-6.  The third part of a value below 2^-110 (8e-34)
+// underflows: such values are rounded to 2^-133 (1e-40) instead of 2^-149.
 //
 // In place: outputs of block b are stored once its product is complete; all
 // input blocks that hold those positions are in tensor memory by then, and
@@ -512,7 +513,7 @@ __device__ __forceinline__ void band_convert(const BandTiles &T, int sums, int n
             asm volatile("bar.sync %0, 64;\n" ::"r"(1 + quad) : "memory");
             const int count = min(BD_BLK * (k + 1) - H, hi) - max(BD_BLK * k - H, lo);
             float off = count > 0 ? __fdividef(vs + S.half[done & 1][half ^ 1][ln], (float)count) : 0.0f;
-            if (!(fabsf(off) < 1e30f)) off = 0.0f;
+            if (!(fabsf(off) < 1e37f)) off = 0.0f;
             if (half == 0) S.off[done % BD_OFFS][ln] = off;
             __syncwarp();
             const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(slot * BD_PART_COLS + half * 16);
@@ -639,7 +640,7 @@ __device__ __forceinline__ void band_issuer(const BandTiles &T, int par, int slo
             // the latter's sums is truncated once a k-step.  A product takes 45
             // cycles; this loop issues one in 58, a loop of one in 90, and
             // unrolled over the k-steps the code outgrows the instruction cache
-            // (130): hence two issuing threads.
+            // (130): hence two issuing threads (one product in 48 cycles together).
             uint32_t col = col0;
             uint64_t desc = desc0;
 #pragma unroll 1
@@ -966,7 +967,7 @@ __global__ void band_wait_probe_kernel(long long limit, int *gave_up)
 // ---------------------------------------------------------------------------
 // Set-up of the operators.
 // ---------------------------------------------------------------------------
-constexpr int BD_ROWHW = 160;  // half-width a row of B^m is computed with (its tails beyond H are negligible)
+constexpr int BD_ROWHW = 160;  // half-width a row of B^m is computed with (what lies beyond is far below 1e-8)
 
 // One warp per row of an image: row i of B^m = (A M)^m in FP64, A the cropped
 // convolution, M the interior mask, then its three bf16 parts.

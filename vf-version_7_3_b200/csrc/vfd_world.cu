@@ -686,7 +686,8 @@ static bool band_enabled()
 }
 
 // Half-width of field f's operator along axis a for m = 1 .. (returned count)
-// substeps: the dropped-tail width, or the whole line when that is shorter.
+// substeps: where the tails sum to less than 1e-8, or the whole line when that
+// is shorter.
 static int band_widths(const vfd_world *w, int f, int a, int mmax, int *out)
 {
     const int n = a == 0 ? w->nx : a == 1 ? w->ny : w->nz;
