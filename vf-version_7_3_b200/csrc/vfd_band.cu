@@ -30,7 +30,7 @@
 // blocks still to be read start at 64 (b + 2) - H or later.
 //
 // Roles (one CTA per SM, persistent): warps 0..7 read the accumulators back
-// and store the outputs (four warps an accumulator), warps 8..15 convert input
+// and store the outputs, warps 8..15 convert input
 // blocks and store them to tensor memory, warps 16..19 copy input blocks to
 // shared memory (bulk tensor copies, or cp.async where the layout does not
 // allow them; nstage blocks deep), warps 20 and 21 issue the
@@ -249,11 +249,14 @@ __device__ __forceinline__ int band_at(int line, int pos)
 }
 
 // ---------------------------------------------------------------------------
-// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.71-0.75 ms a pass for
-// ten folded substeps (4.3-4.5 TB/s of the 8 bytes a voxel it moves; without its
-// products 0.60; with one offset a line instead of one a block 0.69-0.70), so a
-// tick of ten substeps and its deposit takes 2.7 ms back to back against 19.0 ms
-// on 30 register-FFT passes of 0.58-0.66 ms.  768x384x576: 9.7 against 60 ms.
+// The pass.  Measured on B200, 512x256x384 x 8 fields: 0.70-0.72 ms a pass for
+// ten folded substeps (4.5 TB/s of the 8 bytes a voxel it moves; without its
+// products 0.60), so a tick of ten substeps and its deposit takes 2.64 ms back to
+// back against 19.0 ms on 30 register-FFT passes of 0.58-0.66 ms.  768x384x576:
+// 9.4 against 60 ms.  An accumulator is free for the next block as soon as its
+// eight warps have read it (each a quarter of the lines, half of the outputs);
+// four warps that worked through the halves in turn held it for 0.71-0.75 ms a
+// pass (97x61x45 x 3, ten substeps: 52 -> 47 us a tick).
 // What bounds it: HBM, with the products (48 cycles each, two issuing threads
 // together), the read-back of the accumulators and the ring of four input
 // blocks limiting how far its stages overlap.
@@ -691,16 +694,18 @@ __device__ __forceinline__ void band_issuer(const BandTiles &T, int par, int slo
     if (mine >= 1) band_wait(&S.dfull[par], (mine - 1) & 1, &S.dead);
 }
 
-// Stores the outputs: 32 positions of the warp's 32 lines at a time.
+// Stores the outputs: 32 positions of a block, of the warp's 32 lines.
 template <int AXIS>
 __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsigned char *xout, BandShared &S,
                                               uint32_t tmem)
 {
     constexpr bool XP = AXIS == PASS_X, zl = AXIS == PASS_Z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int quad = warp & 3, team = warp >> 2;  // team: the accumulator (every other block) this warp reads
-    const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + BD_ACC_COL + team * BD_BLK;
-    int i = 0, phase = 0, job = -1;
+    // the lines and the half of every block's outputs this warp reads: all warps
+    // have read an accumulator before they work on its values
+    const int quad = warp & 3, half = warp >> 2;
+    const uint32_t ta = tmem + ((uint32_t)(quad * 32) << 16) + BD_ACC_COL + 32 * half;
+    int i = 0, job = -1;
     double acc_ot = 0.0, acc_ct = 0.0;  // of the values stored, and (where there is a baseline) before it is added
     const BandJob &J = S.job[warp];
     auto flush = [&]() {
@@ -732,144 +737,138 @@ __device__ __forceinline__ void band_epilogue(const BandTiles &T, int sums, unsi
             dst += lok ? (int64_t)o * J.outer_stride + (l - o * J.n0) : 0;
         }
         for (int b = 0; b < J.nb; ++b, ++i) {
-            if ((i & 1) != team) continue;
-            band_wait(&S.dfull[team], phase, &S.dead);
-            phase ^= 1;
+            const int par = i & 1;
+            band_wait(&S.dfull[par], (i >> 1) & 1, &S.dead);
             tc_fence_after();
             const bool live = !*(volatile int *)&S.dead;
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                float2 t[16];  // positions 2 c, 2 c + 1 of this half
-                // the offsets of the window's blocks (two, or three where it spans as
-                // many): the last one's, the steps to it from the first (d0) and
-                // from the second (d1)
-                const bool three = J.ksteps > 2 * BD_BLK / 16;
-                auto offset = [&](int k) { return S.off[(ein + min(k, J.nin - 1)) % BD_OFFS][quad * 32 + lane]; };
-                float off = offset(b + 1), d1 = 0.0f;
-                const float d0 = offset(b) - off;
-                if (three) {
-                    const float last = offset(b + 2);
-                    d1 = off - last;
-                    off = last;
+            // the offsets of the window's blocks (two, or three where it spans as
+            // many): the last one's, the steps to it from the first (d0) and from
+            // the second (d1)
+            const bool three = J.ksteps > 2 * BD_BLK / 16;
+            auto offset = [&](int k) { return S.off[(ein + min(k, J.nin - 1)) % BD_OFFS][quad * 32 + lane]; };
+            float off = offset(b + 1), d1 = 0.0f;
+            const float d0 = offset(b) - off;
+            if (three) {
+                const float last = offset(b + 2);
+                d1 = off - last;
+                off = last;
+            }
+            float2 t[16];  // positions 2 c, 2 c + 1 of this half
+            __syncwarp();
+            tc_ld32(ta + par * BD_BLK, t);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.dempty[par]);
+            // the offsets' share: the weights' sums over the window's first
+            // block, its first two and all of it
+            const float4 *rho = reinterpret_cast<const float4 *>(J.rho + J.image(b) * (3 * BD_BLK) + 32 * half);
+            auto add = [&](float d, const float4 *r) {
+                const float2 d2 = make_float2(d, d);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float4 q = __ldg(r + c);
+                    t[2 * c] = __ffma2_rn(d2, make_float2(q.x, q.y), t[2 * c]);
+                    t[2 * c + 1] = __ffma2_rn(d2, make_float2(q.z, q.w), t[2 * c + 1]);
                 }
-                __syncwarp();
-                tc_ld32(ta + 32 * half, t);
-                if (half == 1) {
-                    tc_fence_before();
+            };
+            add(d0, rho);
+            if (three) add(d1, rho + BD_BLK / 4);
+            const bool inner = b >= J.b0 && b < J.b1;  // the sums over all of a window are all the same
+            if (!inner) add(off, rho + 2 * (BD_BLK / 4));
+            auto shift = [&](float o) {
+                const float2 o2 = make_float2(o, o);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
+            };
+            if (inner) shift(off * J.fscale);
+            const int p0 = BD_BLK * b + 32 * half;
+            if (XP) {
+                // 32 rows x 16 positions at a time through shared memory,
+                // 64-byte row segments out
+                unsigned char *o = xout + warp * 2048;
+                const int rmax = live ? J.nlines - l0 : 0;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&S.dempty[team]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<float4 *>(o + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+                            make_float4(t[8 * g + 2 * c].x, t[8 * g + 2 * c].y, t[8 * g + 2 * c + 1].x,
+                                        t[8 * g + 2 * c + 1].y);
+                    __syncwarp();
+                    if (J.vec) {
+                        const int c = lane & 3, r0 = lane >> 2, p = p0 + 16 * g + 4 * c;
+                        const int rm = p < n ? rmax : 0;
+                        float *q = dst + (int64_t)(l0 + r0) * n + p;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e, q += 8 * n) {
+                            const int r = 8 * e + r0;
+                            const float4 x =
+                                *reinterpret_cast<const float4 *>(o + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+                            if (r < rm) *reinterpret_cast<float4 *>(q) = x;
+                        }
+                    } else {
+                        const int c = lane & 15, r0 = lane >> 4, p = p0 + 16 * g + c;
+                        const int rm = p < n ? rmax : 0;
+                        float *q = dst + (int64_t)(l0 + r0) * n + p;
+#pragma unroll 8
+                        for (int e = 0; e < 16; ++e, q += 2 * n) {
+                            const int r = 2 * e + r0;
+                            const float x = *reinterpret_cast<const float *>(
+                                o + r * 64 + (((c >> 2) ^ ((r >> 1) & 3)) << 4) + ((c & 3) << 2));
+                            if (r < rm) *q = x;
+                        }
+                    }
                 }
-                // the offsets' share: the weights' sums over the window's first
-                // block, its first two and all of it
-                const float4 *rho = reinterpret_cast<const float4 *>(J.rho + J.image(b) * (3 * BD_BLK) + 32 * half);
-                auto add = [&](float d, const float4 *r) {
-                    const float2 d2 = make_float2(d, d);
+            } else {
+                const int naff = zl ? J.naff : 0, ly = naff ? l / J.nx : 0, lx = l - ly * J.nx;
+                for (int g = 0; g < naff; ++g) {
+                    // the affine rows, decayed like the rest
+                    const float q = lok ? J.keep * J.affc[g] * J.aff[0][(int64_t)g * J.affs[0] + lx] *
+                                              J.aff[1][(int64_t)g * J.affs[1] + ly]
+                                        : 0.0f;
+                    const float2 q2 = make_float2(q, q);
+                    const float4 *z = reinterpret_cast<const float4 *>(J.aff[2] + (int64_t)g * J.affs[2] + p0);
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
-                        const float4 q = __ldg(r + c);
-                        t[2 * c] = __ffma2_rn(d2, make_float2(q.x, q.y), t[2 * c]);
-                        t[2 * c + 1] = __ffma2_rn(d2, make_float2(q.z, q.w), t[2 * c + 1]);
+                        const float4 zz = __ldg(z + c);
+                        t[2 * c] = __ffma2_rn(q2, make_float2(zz.x, zz.y), t[2 * c]);
+                        t[2 * c + 1] = __ffma2_rn(q2, make_float2(zz.z, zz.w), t[2 * c + 1]);
                     }
-                };
-                add(d0, rho);
-                if (three) add(d1, rho + BD_BLK / 4);
-                const bool inner = b >= J.b0 && b < J.b1;  // the sums over all of a window are all the same
-                if (!inner) add(off, rho + 2 * (BD_BLK / 4));
-                auto shift = [&](float o) {
-                    const float2 o2 = make_float2(o, o);
-#pragma unroll
-                    for (int c = 0; c < 16; ++c) t[c] = __fadd2_rn(t[c], o2);
-                };
-                if (inner) shift(off * J.fscale);
-                const int p0 = BD_BLK * b + 32 * half;
-                if (XP) {
-                    // 32 rows x 16 positions at a time through shared memory,
-                    // 64-byte row segments out
-                    unsigned char *o = xout + warp * 2048;
-                    const int rmax = live ? J.nlines - l0 : 0;
-#pragma unroll
-                    for (int g = 0; g < 2; ++g) {
-                        __syncwarp();
-#pragma unroll
-                        for (int c = 0; c < 4; ++c)
-                            *reinterpret_cast<float4 *>(o + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
-                                make_float4(t[8 * g + 2 * c].x, t[8 * g + 2 * c].y, t[8 * g + 2 * c + 1].x,
-                                            t[8 * g + 2 * c + 1].y);
-                        __syncwarp();
-                        if (J.vec) {
-                            const int c = lane & 3, r0 = lane >> 2, p = p0 + 16 * g + 4 * c;
-                            const int rm = p < n ? rmax : 0;
-                            float *q = dst + (int64_t)(l0 + r0) * n + p;
-#pragma unroll
-                            for (int e = 0; e < 4; ++e, q += 8 * n) {
-                                const int r = 8 * e + r0;
-                                const float4 x =
-                                    *reinterpret_cast<const float4 *>(o + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-                                if (r < rm) *reinterpret_cast<float4 *>(q) = x;
-                            }
-                        } else {
-                            const int c = lane & 15, r0 = lane >> 4, p = p0 + 16 * g + c;
-                            const int rm = p < n ? rmax : 0;
-                            float *q = dst + (int64_t)(l0 + r0) * n + p;
-#pragma unroll 8
-                            for (int e = 0; e < 16; ++e, q += 2 * n) {
-                                const int r = 2 * e + r0;
-                                const float x = *reinterpret_cast<const float *>(
-                                    o + r * 64 + (((c >> 2) ^ ((r >> 1) & 3)) << 4) + ((c & 3) << 2));
-                                if (r < rm) *q = x;
-                            }
-                        }
-                    }
-                } else {
-                    const int naff = zl ? J.naff : 0, ly = naff ? l / J.nx : 0, lx = l - ly * J.nx;
-                    for (int g = 0; g < naff; ++g) {
-                        // the affine rows, decayed like the rest
-                        const float q = lok ? J.keep * J.affc[g] * J.aff[0][(int64_t)g * J.affs[0] + lx] *
-                                                  J.aff[1][(int64_t)g * J.affs[1] + ly]
-                                            : 0.0f;
-                        const float2 q2 = make_float2(q, q);
-                        const float4 *z = reinterpret_cast<const float4 *>(J.aff[2] + (int64_t)g * J.affs[2] + p0);
-#pragma unroll
-                        for (int c = 0; c < 8; ++c) {
-                            const float4 zz = __ldg(z + c);
-                            t[2 * c] = __ffma2_rn(q2, make_float2(zz.x, zz.y), t[2 * c]);
-                            t[2 * c + 1] = __ffma2_rn(q2, make_float2(zz.z, zz.w), t[2 * c + 1]);
-                        }
-                    }
-                    const int m = lok ? min(32, n - p0) : 0;
-                    auto sum = [&]() {  // over the line's positions
-                        if (m < 32) {
-#pragma unroll
-                            for (int x = 0; x < 16; ++x) {
-                                if (2 * x >= m) t[x].x = 0.0f;
-                                if (2 * x + 1 >= m) t[x].y = 0.0f;
-                            }
-                        }
-                        return (double)sum32(t);
-                    };
-                    const bool acc = zl && sums && J.sums && m > 0;
-                    if (zl && J.b != 0.0f) {
-                        // out = keep (t + baseline), keep being part of the operator
-                        if (acc) acc_ct += sum();
-                        shift(J.keep * J.b);
-                    }
-                    if (acc) acc_ot += sum();
-                    const int64_t ps = J.pos_stride;
-                    float *q = dst + (int64_t)p0 * ps;
-                    if (m == 32 && live) {
+                }
+                const int m = lok ? min(32, n - p0) : 0;
+                auto sum = [&]() {  // over the line's positions
+                    if (m < 32) {
 #pragma unroll
                         for (int x = 0; x < 16; ++x) {
-                            q[0] = t[x].x;
-                            q[ps] = t[x].y;
-                            q += 2 * ps;
+                            if (2 * x >= m) t[x].x = 0.0f;
+                            if (2 * x + 1 >= m) t[x].y = 0.0f;
                         }
-                    } else if (live) {
+                    }
+                    return (double)sum32(t);
+                };
+                const bool acc = zl && sums && J.sums && m > 0;
+                if (zl && J.b != 0.0f) {
+                    // out = keep (t + baseline), keep being part of the operator
+                    if (acc) acc_ct += sum();
+                    shift(J.keep * J.b);
+                }
+                if (acc) acc_ot += sum();
+                const int64_t ps = J.pos_stride;
+                float *q = dst + (int64_t)p0 * ps;
+                if (m == 32 && live) {
 #pragma unroll
-                        for (int x = 0; x < 16; ++x) {
-                            if (2 * x < m) q[0] = t[x].x;
-                            if (2 * x + 1 < m) q[ps] = t[x].y;
-                            q += 2 * ps;
-                        }
+                    for (int x = 0; x < 16; ++x) {
+                        q[0] = t[x].x;
+                        q[ps] = t[x].y;
+                        q += 2 * ps;
+                    }
+                } else if (live) {
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) {
+                        if (2 * x < m) q[0] = t[x].x;
+                        if (2 * x + 1 < m) q[ps] = t[x].y;
+                        q += 2 * ps;
                     }
                 }
             }
@@ -903,7 +902,7 @@ __global__ void __launch_bounds__(BD_THREADS, 1)
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&S.dfull[s], 1);
-            mbar_init(&S.dempty[s], BD_EPI_WARPS / 2);
+            mbar_init(&S.dempty[s], BD_EPI_WARPS);
             mbar_init(&S.wfull[s], 1);
         }
         mbar_fence_init();
