@@ -716,7 +716,7 @@ def main():
     per_pass = {k: prof[k][0] / max(prof[k][1], 1) for k in prof}
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": AXIS_TRAFFIC_BYTES,
-                "kernel": "axis passes: band_kernel (x; y and z), a tick's substeps in one pass per axis",
+                "kernel": "axis passes: band_kernel (x, y, z), a tick's substeps in one pass per axis",
                 "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms,
                 "peak_source": f"{peak_kind} hbm_gbs",
                 "share_of_step": axis_ms / ms if ms > 0 else None,

@@ -30,12 +30,11 @@
 // blocks still to be read start at 64 (b + 2) - H or later.
 //
 // Roles (one CTA per SM, persistent): warps 0..7 read the accumulators back
-// and store the outputs, warps 8..15 convert input
-// blocks and store them to tensor memory, warps 16..19 copy input blocks to
-// shared memory (bulk tensor copies, or cp.async where the layout does not
-// allow them; nstage blocks deep), warps 20 and 21 issue the
-// products of even and of odd blocks, warp 22 fetches weight images (bulk
-// copies).
+// and store the outputs, warps 8..15 convert input blocks and store them to
+// tensor memory, warps 16..19 copy input blocks to shared memory (bulk tensor
+// copies, or cp.async where the layout does not allow them; nstage blocks
+// deep), warps 20 and 21 issue the products of even and of odd blocks, warp 22
+// fetches weight images (bulk copies).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
