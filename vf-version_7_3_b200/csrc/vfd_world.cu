@@ -953,9 +953,10 @@ static std::vector<int> band_groups(int n_substeps, int limit)
 // on it when the kernels are narrow and the fields not small: a banded pass
 // takes the same time at every radius up to 8, an FFT pass's blocks give 64 -
 // 2r outputs.  Measured, 8 fields, one substep, banded / FFT (us): mean radius
-// 3.5: 64x64x32 35 / 46, 96x64x64 54 / 58, 128x96x96 95 / 85, 256x128x192 309 /
-// 304, 512x256x256 1236 / 1168; mean radius 5.1: 512x256x384 2094 / 2067; mean
-// radius 6.5: 35 / 46, 53 / 68, 96 / 116, 307 / 378, 1226 / 1318.
+// 3.5: 64x64x32 34 / 46, 96x64x64 52 / 59, 128x64x64 61 / 64, 128x96x64 76 / 74,
+// 128x96x96 97 / 86, 256x128x192 326 / 304, 512x256x256 1316 / 1168; mean radius
+// 5.4: 128x96x96 97 / 125, 256x128x192 327 / 398, 512x256x256 1306 / 1306; mean
+// radius 6.5: 34 / 46, 52 / 70, 97 / 115, 326 / 378, 1305 / 1320.
 constexpr int64_t BAND_SMALL = (int64_t)4 << 20;  // voxels x fields
 // single: what was timed for the batch the tick is of (-1: nothing).
 static bool runs_band(const vfd_world *w, int n_substeps, int single = -1)
